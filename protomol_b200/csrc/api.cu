@@ -488,10 +488,9 @@ int evaluate_forces(System *s, int only, int mode, int fold) {
           }
           if (f.ewald_flags & PMGPU_EWALD_RECIPROCAL) {
             prof_begin(s, PMGPU_PHASE_PME);
-            r = pme_reciprocal(s, &f, em);
+            r = pme_reciprocal(s, &f, em, &s->kernels);
             prof_end(s);
             PM_CHECK(r);
-            s->kernels += 4;  // spread, fixed->float, convolve, gather (+ cuFFT)
           }
           break;
         case FK_GB:

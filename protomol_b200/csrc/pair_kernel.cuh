@@ -695,19 +695,6 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   }
 }
 
-// The launch arguments of a batched launch's member, copied into shared
-// memory by the block (every thread reads them many times).
-template <typename A>
-__device__ __forceinline__ const A &batch_args_shared(const A *__restrict__ tab, int m,
-                                                      unsigned char *raw) {
-  static_assert(sizeof(A) % 4 == 0, "argument structs are whole words");
-  const int *src = reinterpret_cast<const int *>(tab + m);
-  int *dst = reinterpret_cast<int *>(raw);
-  for (int k = threadIdx.x; k < (int)(sizeof(A) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
-  __syncthreads();
-  return *reinterpret_cast<const A *>(raw);
-}
-
 template <typename Real, int TERMS, int MODE, typename SPEC>
 __global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE, SPEC>::blocks)
     k_pairs(PairArgs<Real> a) {

@@ -415,6 +415,19 @@ __device__ __forceinline__ Blk batch_blk(const int *__restrict__ first, int m) {
   return Blk{(int)blockIdx.x - f, __ldg(first + m + 1) - f};
 }
 
+// The launch arguments of a batched launch's member, copied into shared
+// memory by the block (every thread reads them many times).
+template <typename A>
+__device__ __forceinline__ const A &batch_args_shared(const A *__restrict__ tab, int m,
+                                                      unsigned char *raw) {
+  static_assert(sizeof(A) % 4 == 0, "argument structs are whole words");
+  const int *src = reinterpret_cast<const int *>(tab + m);
+  int *dst = reinterpret_cast<int *>(raw);
+  for (int k = threadIdx.x; k < (int)(sizeof(A) / 4); k += blockDim.x) dst[k] = __ldg(src + k);
+  __syncthreads();
+  return *reinterpret_cast<const A *>(raw);
+}
+
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll

@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "fft.cuh"
 #include "pmgpu.h"
 
 namespace pmgpu {
@@ -227,7 +228,10 @@ struct Force {
   int grid[3] = {0, 0, 0};
   double self_energy = 0, charged_energy = 0;
   // pme device state
-  cufftHandle plan_r2c = 0, plan_c2r = 0;
+  int own_fft = 0;                    // the grid is transformed by fft.cuh's kernels
+  FftGrid fft{};                      // its plan (twiddles in d_twiddle)
+  float2 *d_twiddle = nullptr;
+  cufftHandle plan_r2c = 0, plan_c2r = 0;  // other grids: cuFFT
   float *d_grid = nullptr;            // real grid (K1*K2*K3)
   long long *d_grid_fixed = nullptr;  // fixed-point spread target
   float2 *d_cgrid = nullptr;          // complex grid (K1*K2*(K3/2+1))
@@ -539,7 +543,7 @@ int pme_init(System *s, Force *f);
 int pme_free(System *s, Force *f);
 // builds f->d_ewtab for f->alpha (nonbonded.cu)
 int ewald_table_build(System *s, Force *f);
-int pme_reciprocal(System *s, Force *f, int em);
+int pme_reciprocal(System *s, Force *f, int em, long long *launched);
 int ewald_correction(System *s, Force *f, int em);
 
 // gb.cu

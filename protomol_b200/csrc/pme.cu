@@ -3,9 +3,10 @@
 // NonbondedFullEwaldSystemForce:
 //   * spread: cardinal B-spline (order p) charge spreading into an int64
 //     fixed-point grid (order independent, bit reproducible);
-//   * 3-D real-to-complex FFT (cuFFT, same stream), convolution with the
-//     influence function exp(-pi^2 m^2/alpha^2)/(pi V m^2) |b(m)|^2 with the
-//     energy and virial reduced on the way, complex-to-real FFT;
+//   * 3-D real-to-complex FFT, convolution with the influence function
+//     exp(-pi^2 m^2/alpha^2)/(pi V m^2) |b(m)|^2 with the energy and virial
+//     reduced on the way, complex-to-real FFT: three kernels (fft.cuh), or
+//     cuFFT and two kernels for grids those do not take;
 //   * gather: forces from the B-spline derivatives;
 //   * correctionTerm (NonbondedFullEwaldSystemForce.h:1092-1131) in FP64.
 // The reciprocal energy matches the reference's convention
@@ -173,60 +174,230 @@ struct ConvolveArgs {
   long long *acc;
   int em;
 };
+// Mode idx's share of the reciprocal energy (em >= 1) and virial (em 2): g
+// its influence, f its amplitude before the convolution.
+__device__ __forceinline__ void mode_energy(const ConvolveArgs &A, int idx, float g, float2 f,
+                                            double &e, double (&v)[6]) {
+  const int Kh = A.K2 / 2 + 1;
+  const int mz = idx % Kh;
+  const double w = (mz == 0 || (A.K2 % 2 == 0 && mz == A.K2 / 2)) ? 1.0 : 2.0;
+  const double f2 = (double)f.x * f.x + (double)f.y * f.y;
+  const double emode = 0.5 * w * (double)g * f2;
+  e += emode;
+  if (A.em == 2 && g != 0.f) {
+    const int my_ = (idx / Kh) % A.K1, mx_ = idx / (Kh * A.K1);
+    const int mx = mx_ <= A.K0 / 2 ? mx_ : mx_ - A.K0;
+    const int my = my_ <= A.K1 / 2 ? my_ : my_ - A.K1;
+    const double hx = mx / A.L0, hy = my / A.L1, hz = mz / A.L2;
+    const double h2 = hx * hx + hy * hy + hz * hz;
+    const double pa = M_PI * M_PI / (A.alpha * A.alpha);
+    const double cc = 2.0 * (1.0 / h2 + pa);
+    v[0] += emode * (1.0 - cc * hx * hx);
+    v[1] -= emode * cc * hx * hy;
+    v[2] -= emode * cc * hx * hz;
+    v[3] += emode * (1.0 - cc * hy * hy);
+    v[4] -= emode * cc * hy * hz;
+    v[5] += emode * (1.0 - cc * hz * hz);
+  }
+}
+__device__ __forceinline__ void mode_reduce(const ConvolveArgs &A, double e, double (&v)[6]) {
+  if (!A.em) return;
+  e = warp_sum(e);
+  if (A.em == 2)
+    for (int q = 0; q < 6; q++) v[q] = warp_sum(v[q]);
+  if ((threadIdx.x & 31) == 0) {
+    red_add(&A.acc[ACC_COULOMB], to_fixed(e, kEnergyScale));
+    if (A.em == 2) {
+      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+      for (int q = 0; q < 9; q++)
+        red_add(&A.acc[ACC_VIRIAL + q], to_fixed(v[map[q]], kEnergyScale));
+    }
+  }
+}
 __device__ __forceinline__ void convolve_body(const ConvolveArgs &A, Blk b) {
-  const int K0 = A.K0, K1 = A.K1, K2 = A.K2, em = A.em;
-  const double L0 = A.L0, L1 = A.L1, L2 = A.L2, alpha = A.alpha;
-  const float *__restrict__ infl = A.infl;
-  float2 *__restrict__ c = A.c;
-  long long *__restrict__ acc = A.acc;
-  const int Kh = K2 / 2 + 1;
-  const int total = K0 * K1 * Kh;
+  const int total = A.K0 * A.K1 * (A.K2 / 2 + 1);
   const int idx = b.x * blockDim.x + threadIdx.x;
   double e = 0, v[6] = {0, 0, 0, 0, 0, 0};
   if (idx < total) {
-    const float g = infl[idx];
-    const float2 f = c[idx];
-    c[idx] = make_float2(g * f.x, g * f.y);
-    if (em) {
-      const int mz = idx % Kh;
-      const double w = (mz == 0 || (K2 % 2 == 0 && mz == K2 / 2)) ? 1.0 : 2.0;
-      const double f2 = (double)f.x * f.x + (double)f.y * f.y;
-      const double emode = 0.5 * w * (double)g * f2;
-      e = emode;
-      if (em == 2 && g != 0.f) {
-        const int my_ = (idx / Kh) % K1, mx_ = idx / (Kh * K1);
-        const int mx = mx_ <= K0 / 2 ? mx_ : mx_ - K0;
-        const int my = my_ <= K1 / 2 ? my_ : my_ - K1;
-        const double hx = mx / L0, hy = my / L1, hz = mz / L2;
-        const double h2 = hx * hx + hy * hy + hz * hz;
-        const double pa = M_PI * M_PI / (alpha * alpha);
-        const double cc = 2.0 * (1.0 / h2 + pa);
-        v[0] = emode * (1.0 - cc * hx * hx);
-        v[1] = -emode * cc * hx * hy;
-        v[2] = -emode * cc * hx * hz;
-        v[3] = emode * (1.0 - cc * hy * hy);
-        v[4] = -emode * cc * hy * hz;
-        v[5] = emode * (1.0 - cc * hz * hz);
-      }
-    }
+    const float g = A.infl[idx];
+    const float2 f = A.c[idx];
+    A.c[idx] = make_float2(g * f.x, g * f.y);
+    if (A.em) mode_energy(A, idx, g, f, e, v);
   }
-  if (!em) return;
-  e = warp_sum(e);
-  if (em == 2)
-    for (int q = 0; q < 6; q++) v[q] = warp_sum(v[q]);
-  if ((threadIdx.x & 31) == 0) {
-    red_add(&acc[ACC_COULOMB], to_fixed(e, kEnergyScale));
-    if (em == 2) {
-      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-      for (int q = 0; q < 9; q++) red_add(&acc[ACC_VIRIAL + q], to_fixed(v[map[q]], kEnergyScale));
-    }
-  }
+  mode_reduce(A, e, v);
 }
 __global__ void k_pme_convolve(ConvolveArgs a) { convolve_body(a, own_blk()); }
 __global__ void k_pme_convolve_batch(const ConvolveArgs *__restrict__ tab,
                                      const int *__restrict__ first, int nm) {
   const int m = batch_member(first, nm, blockIdx.x);
   convolve_body(tab[m], batch_blk(first, m));
+}
+
+// ---------------------------------------------------------- own FFT
+// The transforms and the convolution of a grid (fft.cuh).  Ten dependent
+// launches of spread, conversion, six cuFFT kernels, convolution and gather
+// become five, and an ensemble's launches no longer grow with the number of
+// its grid sizes: a launch's plane or column blocks come from every member.
+// Bound by latency (trips to memory, then five to seven short synchronised
+// passes): at 64^3 the three kernels take 8.1, 8.8 and 7.6 us against 28 us
+// for the eight they replace, at 40^3 6.9, 7.6 and 6.5 against 23 us (caches
+// warm); a 5,001-atom MD step 52.7 against 55.2 us, 24 boxes of nine grid
+// sizes 259 against 338 us a step.  Launching the chain as programmatic
+// dependents was slower (5,776 against 5,048 us for 50 steps of 23,550
+// atoms: waiting blocks hold room the pair kernel needs).
+struct FftArgs {
+  FftGrid g;
+  long long *fixed;  // fixed-point charges (read and cleared)
+  float *grid;       // potential
+  ConvolveArgs cv;   // c: the half-complex grid between the kernels
+};
+constexpr int kFftXThreads = 128;  // also fixes the energy's partial sums
+
+extern __shared__ float2 fft_smem[];
+
+// Elements 0..n-1 dealt to the block's threads, load(k) of kFftLoads of them
+// in flight before the first store(k, value): one trip to memory per
+// kFftLoads elements of a thread instead of one per element.
+constexpr int kFftLoads = 8;
+template <typename T, typename L, typename S>
+__device__ __forceinline__ void fft_stream(int n, L load, S store) {
+  for (int k0 = threadIdx.x; k0 < n; k0 += kFftLoads * blockDim.x) {
+    T v[kFftLoads];
+#pragma unroll
+    for (int u = 0; u < kFftLoads; u++) {
+      const int k = k0 + u * blockDim.x;
+      if (k < n) v[u] = load(k);
+    }
+#pragma unroll
+    for (int u = 0; u < kFftLoads; u++) {
+      const int k = k0 + u * blockDim.x;
+      if (k < n) store(k, v[u]);
+    }
+  }
+}
+
+__device__ __forceinline__ void fft_yz_body(const FftArgs &A, Blk b) {
+  const FftGrid &g = A.g;
+  float2 *sm = fft_smem;
+  const int t0 = threadIdx.x, nt = blockDim.x, buf = fft_plane_buf(g);
+  const int ty = 2 * buf, tz = ty + g.K1, nz = g.K2, np = g.K1 * g.K2;
+  // a plane's charges: element (row, z) is the real part of pair row / 2 for
+  // an even row, the imaginary part for an odd one
+  long long *plane = A.fixed + (size_t)b.x * np;
+  const float iz = 1.0f / (float)nz;
+  float *sf = reinterpret_cast<float *>(sm);
+  for (int k = t0; k < g.K1 + g.K2; k += nt) sm[ty + k] = __ldg(g.tw + g.K0 + k);
+  fft_stream<long long>(np, [&](int k) { return plane[k]; },
+                        [&](int k, long long q) {
+                          const int row = fft_div(k, iz), z = k - row * nz;
+                          // the same rounding as through FP64: scaling by 2^-32 is exact
+                          sf[2 * (z * g.ldz + (row >> 1)) + (row & 1)] =
+                              __ll2float_rn(q) * (float)(1.0 / kGridScale);
+                        });
+  if (g.K1 & 1)
+    for (int z = t0; z < nz; z += nt) sf[2 * (z * g.ldz + g.P - 1) + 1] = 0.f;
+  for (int k = t0; k < np; k += nt) plane[k] = 0;  // ready for the next spread
+  __syncthreads();
+  int r = fft_lines(g.d[2], sm, 0, buf, g.P, g.ldz, tz, t0, nt);
+  fft_unpack_rows(g, sm, r, buf - r, t0, nt);
+  __syncthreads();
+  r = fft_lines(g.d[1], sm, buf - r, r, g.Kh, g.Kh, ty, t0, nt);
+  float2 *c = A.cv.c + (size_t)b.x * g.K1 * g.Kh;
+  for (int k = t0; k < g.K1 * g.Kh; k += nt) c[k] = sm[r + k];
+}
+
+__device__ __forceinline__ void fft_x_body(const FftArgs &A, Blk b) {
+  const FftGrid &g = A.g;
+  float2 *sm = fft_smem;
+  const int t0 = threadIdx.x, nt = blockDim.x, C = g.cols, ncol = g.K1 * g.Kh;
+  const int lc = C == 16 ? 4 : 3, c0 = b.x * C, buf = g.K0 * C, tx = 2 * buf;
+  for (int k = t0; k < g.K0; k += nt) sm[tx + k] = __ldg(g.tw + k);
+  fft_stream<float2>(buf,
+                     [&](int k) {
+                       const int col = c0 + (k & (C - 1));
+                       return col < ncol ? A.cv.c[(size_t)(k >> lc) * ncol + col]
+                                         : make_float2(0.f, 0.f);
+                     },
+                     [&](int k, float2 v) { sm[k] = v; });
+  __syncthreads();
+  int r = 0;
+#pragma unroll 1
+  for (int inverse = 0; inverse < 2; inverse++) {
+    r = fft_lines(g.d[0], sm, r, buf - r, C, C, tx, t0, nt);
+    if (inverse) break;
+    double e = 0, v[6] = {0, 0, 0, 0, 0, 0};
+    fft_stream<float>(buf,
+                      [&](int k) {
+                        const int col = c0 + (k & (C - 1));
+                        return col < ncol ? __ldg(A.cv.infl + (k >> lc) * ncol + col) : 0.f;
+                      },
+                      [&](int k, float w) {
+                        const int col = c0 + (k & (C - 1));
+                        const float2 f = sm[r + k];
+                        // swapped: the next transform is the inverse
+                        sm[r + k] = make_float2(w * f.y, w * f.x);
+                        if (A.cv.em && col < ncol)
+                          mode_energy(A.cv, (k >> lc) * ncol + col, w, f, e, v);
+                      });
+    mode_reduce(A.cv, e, v);
+    __syncthreads();
+  }
+  for (int k = t0; k < buf; k += nt) {
+    const int col = c0 + (k & (C - 1));
+    if (col < ncol) A.cv.c[(size_t)(k >> lc) * ncol + col] = sm[r + k];
+  }
+}
+
+__device__ __forceinline__ void fft_zy_body(const FftArgs &A, Blk b) {
+  const FftGrid &g = A.g;
+  float2 *sm = fft_smem;
+  const int t0 = threadIdx.x, nt = blockDim.x, buf = fft_plane_buf(g);
+  const int ty = 2 * buf, tz = ty + g.K1, nz = g.K2, np = g.K1 * g.K2;
+  const float2 *c = A.cv.c + (size_t)b.x * g.K1 * g.Kh;
+  for (int k = t0; k < g.K1 + g.K2; k += nt) sm[ty + k] = __ldg(g.tw + g.K0 + k);
+  fft_stream<float2>(g.K1 * g.Kh, [&](int k) { return c[k]; },
+                     [&](int k, float2 v) { sm[k] = v; });
+  __syncthreads();
+  int r = fft_lines(g.d[1], sm, 0, buf, g.Kh, g.Kh, ty, t0, nt);
+  fft_pack_rows(g, sm, r, buf - r, t0, nt);
+  __syncthreads();
+  r = fft_lines(g.d[2], sm, buf - r, r, g.P, g.ldz, tz, t0, nt);
+  // swapped: row 2p in the imaginary part, row 2p + 1 in the real part
+  float *plane = A.grid + (size_t)b.x * np;
+  const float iz = 1.0f / (float)nz;
+  const float *sf = reinterpret_cast<const float *>(sm + r);
+  for (int k = t0; k < np; k += nt) {
+    const int row = fft_div(k, iz), z = k - row * nz;
+    plane[k] = sf[2 * (z * g.ldz + (row >> 1)) + 1 - (row & 1)];
+  }
+}
+
+__global__ void __launch_bounds__(512) k_fft_yz(FftArgs a) {
+  fft_yz_body(a, own_blk());
+}
+__global__ void __launch_bounds__(kFftXThreads) k_fft_x(FftArgs a) {
+  fft_x_body(a, own_blk());
+}
+__global__ void __launch_bounds__(512) k_fft_zy(FftArgs a) {
+  fft_zy_body(a, own_blk());
+}
+__global__ void __launch_bounds__(512)
+k_fft_yz_batch(const FftArgs *__restrict__ tab, const int *__restrict__ first, int nm) {
+  __shared__ __align__(16) unsigned char raw[sizeof(FftArgs)];
+  const int m = batch_member(first, nm, blockIdx.x);
+  fft_yz_body(batch_args_shared(tab, m, raw), batch_blk(first, m));
+}
+__global__ void __launch_bounds__(kFftXThreads)
+k_fft_x_batch(const FftArgs *__restrict__ tab, const int *__restrict__ first, int nm) {
+  __shared__ __align__(16) unsigned char raw[sizeof(FftArgs)];
+  const int m = batch_member(first, nm, blockIdx.x);
+  fft_x_body(batch_args_shared(tab, m, raw), batch_blk(first, m));
+}
+__global__ void __launch_bounds__(512)
+k_fft_zy_batch(const FftArgs *__restrict__ tab, const int *__restrict__ first, int nm) {
+  __shared__ __align__(16) unsigned char raw[sizeof(FftArgs)];
+  const int m = batch_member(first, nm, blockIdx.x);
+  fft_zy_body(batch_args_shared(tab, m, raw), batch_blk(first, m));
 }
 
 // Gather: L lanes per atom, lane kx < P sums its x plane; the partial
@@ -413,6 +584,30 @@ static void bspline_moduli(int K, int p, std::vector<float> &out) {
   for (int i = 0; i < K; i++) out[i] = (float)(1.0 / mod[i]);
 }
 
+// Planes above 48 KB need the kernels' dynamic shared memory raised.
+static int fft_set_smem() {
+  const int most = (int)kFftSmem;
+  const void *k[] = {(const void *)k_fft_yz,       (const void *)k_fft_x,
+                     (const void *)k_fft_zy,       (const void *)k_fft_yz_batch,
+                     (const void *)k_fft_x_batch,  (const void *)k_fft_zy_batch};
+  for (const void *q : k)
+    PM_CUDA(cudaFuncSetAttribute(q, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+  return PMGPU_OK;
+}
+
+// Threads of a plane block: eight points of the plane each (one trip to
+// memory, about one butterfly a pass).
+static int fft_plane_threads(const FftGrid &g) {
+  return std::min(512, std::max(128, ((g.K1 * g.K2 / 8 + 31) / 32) * 32));
+}
+static int fft_x_blocks(const FftGrid &g) { return (g.K1 * g.Kh + g.cols - 1) / g.cols; }
+
+static FftArgs fft_args(const System *s, const Force *f, int em) {
+  return FftArgs{f->fft, f->d_grid_fixed, f->d_grid,
+                 ConvolveArgs{f->grid[0], f->grid[1], f->grid[2], s->box.e[0], s->box.e[1],
+                              s->box.e[2], f->alpha, f->d_influence, f->d_cgrid, s->d_acc, em}};
+}
+
 int pme_init(System *s, Force *f) {
   if (!s->box.periodic) return fail(PMGPU_ERR_UNSUPPORTED, "PME needs a periodic box");
   if (f->order < 2 || f->order > kMaxOrder)
@@ -456,9 +651,25 @@ int pme_init(System *s, Force *f) {
                             cudaMemcpyHostToDevice, s->stream));
     PM_CUDA(cudaStreamSynchronize(s->stream));
   }
-  // cuFFT plans without their own work area: one stream-ordered work area
-  // serves both (they run back to back on the system's stream).  A pair
-  // left by an ended system of the same grid is taken from the context
+  if (fft_plan(K0, K1, K2, &f->fft)) {
+    std::vector<float2> tw;
+    for (int a = 0; a < 3; a++)
+      for (int m = 0; m < f->grid[a]; m++) {
+        const double x = 2.0 * M_PI * m / f->grid[a];
+        tw.push_back(make_float2((float)std::cos(x), (float)-std::sin(x)));
+      }
+    PM_CHECK(dev_alloc(s, &f->d_twiddle, sizeof(float2) * tw.size()));
+    PM_CUDA(cudaMemcpyAsync(f->d_twiddle, tw.data(), sizeof(float2) * tw.size(),
+                            cudaMemcpyHostToDevice, s->stream));
+    PM_CUDA(cudaStreamSynchronize(s->stream));
+    f->fft.tw = f->d_twiddle;
+    PM_CHECK(fft_set_smem());
+    f->own_fft = 1;
+    return PMGPU_OK;
+  }
+  // other grids: cuFFT plans without their own work area: one stream-ordered
+  // work area serves both (they run back to back on the system's stream).  A
+  // pair left by an ended system of the same grid is taken from the context
   // first.
   size_t ws_r2c = 0, ws_c2r = 0;
   bool reused = false;
@@ -505,11 +716,13 @@ int pme_free(System *s, Force *f) {
   }
   f->plan_r2c = f->plan_c2r = 0;
   void *ptrs[] = {f->d_grid, f->d_grid_fixed, f->d_cgrid, f->d_influence, f->d_fft_work,
-                  f->d_ewtab};
+                  f->d_ewtab, f->d_twiddle};
   for (void *p : ptrs) dev_free(s, p);
   f->d_grid = nullptr; f->d_grid_fixed = nullptr; f->d_cgrid = nullptr;
   f->d_influence = nullptr;
   f->d_ewtab = nullptr;
+  f->d_twiddle = nullptr;
+  f->own_fft = 0;
   f->terms.ewtab = nullptr;
   f->d_fft_work = nullptr;
   return PMGPU_OK;
@@ -540,7 +753,7 @@ static void spread_gather(const PmeArgs &a, System *s, Force *f,
 }
 
 // em: 0 forces only, 1 + energy, 2 + energy and virial.
-int pme_reciprocal(System *s, Force *f, int em) {
+int pme_reciprocal(System *s, Force *f, int em, long long *launched) {
   int n = s->n;
   if (n == 0) return PMGPU_OK;
   PmeArgs a;
@@ -557,24 +770,34 @@ int pme_reciprocal(System *s, Force *f, int em) {
   a.phi = f->d_grid;
   a.force = s->d_force;
   int K0 = f->grid[0], K1 = f->grid[1], K2 = f->grid[2];
-  size_t nreal = (size_t)K0 * K1 * K2;
-  size_t ncplx = (size_t)K0 * K1 * (K2 / 2 + 1);
   // Atoms are spread and gathered in their own order: PME does not wait for
-  // the pair list's sort, so it runs beside the list work of a step.  The
-  // plans run on whichever stream this evaluation uses.
-  if (cufftSetStream(f->plan_r2c, s->stream) != CUFFT_SUCCESS ||
-      cufftSetStream(f->plan_c2r, s->stream) != CUFFT_SUCCESS)
-    return fail(PMGPU_ERR_CUDA, "cufftSetStream failed");
+  // the pair list's sort, so it runs beside the list work of a step.
   spread_gather(a, s, f, 0);
-  k_pme_fixed_to_float<<<(int)((nreal + 255) / 256), 256, 0, s->stream>>>(
-      GridConvArgs{(int)nreal, f->d_grid_fixed, f->d_grid});
-  if (cufftExecR2C(f->plan_r2c, f->d_grid, (cufftComplex *)f->d_cgrid) != CUFFT_SUCCESS)
-    return fail(PMGPU_ERR_CUDA, "cufftExecR2C failed");
-  k_pme_convolve<<<(int)((ncplx + 255) / 256), 256, 0, s->stream>>>(
-      ConvolveArgs{K0, K1, K2, s->box.e[0], s->box.e[1], s->box.e[2], f->alpha, f->d_influence,
-                   f->d_cgrid, s->d_acc, em});
-  if (cufftExecC2R(f->plan_c2r, (cufftComplex *)f->d_cgrid, f->d_grid) != CUFFT_SUCCESS)
-    return fail(PMGPU_ERR_CUDA, "cufftExecC2R failed");
+  if (f->own_fft) {
+    const FftArgs fa = fft_args(s, f, em);
+    const int T = fft_plane_threads(fa.g);
+    const size_t plane = fft_plane_smem(fa.g);
+    k_fft_yz<<<K0, T, plane, s->stream>>>(fa);
+    k_fft_x<<<fft_x_blocks(fa.g), kFftXThreads, fft_x_smem(fa.g), s->stream>>>(fa);
+    k_fft_zy<<<K0, T, plane, s->stream>>>(fa);
+    *launched += 5;
+  } else {
+    // the plans run on whichever stream this evaluation uses
+    if (cufftSetStream(f->plan_r2c, s->stream) != CUFFT_SUCCESS ||
+        cufftSetStream(f->plan_c2r, s->stream) != CUFFT_SUCCESS)
+      return fail(PMGPU_ERR_CUDA, "cufftSetStream failed");
+    const size_t nreal = (size_t)K0 * K1 * K2, ncplx = (size_t)K0 * K1 * (K2 / 2 + 1);
+    k_pme_fixed_to_float<<<(int)((nreal + 255) / 256), 256, 0, s->stream>>>(
+        GridConvArgs{(int)nreal, f->d_grid_fixed, f->d_grid});
+    if (cufftExecR2C(f->plan_r2c, f->d_grid, (cufftComplex *)f->d_cgrid) != CUFFT_SUCCESS)
+      return fail(PMGPU_ERR_CUDA, "cufftExecR2C failed");
+    k_pme_convolve<<<(int)((ncplx + 255) / 256), 256, 0, s->stream>>>(
+        ConvolveArgs{K0, K1, K2, s->box.e[0], s->box.e[1], s->box.e[2], f->alpha,
+                     f->d_influence, f->d_cgrid, s->d_acc, em});
+    if (cufftExecC2R(f->plan_c2r, (cufftComplex *)f->d_cgrid, f->d_grid) != CUFFT_SUCCESS)
+      return fail(PMGPU_ERR_CUDA, "cufftExecC2R failed");
+    *launched += 4;  // spread, conversion, convolution, gather (+ cuFFT's)
+  }
   spread_gather(a, s, f, 1);
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;
@@ -591,9 +814,10 @@ int ewald_correction(System *s, Force *f, int em) {
 
 // ---------------------------------------------------------------- batches
 // The PME chain and the Ewald correction of an ensemble's members as
-// batched launches.  Members whose grids have the same dimensions form a
-// bucket: their real and complex grids are slices of one buffer, and one
-// batched cuFFT plan pair transforms the bucket at once.
+// batched launches: the members' own FFTs share one launch per kernel.
+// Members whose grids need cuFFT form a bucket per grid size: their real
+// and complex grids are slices of one buffer, and one batched cuFFT plan
+// pair transforms the bucket at once.
 struct PmeBucket {
   int K[3];
   std::vector<int> members;
@@ -604,7 +828,11 @@ struct PmeBucket {
 struct PmeBatch {
   int order = 4;
   BatchTable<PmeArgs> atoms;  // spread and gather
-  BatchTable<GridConvArgs> conv;
+  BatchTable<FftArgs> yz, fx[2], zy;  // members with the own FFT
+  int plane_threads = 128;
+  size_t plane_smem = 0, x_smem = 0;
+  int sizes = 0;                      // distinct grid dimensions
+  BatchTable<GridConvArgs> conv;      // members with cuFFT
   BatchTable<ConvolveArgs> convolve[2];
   BatchTable<CorrectionArgs> corr[2];
   std::vector<PmeBucket> buckets;
@@ -636,7 +864,10 @@ void pme_batch_free(PmeBatch *b) {
   }
   b->atoms.release();
   b->conv.release();
+  b->yz.release();
+  b->zy.release();
   for (int e = 0; e < 2; e++) {
+    b->fx[e].release();
     b->convolve[e].release();
     b->corr[e].release();
   }
@@ -648,11 +879,16 @@ int pme_batch_build(PmeBatch *b, System *const *m, int n, Force *const *fs) {
   b->forces.assign(fs, fs + n);
   b->order = fs[0]->order;
   // buckets by grid dimensions
-  std::vector<int> bucket_of(n, -1);
+  std::vector<const Force *> seen;
   for (int k = 0; k < n; k++) {
     const Force *f = fs[k];
     if (f->order != b->order || !(f->ewald_flags & PMGPU_EWALD_RECIPROCAL))
       return fail(PMGPU_ERR_UNSUPPORTED, "ensemble members need one PME order");
+    const bool known = std::any_of(seen.begin(), seen.end(), [f](const Force *o) {
+      return o->grid[0] == f->grid[0] && o->grid[1] == f->grid[1] && o->grid[2] == f->grid[2];
+    });
+    if (!known) seen.push_back(f);
+    if (f->own_fft) continue;
     int found = -1;
     for (size_t q = 0; q < b->buckets.size(); q++)
       if (b->buckets[q].K[0] == f->grid[0] && b->buckets[q].K[1] == f->grid[1] &&
@@ -664,8 +900,8 @@ int pme_batch_build(PmeBatch *b, System *const *m, int n, Force *const *fs) {
       for (int a = 0; a < 3; a++) b->buckets[found].K[a] = f->grid[a];
     }
     b->buckets[found].members.push_back(k);
-    bucket_of[k] = found;
   }
+  b->sizes = (int)seen.size();
   for (auto &bk : b->buckets) {
     const int B = (int)bk.members.size();
     const size_t G = (size_t)bk.K[0] * bk.K[1] * bk.K[2];
@@ -692,7 +928,10 @@ int pme_batch_build(PmeBatch *b, System *const *m, int n, Force *const *fs) {
   // argument tables in member order
   b->atoms.clear();
   b->conv.clear();
+  b->yz.clear();
+  b->zy.clear();
   for (int e = 0; e < 2; e++) {
+    b->fx[e].clear();
     b->convolve[e].clear();
     b->corr[e].clear();
   }
@@ -714,14 +953,26 @@ int pme_batch_build(PmeBatch *b, System *const *m, int n, Force *const *fs) {
     a.phi = f->d_grid;
     a.force = s->d_force;
     b->atoms.add(a, (int)(((long long)s->n * L + 127) / 128));
-    const size_t nreal = (size_t)f->grid[0] * f->grid[1] * f->grid[2];
-    const size_t ncplx = (size_t)f->grid[0] * f->grid[1] * (f->grid[2] / 2 + 1);
-    b->conv.add(GridConvArgs{(int)nreal, f->d_grid_fixed, f->d_grid}, (int)((nreal + 255) / 256));
+    if (f->own_fft) {
+      const FftArgs fa = fft_args(s, f, 0);
+      b->yz.add(fa, f->grid[0]);
+      b->zy.add(fa, f->grid[0]);
+      for (int e = 0; e < 2; e++) b->fx[e].add(fft_args(s, f, e), fft_x_blocks(fa.g));
+      b->plane_threads = std::max(b->plane_threads, fft_plane_threads(fa.g));
+      b->plane_smem = std::max(b->plane_smem, fft_plane_smem(fa.g));
+      b->x_smem = std::max(b->x_smem, fft_x_smem(fa.g));
+    } else {
+      const size_t nreal = (size_t)f->grid[0] * f->grid[1] * f->grid[2];
+      const size_t ncplx = (size_t)f->grid[0] * f->grid[1] * (f->grid[2] / 2 + 1);
+      b->conv.add(GridConvArgs{(int)nreal, f->d_grid_fixed, f->d_grid},
+                  (int)((nreal + 255) / 256));
+      for (int e = 0; e < 2; e++)
+        b->convolve[e].add(ConvolveArgs{f->grid[0], f->grid[1], f->grid[2], s->box.e[0],
+                                        s->box.e[1], s->box.e[2], f->alpha, f->d_influence,
+                                        f->d_cgrid, s->d_acc, e},
+                           (int)((ncplx + 255) / 256));
+    }
     for (int e = 0; e < 2; e++) {
-      b->convolve[e].add(ConvolveArgs{f->grid[0], f->grid[1], f->grid[2], s->box.e[0],
-                                      s->box.e[1], s->box.e[2], f->alpha, f->d_influence,
-                                      f->d_cgrid, s->d_acc, e},
-                         (int)((ncplx + 255) / 256));
       b->corr[e].add(CorrectionArgs{s->box, s->n_excl, s->d_excl_pairs, s->d_pos, s->d_charge,
                                     f->alpha, s->coulomb_scaling, s->n, s->d_force, s->d_acc, e},
                      (s->n_excl + 127) / 128);
@@ -729,7 +980,10 @@ int pme_batch_build(PmeBatch *b, System *const *m, int n, Force *const *fs) {
   }
   PM_CUDA(b->atoms.upload());
   PM_CUDA(b->conv.upload());
+  PM_CUDA(b->yz.upload());
+  PM_CUDA(b->zy.upload());
   for (int e = 0; e < 2; e++) {
+    PM_CUDA(b->fx[e].upload());
     PM_CUDA(b->convolve[e].upload());
     PM_CUDA(b->corr[e].upload());
   }
@@ -764,27 +1018,40 @@ static void pme_batch_sg(PmeBatch *b, int gather, cudaStream_t st) {
 int pme_batch_reciprocal(PmeBatch *b, int em, cudaStream_t st, long long *launched) {
   const int nm = b->atoms.members();
   if (!nm) return PMGPU_OK;
-  *launched += 4;  // spread, fixed->float, convolve, gather (+ cuFFT's)
+  *launched += 2;  // spread, gather
   pme_batch_sg(b, 0, st);
-  k_pme_fixed_to_float_batch<<<b->conv.total(), 256, 0, st>>>(b->conv.d, b->conv.d_first, nm);
-  for (auto &bk : b->buckets) {
-    if (cufftSetStream(bk.r2c, st) != CUFFT_SUCCESS ||
-        cufftExecR2C(bk.r2c, bk.grid, (cufftComplex *)bk.cgrid) != CUFFT_SUCCESS)
-      return fail(PMGPU_ERR_CUDA, "batched cufftExecR2C failed");
+  if (b->yz.members()) {
+    BatchTable<FftArgs> &fx = b->fx[em ? 1 : 0];
+    k_fft_yz_batch<<<b->yz.total(), b->plane_threads, b->plane_smem, st>>>(b->yz.d, b->yz.d_first,
+                                                                           b->yz.members());
+    k_fft_x_batch<<<fx.total(), kFftXThreads, b->x_smem, st>>>(fx.d, fx.d_first, fx.members());
+    k_fft_zy_batch<<<b->zy.total(), b->plane_threads, b->plane_smem, st>>>(b->zy.d, b->zy.d_first,
+                                                                           b->zy.members());
+    *launched += 3;
   }
-  BatchTable<ConvolveArgs> &cv = b->convolve[em ? 1 : 0];
-  k_pme_convolve_batch<<<cv.total(), 256, 0, st>>>(cv.d, cv.d_first, nm);
-  for (auto &bk : b->buckets) {
-    if (cufftSetStream(bk.c2r, st) != CUFFT_SUCCESS ||
-        cufftExecC2R(bk.c2r, (cufftComplex *)bk.cgrid, bk.grid) != CUFFT_SUCCESS)
-      return fail(PMGPU_ERR_CUDA, "batched cufftExecC2R failed");
+  if (b->conv.members()) {
+    const int nc = b->conv.members();
+    k_pme_fixed_to_float_batch<<<b->conv.total(), 256, 0, st>>>(b->conv.d, b->conv.d_first, nc);
+    for (auto &bk : b->buckets) {
+      if (cufftSetStream(bk.r2c, st) != CUFFT_SUCCESS ||
+          cufftExecR2C(bk.r2c, bk.grid, (cufftComplex *)bk.cgrid) != CUFFT_SUCCESS)
+        return fail(PMGPU_ERR_CUDA, "batched cufftExecR2C failed");
+    }
+    BatchTable<ConvolveArgs> &cv = b->convolve[em ? 1 : 0];
+    k_pme_convolve_batch<<<cv.total(), 256, 0, st>>>(cv.d, cv.d_first, nc);
+    for (auto &bk : b->buckets) {
+      if (cufftSetStream(bk.c2r, st) != CUFFT_SUCCESS ||
+          cufftExecC2R(bk.c2r, (cufftComplex *)bk.cgrid, bk.grid) != CUFFT_SUCCESS)
+        return fail(PMGPU_ERR_CUDA, "batched cufftExecC2R failed");
+    }
+    *launched += 2;  // conversion, convolution (+ cuFFT's)
   }
   pme_batch_sg(b, 1, st);
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;
 }
 
-int pme_batch_buckets(const PmeBatch *b) { return (int)b->buckets.size(); }
+int pme_batch_buckets(const PmeBatch *b) { return b->sizes; }
 
 int pme_batch_correction(PmeBatch *b, int em, cudaStream_t st, long long *launched) {
   BatchTable<CorrectionArgs> &t = b->corr[em ? 1 : 0];
