@@ -53,13 +53,17 @@ __device__ __forceinline__ void bspline(float fr, float *th, float *dth) {
 #pragma unroll
       for (int k = 1; k < P; k++) dth[k] = m[k] - m[k - 1];
     }
+    // 1 / (n - 1) as an FP32 pair: the rounding of 1/3 alone would scale every
+    // charge on the grid by 3e-8 per axis and the energy by 1.8e-7
     const float div = 1.f / (float)(n - 1);
+    const float div_lo = (float)(1.0 / (double)(n - 1) - (double)div);
     float prev = 0.f;
 #pragma unroll
     for (int k = 0; k < n; k++) {
       float cur = k < n - 1 ? m[k] : 0.f;
       float x = fr + (float)k;
-      m[k] = div * (x * cur + ((float)n - x) * prev);
+      const float v = x * cur + ((float)n - x) * prev;
+      m[k] = div_lo != 0.f ? fmaf(v, div, v * div_lo) : div * v;
       prev = cur;
     }
   }
