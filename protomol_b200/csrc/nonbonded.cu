@@ -1255,7 +1255,9 @@ static void fill_pair_args(PairArgs<Real> &a, System *s, NeighborList *nl,
   a.pairbuf_cap = s->pairbuf_cap;
   a.paircount = s->d_paircount;
   a.count_pairs = s->count_pairs;
-  a.energy_only = 0;
+  const SwitchParams &ls = t.lj_sw, &cs = t.coul_sw;
+  a.same_sw = (t.mask & TERM_LJ) && (t.mask & TERM_COUL) && ls.modify && cs.modify &&
+              std::memcmp(&ls, &cs, sizeof(ls)) == 0;
 }
 
 // Compile-time switch kind of a term for the specialised force-only
@@ -1288,11 +1290,13 @@ static void launch_pairs_spec(PairArgs<Real> &a, cudaStream_t st, int mode) {
   const int T = kPairWarps * 32;
   const int nb = (int)(((long long)a.nclusters * a.splits + kPairWarps - 1) / kPairWarps);
   if (nb == 0) return;
-  switch (mode) {
-    case PAIR_FORCE: k_pairs<Real, TERMS, PAIR_FORCE, SPEC><<<nb, T, 0, st>>>(a); break;
-    case PAIR_ENERGY: k_pairs<Real, TERMS, PAIR_ENERGY, SPEC><<<nb, T, 0, st>>>(a); break;
-    case PAIR_VIRIAL: k_pairs<Real, TERMS, PAIR_VIRIAL, SPEC><<<nb, T, 0, st>>>(a); break;
-    default: k_pairs<Real, TERMS, PAIR_RECORD, SPEC><<<nb, T, 0, st>>>(a); break;
+  if (mode == PAIR_FORCE) {
+    k_pairs<Real, TERMS, PAIR_FORCE, SPEC><<<nb, T, 0, st>>>(a);
+  } else if (mode == PAIR_RECORD) {
+    k_pairs<Real, TERMS, PAIR_RECORD, SPEC><<<nb, T, 0, st>>>(a);
+  } else if constexpr (sizeof(Real) == 8) {  // mixed precision: launch_e64
+    if (mode == PAIR_ENERGY) k_pairs<Real, TERMS, PAIR_ENERGY, SPEC><<<nb, T, 0, st>>>(a);
+    else k_pairs<Real, TERMS, PAIR_VIRIAL, SPEC><<<nb, T, 0, st>>>(a);
   }
 }
 
@@ -1343,27 +1347,84 @@ static void launch_force_spec(PairArgs<Real> &a, cudaStream_t st) {
   }
 }
 
+// The specialised force-only form of a launch's terms (every term with one
+// cutoff, box edges at least twice the cutoff), or PMGPU_PAIRK_GENERIC.
+template <typename Real>
+static int special_form(const PairArgs<Real> &a, const PairTerms &t) {
+  if (sizeof(Real) != 4 || !a.same_cut || a.minimal_image) return PMGPU_PAIRK_GENERIC;
+  const int lk = spec_kind(t.lj_sw), ck = spec_kind(t.coul_sw);
+  if (t.mask == (TERM_LJ | TERM_EWALD) && !t.exact_erf && lk == PMGPU_SW_C2)
+    return PMGPU_PAIRK_LJC2_EWALD;
+  if (t.mask == (TERM_LJ | TERM_COUL) && lk == PMGPU_SW_C2 && ck == PMGPU_SW_C2)
+    return PMGPU_PAIRK_LJC2_COULC2;
+  if (t.mask == (TERM_LJ | TERM_COUL) && lk == PMGPU_SW_C2 && ck == PMGPU_SW_C1)
+    return PMGPU_PAIRK_LJC2_COULC1;
+  return PMGPU_PAIRK_GENERIC;
+}
+
+// The instantiation of the FP64 energy kernel for a launch's terms, given
+// to go: compiled switch kinds for the specialised forms, run-time switches
+// for the others.
+template <bool VIRIAL, typename F>
+static void e64_kernel(int mask, int form, F go) {
+  constexpr int LC = TERM_LJ | TERM_COUL, LE = TERM_LJ | TERM_EWALD;
+  constexpr int C2 = PMGPU_SW_C2, C1 = PMGPU_SW_C1;
+  if (form == PMGPU_PAIRK_LJC2_EWALD)
+    go(k_pairs_e64<LE, VIRIAL, C2, -1>, k_pairs_e64_batch<LE, VIRIAL, C2, -1>);
+  else if (form == PMGPU_PAIRK_LJC2_COULC2)
+    go(k_pairs_e64<LC, VIRIAL, C2, C2>, k_pairs_e64_batch<LC, VIRIAL, C2, C2>);
+  else if (form == PMGPU_PAIRK_LJC2_COULC1)
+    go(k_pairs_e64<LC, VIRIAL, C2, C1>, k_pairs_e64_batch<LC, VIRIAL, C2, C1>);
+  else if (mask == TERM_LJ)
+    go(k_pairs_e64<TERM_LJ, VIRIAL, -1, -1>, k_pairs_e64_batch<TERM_LJ, VIRIAL, -1, -1>);
+  else if (mask == TERM_COUL)
+    go(k_pairs_e64<TERM_COUL, VIRIAL, -1, -1>, k_pairs_e64_batch<TERM_COUL, VIRIAL, -1, -1>);
+  else if (mask == LC)
+    go(k_pairs_e64<LC, VIRIAL, -1, -1>, k_pairs_e64_batch<LC, VIRIAL, -1, -1>);
+  else if (mask == TERM_EWALD)
+    go(k_pairs_e64<TERM_EWALD, VIRIAL, -1, -1>, k_pairs_e64_batch<TERM_EWALD, VIRIAL, -1, -1>);
+  else
+    go(k_pairs_e64<LE, VIRIAL, -1, -1>, k_pairs_e64_batch<LE, VIRIAL, -1, -1>);
+}
+
+// The energy launch's shape: work items as the force-only kernel's.
+static int e64_blocks(const PairArgs<float> &a) {
+  return (int)(((long long)a.nclusters * a.splits + kE64Warps - 1) / kE64Warps);
+}
+template <bool VIRIAL>
+static size_t e64_smem_bytes() { return kE64Warps * sizeof(E64Warp<VIRIAL>); }
+template <bool VIRIAL, typename K>
+static cudaError_t e64_raise_smem(K kern) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)e64_smem_bytes<VIRIAL>());
+}
+
+template <bool VIRIAL>
+static cudaError_t launch_e64(PairArgs<float> a, int form, cudaStream_t st) {
+  a.splits = jl_splits(a.nclusters);
+  const int nb = e64_blocks(a);
+  cudaError_t err = cudaSuccess;
+  if (nb)
+    e64_kernel<VIRIAL>(a.mask, form, [&](auto kern, auto) {
+      err = e64_raise_smem<VIRIAL>(kern);
+      if (err == cudaSuccess)
+        kern<<<nb, kE64Warps * 32, e64_smem_bytes<VIRIAL>(), st>>>(a);
+    });
+  return err;
+}
+
 // Returns the form launched: PMGPU_PAIRK_GENERIC or one of the specialised
 // force-only forms (PMGPU_PAIRK_*).
 template <typename Real, int TERMS>
 static int launch_pairs_t(PairArgs<Real> &a, cudaStream_t st, int mode, const PairTerms &t) {
-  // specialised force-only FP32 kernels of the common configurations
-  // (every term with one cutoff, box edges at least twice the cutoff)
-  if (sizeof(Real) == 4 && mode != PAIR_RECORD && a.same_cut && !a.minimal_image) {
-    const int lk = spec_kind(t.lj_sw), ck = spec_kind(t.coul_sw);
-    int form = PMGPU_PAIRK_GENERIC;
-    if (TERMS == (TERM_LJ | TERM_EWALD) && !t.exact_erf && lk == PMGPU_SW_C2)
-      form = PMGPU_PAIRK_LJC2_EWALD;
-    else if (TERMS == (TERM_LJ | TERM_COUL) && lk == PMGPU_SW_C2 && ck == PMGPU_SW_C2)
-      form = PMGPU_PAIRK_LJC2_COULC2;
-    else if (TERMS == (TERM_LJ | TERM_COUL) && lk == PMGPU_SW_C2 && ck == PMGPU_SW_C1)
-      form = PMGPU_PAIRK_LJC2_COULC1;
-    if (form != PMGPU_PAIRK_GENERIC) {
-      // The forces of every mode come from the specialised kernel, so an
+  if constexpr (sizeof(Real) == 4) {
+    if (mode != PAIR_RECORD) {
+      // The forces of every mode come from the force-only kernels, so an
       // energy step's forces equal a force-only step's bit for bit (a run
       // split into several calls, whose energy steps fall elsewhere, gives
-      // the same trajectory); energies and virial then come from the
-      // generic kernel in its energy-only form.
+      // the same trajectory); energies and virial then come from the FP64
+      // energy kernel.
+      const int form = special_form(a, t);
       PairArgs<Real> fa = a;
       if (mode != PAIR_FORCE) fa.count_pairs = 0;  // the energy pass counts
       if (form == PMGPU_PAIRK_LJC2_EWALD)
@@ -1371,14 +1432,14 @@ static int launch_pairs_t(PairArgs<Real> &a, cudaStream_t st, int mode, const Pa
       else if (form == PMGPU_PAIRK_LJC2_COULC2)
         launch_force_spec<Real, TERM_LJ | TERM_COUL, PairSpec<PMGPU_SW_C2, PMGPU_SW_C2, -1>>(fa,
                                                                                           st);
-      else
+      else if (form == PMGPU_PAIRK_LJC2_COULC1)
         launch_force_spec<Real, TERM_LJ | TERM_COUL, PairSpec<PMGPU_SW_C2, PMGPU_SW_C1, -1>>(fa,
                                                                                           st);
-      if (mode != PAIR_FORCE) {
-        PairArgs<Real> ea = a;
-        ea.energy_only = 1;
-        launch_pairs_spec<Real, TERMS, GenericSpec>(ea, st, mode);
-      }
+      else
+        launch_pairs_spec<Real, TERMS, GenericSpec>(fa, st, PAIR_FORCE);
+      // (a failed launch is found by the caller's cudaGetLastError)
+      if (mode == PAIR_ENERGY) (void)launch_e64<false>(a, form, st);
+      if (mode == PAIR_VIRIAL) (void)launch_e64<true>(a, form, st);
       return form;
     }
   }
@@ -1459,7 +1520,7 @@ struct NbBatch {
   int tab = 1;                         // every jl member has the Ewald force table
   BatchTable<PairArgs<float>> jl;      // members with the specialised force-only form
   BatchTable<PairArgs<float>> gforce;  // members without one (force-only, generic kernel)
-  BatchTable<PairArgs<float>> energy;  // every member on energy steps
+  BatchTable<PairArgs<float>> energy, genergy;  // on energy steps: the jl members, the others
   BatchTable<SlotArgs> slots;
   std::vector<int> has_form;           // per member: 1 if in jl
   std::vector<PairArgs<float>> base;   // per member: its force-only pair arguments
@@ -1471,22 +1532,8 @@ void nb_batch_free(NbBatch *b) {
   if (!b) return;
   b->bin.release(); b->sort.release();
   b->gather.release(); b->build.release(); b->jl.release(); b->gforce.release();
-  b->energy.release(); b->slots.release(); b->probe.release();
+  b->energy.release(); b->genergy.release(); b->slots.release(); b->probe.release();
   delete b;
-}
-
-// The specialised force-only form a member's pair launch takes
-// (launch_pairs_t), or PMGPU_PAIRK_GENERIC.
-static int special_form(const PairArgs<float> &a, const PairTerms &t) {
-  if (!a.same_cut || a.minimal_image) return PMGPU_PAIRK_GENERIC;
-  const int lk = spec_kind(t.lj_sw), ck = spec_kind(t.coul_sw);
-  if (t.mask == (TERM_LJ | TERM_EWALD) && !t.exact_erf && lk == PMGPU_SW_C2)
-    return PMGPU_PAIRK_LJC2_EWALD;
-  if (t.mask == (TERM_LJ | TERM_COUL) && lk == PMGPU_SW_C2 && ck == PMGPU_SW_C2)
-    return PMGPU_PAIRK_LJC2_COULC2;
-  if (t.mask == (TERM_LJ | TERM_COUL) && lk == PMGPU_SW_C2 && ck == PMGPU_SW_C1)
-    return PMGPU_PAIRK_LJC2_COULC1;
-  return PMGPU_PAIRK_GENERIC;
 }
 
 // splits[k] > 0 sets member k's jl splits (the tiles of each i cluster
@@ -1499,7 +1546,8 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
                    cudaSuccess || sms <= 0))
     sms = 148;
   b->bin.clear(); b->sort.clear(); b->gather.clear();
-  b->build.clear(); b->jl.clear(); b->gforce.clear(); b->energy.clear(); b->slots.clear();
+  b->build.clear(); b->jl.clear(); b->gforce.clear(); b->energy.clear();
+  b->genergy.clear(); b->slots.clear();
   b->has_form.assign(n, 0);
   b->base.assign(n, PairArgs<float>());
   b->terms = terms[0].mask;
@@ -1539,13 +1587,15 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
     } else {
       b->gforce.add(a, (int)(((long long)a.nclusters * a.splits + kPairWarps - 1) / kPairWarps));
     }
+    // the energy kernel of a special form compiles its switches in, so the
+    // members without one take a table of their own
     PairArgs<float> ea = a;
-    ea.energy_only = form != PMGPU_PAIRK_GENERIC;
-    b->energy.add(ea, (int)(((long long)a.nclusters * a.splits + kPairWarps - 1) / kPairWarps));
+    ea.splits = jl_splits(a.nclusters);
+    (form != PMGPU_PAIRK_GENERIC ? b->energy : b->genergy).add(ea, e64_blocks(ea));
     b->slots.add(SlotArgs{nl->ns_max, s->n, nl->d_sorted, nl->d_fslot, s->d_force},
                  (nl->ns_max + 255) / 256);
   }
-  BatchTable<PairArgs<float>> *pt[] = {&b->jl, &b->gforce, &b->energy};
+  BatchTable<PairArgs<float>> *pt[] = {&b->jl, &b->gforce, &b->energy, &b->genergy};
   PM_CUDA(b->bin.upload());
   PM_CUDA(b->sort.upload());
   PM_CUDA(b->gather.upload());
@@ -1572,26 +1622,32 @@ int nb_batch_list(NbBatch *b, cudaStream_t st, long long *launched) {
 }
 
 template <int TERMS>
-static int launch_generic_batch(BatchTable<PairArgs<float>> &t, int mode, cudaStream_t st) {
+static int launch_generic_batch(BatchTable<PairArgs<float>> &t, cudaStream_t st) {
   if (!t.members() || !t.total()) return 0;
-  const int T = kPairWarps * 32;
-  if (mode == PAIR_FORCE)
-    k_pairs_batch<float, TERMS, PAIR_FORCE, GenericSpec><<<t.total(), T, 0, st>>>(t.d, t.d_first,
-                                                                                   t.members());
-  else
-    k_pairs_batch<float, TERMS, PAIR_ENERGY, GenericSpec><<<t.total(), T, 0, st>>>(
-        t.d, t.d_first, t.members());
+  k_pairs_batch<float, TERMS, PAIR_FORCE, GenericSpec>
+      <<<t.total(), kPairWarps * 32, 0, st>>>(t.d, t.d_first, t.members());
   return 1;
 }
 
-static int generic_batch(BatchTable<PairArgs<float>> &t, int terms, int mode, cudaStream_t st) {
+static int generic_batch(BatchTable<PairArgs<float>> &t, int terms, cudaStream_t st) {
   switch (terms) {
-    case TERM_LJ: return launch_generic_batch<TERM_LJ>(t, mode, st);
-    case TERM_COUL: return launch_generic_batch<TERM_COUL>(t, mode, st);
-    case TERM_LJ | TERM_COUL: return launch_generic_batch<TERM_LJ | TERM_COUL>(t, mode, st);
-    case TERM_EWALD: return launch_generic_batch<TERM_EWALD>(t, mode, st);
-    default: return launch_generic_batch<TERM_LJ | TERM_EWALD>(t, mode, st);
+    case TERM_LJ: return launch_generic_batch<TERM_LJ>(t, st);
+    case TERM_COUL: return launch_generic_batch<TERM_COUL>(t, st);
+    case TERM_LJ | TERM_COUL: return launch_generic_batch<TERM_LJ | TERM_COUL>(t, st);
+    case TERM_EWALD: return launch_generic_batch<TERM_EWALD>(t, st);
+    default: return launch_generic_batch<TERM_LJ | TERM_EWALD>(t, st);
   }
+}
+
+// The energy launch of the table's members (all of one form).
+static int e64_batch(BatchTable<PairArgs<float>> &t, int terms, int form, cudaStream_t st) {
+  if (!t.members() || !t.total()) return 0;
+  e64_kernel<false>(terms, form, [&](auto, auto kern) {
+    if (e64_raise_smem<false>(kern) == cudaSuccess)
+      kern<<<t.total(), kE64Warps * 32, e64_smem_bytes<false>(), st>>>(t.d, t.d_first,
+                                                                       t.members());
+  });
+  return 1;
 }
 
 template <int TERMS, typename SPEC>
@@ -1629,10 +1685,10 @@ static int jl_form(NbBatch *b, BatchTable<PairArgs<float>> &t, cudaStream_t st) 
 
 int nb_batch_pairs(NbBatch *b, int mode, cudaStream_t st, long long *launched) {
   *launched += jl_form(b, b->jl, st);
-  if (mode == PAIR_FORCE) {
-    *launched += generic_batch(b->gforce, b->terms, PAIR_FORCE, st);
-  } else {
-    *launched += generic_batch(b->energy, b->terms, PAIR_ENERGY, st);
+  *launched += generic_batch(b->gforce, b->terms, st);
+  if (mode != PAIR_FORCE) {
+    *launched += e64_batch(b->energy, b->terms, b->form, st);
+    *launched += e64_batch(b->genergy, b->terms, PMGPU_PAIRK_GENERIC, st);
     if (b->slots.total()) {
       k_slot_forces_batch<<<b->slots.total(), 256, 0, st>>>(b->slots.d, b->slots.d_first,
                                                            b->slots.members());

@@ -12,7 +12,8 @@
 //     FP64 arithmetic, so the accepted pair set is the reference's;
 //   * energies and virial: only when requested (ProtoMol's energies are
 //     observed at output steps), and then in FP64 from the FP64 wrapped
-//     coordinates, because FP32 rounding of large cancelling pair energies
+//     coordinates (in mixed precision by a kernel of their own,
+//     k_pairs_e64), because FP32 rounding of large cancelling pair energies
 //     alone leaves a relative error near 1e-5 on the Ewald real-space sum;
 //   * Cn switching: its polynomial in (r - rc) has large alternating
 //     coefficients (switch/CnSwitchingFunction.cpp:9-23), so it is evaluated
@@ -68,8 +69,7 @@ struct PairArgs {
   long long pairbuf_cap;
   long long *paircount;
   int count_pairs;       // accumulate the accepted-pair count
-  int energy_only;       // energies (and virial) only: the forces come from the
-                         // force-only kernel launched beside
+  int same_sw;           // both cutoff terms take one switch (the same constants)
 };
 
 // Exact FP64 squared distance of the image in hand, formed the way the
@@ -95,11 +95,17 @@ __device__ __forceinline__ double exact_r2(const PairArgs<Real> &a, int oi, int 
 __device__ __forceinline__ float fast_exp(float x) { return __expf(x); }
 __device__ __forceinline__ double fast_exp(double x) { return exp(x); }
 
+// Value and derivative of a run-time switch; sv and sd keep them for a
+// second term under the same switch (known = 1).
 template <typename Real>
 __device__ __forceinline__ void apply_switch(const SwitchDev<Real> &sw,
                                              const SwitchDev<double> &sw64, Real r2,
-                                             Real &ff, Real &en) {
-  Real sv, sd;
+                                             Real &ff, Real &en, Real &sv, Real &sd, int known) {
+  if (known) {
+    ff = ff * sv - en * sd;
+    en = en * sv;
+    return;
+  }
   // the Cn and CmpCnCn polynomials cancel in FP32: evaluated in FP64
   if (sizeof(Real) == 4 && (sw.kind == PMGPU_SW_CN || sw.kind == PMGPU_SW_CMPCNCN)) {
     double v64, d64;
@@ -126,9 +132,10 @@ using GenericSpec = PairSpec<-1, -1, -1>;
 
 template <typename Real, int KIND>
 __device__ __forceinline__ void switch_k(const SwitchDev<Real> &sw, const SwitchDev<double> &sw64,
-                                         int modify, Real r2, Real &ff, Real &en) {
+                                         int modify, Real r2, Real &ff, Real &en, Real &sv,
+                                         Real &sd, int known) {
   if (KIND < 0) {
-    if (modify) apply_switch<Real>(sw, sw64, r2, ff, en);
+    if (modify) apply_switch<Real>(sw, sw64, r2, ff, en, sv, sd, known);
   } else if (KIND == PMGPU_SW_C2) {
     // C2SwitchingFunction::operator() (switch/C2SwitchingFunction.h:42-52)
     if (r2 > sw.cutoff2) {
@@ -164,7 +171,8 @@ __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *
   const bool modified = flags & kQModified;
   const Real rinv = rsqrt_nr(r2);
   const Real rinv2 = rinv * rinv;
-  Real f = 0;
+  Real f = 0, sv = 1, sd = 0;
+  int known = 0;
   if ((TERMS & TERM_LJ) && (flags & kQLJ)) {
     Real A, B;
     if (sizeof(Real) == 4) {
@@ -182,7 +190,8 @@ __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *
     Real r12A = A * r6 * r6;
     Real en = r12A - r6B;
     Real ff = (Real(12) * r12A - Real(6) * r6B) * rinv2;
-    switch_k<Real, SPEC::lj>(a.lj_sw, a.lj_sw64, a.lj_modify, r2, ff, en);
+    switch_k<Real, SPEC::lj>(a.lj_sw, a.lj_sw64, a.lj_modify, r2, ff, en, sv, sd, 0);
+    known = a.same_sw;
     en_lj += en;
     f += ff;
   }
@@ -191,7 +200,7 @@ __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *
     // CoulombForce::operator() (force/CoulombForce.h:29-40)
     Real en = qq * rinv;
     Real ff = en * rinv2;
-    switch_k<Real, SPEC::coul>(a.coul_sw, a.coul_sw64, a.coul_modify, r2, ff, en);
+    switch_k<Real, SPEC::coul>(a.coul_sw, a.coul_sw64, a.coul_modify, r2, ff, en, sv, sd, known);
     en_c += en;
     f += ff;
   }
@@ -309,67 +318,6 @@ __device__ __forceinline__ Real pair_force_fast(const PairArgs<Real> &a, const R
   return pair_force_p<Real, TERMS, SPEC, MOD>(a, p, r2, qq, modified);
 }
 
-// FP64 energies (and, for the virial, the FP64 pair force) of one accepted
-// pair from the FP64 wrapped coordinates: the observables of output steps
-// in the mixed-precision path.
-template <typename Real, int TERMS, bool FORCE64>
-__device__ __forceinline__ void pair_energy64(const PairArgs<Real> &a, const double4 &wi,
-                                              const double4 &wj, int shift, int ti, int tj,
-                                              int flags, double &Elj, double &Ec,
-                                              double *V) {
-  const int sx = (shift & 3) - 1, sy = ((shift >> 2) & 3) - 1, sz = ((shift >> 4) & 3) - 1;
-  double ex = wj.x - (wi.x - sx * a.box.e[0]);
-  double ey = wj.y - (wi.y - sy * a.box.e[1]);
-  double ez = wj.z - (wi.z - sz * a.box.e[2]);
-  double r2e = ex * ex + ey * ey + ez * ez;
-  double rr2 = 1.0 / r2e;
-  double f = 0.0;
-  const bool modified = flags & kQModified;
-  if ((TERMS & TERM_LJ) && (flags & kQLJ)) {
-    double4 p = a.lj64[ti * a.ntypes + tj];
-    double A = modified ? p.z : p.x;
-    double B = modified ? p.w : p.y;
-    double r6 = rr2 * rr2 * rr2;
-    double en = A * r6 * r6 - B * r6;
-    double ff = FORCE64 ? (12.0 * A * r6 * r6 - 6.0 * B * r6) * rr2 : 0.0;
-    if (a.lj_modify) {
-      double sv, sd;
-      switch_eval<double>(a.lj_sw64, r2e, sv, sd);
-      ff = ff * sv - en * sd;
-      en *= sv;
-    }
-    Elj += en;
-    f += ff;
-  }
-  double qq = wi.w * wj.w;
-  if (modified) qq *= a.csf64;
-  if ((TERMS & TERM_COUL) && (flags & kQCoul)) {
-    double en = qq * sqrt(rr2);
-    double ff = en * rr2;
-    if (a.coul_modify) {
-      double sv, sd;
-      switch_eval<double>(a.coul_sw64, r2e, sv, sd);
-      ff = ff * sv - en * sd;
-      en *= sv;
-    }
-    Ec += en;
-    f += ff;
-  }
-  if ((TERMS & TERM_EWALD) && (flags & kQEwald)) {
-    double r = sqrt(r2e);
-    double ar = a.alpha64 * r;
-    double ee = qq * exp(-ar * ar);
-    double en = !a.exact_erf ? poly5<double>(ar) * ee / r : qq * erfc(ar) / r;
-    Ec += en;
-    f += (en + a.a2pi64 * ee) * rr2;
-  }
-  if (FORCE64) {
-    // addVirial(fij, d) with fij = d * f (each pair is listed once)
-    V[0] += ex * ex * f; V[1] += ex * ey * f; V[2] += ex * ez * f;
-    V[3] += ey * ey * f; V[4] += ey * ez * f; V[5] += ez * ez * f;
-  }
-}
-
 // Registers: the specialised force-only FP32 kernels (the inner MD steps)
 // are held to 48 so five blocks fit per SM, the generic force-only FP32
 // kernel to 64; energy/virial/record and FP64 variants get more.
@@ -416,8 +364,9 @@ __device__ __forceinline__ long long fixed_force(double v) { return to_fixed(v, 
 template <typename Real, int TERMS, int MODE, typename SPEC>
 __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   constexpr bool MIXED = sizeof(Real) == 4;
-  constexpr bool ENERGY = MODE != PAIR_FORCE;
-  constexpr bool VIRIAL = MODE == PAIR_VIRIAL;
+  // (in mixed precision energies come from k_pairs_e64)
+  constexpr bool ENERGY = !MIXED && (MODE == PAIR_ENERGY || MODE == PAIR_VIRIAL);
+  constexpr bool VIRIAL = !MIXED && MODE == PAIR_VIRIAL;
   constexpr bool RECORD = MODE == PAIR_RECORD;
   // force-only kernels of a specialised configuration (launched only when
   // every term shares one cutoff and the box holds twice the cutoff): every
@@ -430,7 +379,6 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   const unsigned jbyte = 0xFFu << (8 * jl);   // the 8 lanes of this lane's j atom
   const bool jcomp = il < 3;                  // lane adds j's force component il
   double Elj = 0, Ec = 0;
-  double V64[6] = {0, 0, 0, 0, 0, 0};
   Real vxx = 0, vxy = 0, vxz = 0, vyy = 0, vyz = 0, vzz = 0;
   int npairs = 0;
   // work items (i cluster, share of its tiles); the warps of a smaller
@@ -449,7 +397,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   if (t1 <= t0) continue;
   const int islot = 8 * ci + il;
   const int oi = a.sorted[islot];
-  const double4 wi = a.xw[islot];  // energy modes and the FP64 kernel only
+  const double4 wi = a.xw[islot];  // the FP64 kernel only
   Real xi_h[3], xi_l[3];
   Real qi;
   int ti;
@@ -594,34 +542,23 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
           fabs(dz) <= a.half_edge[2]))
       flags &= ~(kQLJ | kQCoul);
     Real jx = 0, jy = 0, jz = 0;
-    // an energy-only pass (the forces of the step come from the force-only
-    // kernel) skips the FP32 force and the j-force sums
-    const bool forces = !(MIXED && ENERGY && a.energy_only);
     if (flags) {
       if ((tile.z >> lane) & 1u) flags |= kQModified;
       if (!MIXED) tj = a.type[a.sorted[jslot]];
       Real en_lj = 0, en_c = 0;
-      if (forces) {
-        const Real f =
-            pair_force<Real, TERMS, SPEC>(a, ljrow, r2, qi * qj, tj, flags, en_lj, en_c);
-        jx = dx * f;
-        jy = dy * f;
-        jz = dz * f;
-        fx -= jx;
-        fy -= jy;
-        fz -= jz;
-      }
+      const Real f = pair_force<Real, TERMS, SPEC>(a, ljrow, r2, qi * qj, tj, flags, en_lj, en_c);
+      jx = dx * f;
+      jy = dy * f;
+      jz = dz * f;
+      fx -= jx;
+      fy -= jy;
+      fz -= jz;
       npairs++;
       if (ENERGY) {
-        if (MIXED) {
-          pair_energy64<Real, TERMS, VIRIAL>(a, wi, a.xw[jslot], sh, ti, tj, flags, Elj, Ec,
-                                             V64);
-        } else {
-          Elj += (double)en_lj;
-          Ec += (double)en_c;
-        }
+        Elj += (double)en_lj;
+        Ec += (double)en_c;
       }
-      if (VIRIAL && !MIXED) {
+      if (VIRIAL) {
         // addVirial(fij, d) with fij = d * f
         vxx += dx * jx; vxy += dx * jy; vxz += dx * jz;
         vyy += dy * jy; vyz += dy * jz; vzz += dz * jz;
@@ -636,7 +573,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
       }
     }
     // j's share: summed over its 8 lanes, one atomic per component
-    if (forces) {
+    {
       const unsigned act = __ballot_sync(kAll, flags != 0);
       const Real js = group8_sum3<Real>(jx, jy, jz, lane);
       long long *dst = a.fslot + il * a.ns + jslot;
@@ -659,7 +596,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
     fy += __shfl_xor_sync(kAll, fy, o);
     fz += __shfl_xor_sync(kAll, fz, o);
   }
-  if (jl == 0 && oi >= 0 && !a.energy_only) {
+  if (jl == 0 && oi >= 0) {
     red_add(&a.fslot[islot], fixed_force(fx));
     red_add(&a.fslot[a.ns + islot], fixed_force(fy));
     red_add(&a.fslot[2 * a.ns + islot], fixed_force(fz));
@@ -674,13 +611,9 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
     double dc = warp_sum(Ec);
     double V[6] = {0, 0, 0, 0, 0, 0};
     if (VIRIAL) {
-      if (MIXED) {
-        for (int q = 0; q < 6; q++) V[q] = warp_sum(V64[q]);
-      } else {
-        V[0] = warp_sum((double)vxx); V[1] = warp_sum((double)vxy);
-        V[2] = warp_sum((double)vxz); V[3] = warp_sum((double)vyy);
-        V[4] = warp_sum((double)vyz); V[5] = warp_sum((double)vzz);
-      }
+      V[0] = warp_sum((double)vxx); V[1] = warp_sum((double)vxy);
+      V[2] = warp_sum((double)vxz); V[3] = warp_sum((double)vyy);
+      V[4] = warp_sum((double)vyz); V[5] = warp_sum((double)vzz);
     }
     if (lane == 0) {
       if (TERMS & TERM_LJ) red_add(&a.acc[ACC_LJ], to_fixed(dlj, kEnergyScale));
@@ -970,6 +903,309 @@ __global__ void __launch_bounds__(kJlWarps * 32, 3)
   const int m = batch_member(first, nm, blockIdx.x);
   pairs_jl_body<TERMS, SPEC, SMEM_LJ, TAB>(batch_args_shared(tab, m, raw),
                                            batch_blk(first, m));
+}
+
+// ---------------------------------------------------------------------------
+// FP64 energies (and virial) of the mixed-precision path, j atoms on the
+// lanes, accepted pairs compacted.
+//
+// A warp takes an (i cluster, share of its j-lane entries) item as
+// k_pairs_jl does.  Per 32 entries each lane tests its j atom against the
+// cluster's 8 i atoms (FP64 squared distances, the reference's exact test
+// within a rounding band of a cutoff) and appends the accepted pairs to the
+// warp's queue in shared memory; whole batches of 32 queued pairs are then
+// evaluated, one per lane.  A third of the tested pairs lie inside the
+// cutoff, so the FP64 terms (a square root, an exponential, the switches)
+// run on full warps instead of a third of their lanes, and the reciprocal
+// and the square root share one Newton iteration.  FP64 issue bounds the
+// kernel.  Against one pair per lane of a tile with run-time switches:
+// 49,998 atoms, LJ C2 + Ewald, energies: 488 -> 160 us; 648 atoms, LJ C2 +
+// Coulomb C1: 37 -> 12 us; 12,000 atoms, Cn at 10 A, energies and virial:
+// 650 us with the forces -> 146 us, and 119 us for the forces.
+constexpr int kE64Warps = 8;
+constexpr int kE64Queue = 32 + 256;  // pairs left over + pairs of one warp step
+template <bool VIRIAL>
+struct E64Queue {
+  double r2[kE64Queue], qq[kE64Queue];
+  double d[VIRIAL ? 3 : 1][VIRIAL ? kE64Queue : 1];
+  uint2 code[kE64Queue];  // LJ table index; kQ* flags
+};
+template <bool VIRIAL>
+struct E64Warp {
+  E64Queue<VIRIAL> q;
+  double4 wi[8];  // the cluster's atoms
+  int ti[8], oi[8];
+};
+
+// 1 / sqrt(x) in FP64: the hardware's 20-bit estimate and two Newton steps
+// y += y (1 - x y^2) / 2, each of which doubles the correct bits; within two
+// units in the last place for normal x.
+__device__ __forceinline__ double rsqrt_newton(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  double e = fma(-x * y, y, 1.0);
+  y = fma(0.5 * y, e, y);
+  e = fma(-x * y, y, 1.0);
+  return fma(0.5 * y, e, y);
+}
+// 1 / x the same way, y += y (1 - x y).
+__device__ __forceinline__ double rcp_newton(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  y = fma(y, fma(-x, y, 1.0), y);
+  return fma(y, fma(-x, y, 1.0), y);
+}
+
+// Value and, when DER, derivative over the distance of switch KIND at an
+// accepted pair (r2 within the cutoff), 1/r at hand.
+template <int KIND, bool DER>
+__device__ __forceinline__ void switch64(const SwitchDev<double> &w, double r2, double rinv,
+                                         double &val, double &der) {
+  der = 0.0;
+  val = 1.0;
+  if (KIND == PMGPU_SW_C2) {
+    if (r2 >= w.switchon2) {
+      const double c2 = w.cutoff2 - r2, c4 = c2 * (w.s2 + 2.0 * r2);
+      val = w.s1 * (c2 * c4);
+      if (DER) der = w.s3 * (c2 * c2 - c4);
+    }
+  } else if (KIND == PMGPU_SW_C1) {
+    const double d = r2 * rinv;
+    val = 1.0 - d * (w.c1a - r2 * w.c1b);
+    if (DER) der = -w.c1a * rinv + d * w.c1c;
+  } else if (KIND < 0) {
+    switch_eval<double>(w, r2, val, der);
+  }
+}
+
+template <int TERMS, bool VIRIAL, int LJK, int CK>
+__device__ __forceinline__ void pairs_e64_body(const PairArgs<float> &a, Blk blk,
+                                               E64Warp<VIRIAL> *warps) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  E64Warp<VIRIAL> &W = warps[wib];
+  constexpr int kAllTerms = ((TERMS & TERM_LJ) ? kQLJ : 0) | ((TERMS & TERM_COUL) ? kQCoul : 0) |
+                            ((TERMS & TERM_EWALD) ? kQEwald : 0);
+  constexpr double kBand = 1.0e-12;  // of a squared distance formed in FP64
+  double Elj = 0, Ec = 0, V[6] = {0, 0, 0, 0, 0, 0};
+  int npairs = 0, queued = 0;  // (queued: the same in every lane)
+
+  // energies of the queued pair k
+  auto evaluate = [&](int k) {
+    const double r2 = W.q.r2[k];
+    double qq = W.q.qq[k];
+    const uint2 code = W.q.code[k];
+    const bool modified = code.y & kQModified;
+    const double rinv = rsqrt_newton(r2), rr2 = rinv * rinv;
+    double f = 0.0;
+    if ((TERMS & TERM_LJ) && (code.y & kQLJ)) {
+      const double2 *tab = reinterpret_cast<const double2 *>(a.lj64 + code.x);
+      const double2 p = __ldg(tab + (modified ? 1 : 0));  // A, B or A14, B14
+      const double r6 = rr2 * rr2 * rr2, r6B = p.y * r6, r12A = p.x * r6 * r6;
+      double en = r12A - r6B, ff = VIRIAL ? (12.0 * r12A - 6.0 * r6B) * rr2 : 0.0;
+      if (LJK != kSwNone && (LJK >= 0 || a.lj_modify)) {
+        double sv, sd;
+        switch64<LJK, VIRIAL>(a.lj_sw64, r2, rinv, sv, sd);
+        if (VIRIAL) ff = ff * sv - en * sd;
+        en *= sv;
+      }
+      Elj += en;
+      f += ff;
+    }
+    if (modified) qq *= a.csf64;
+    if ((TERMS & TERM_COUL) && (code.y & kQCoul)) {
+      double en = qq * rinv, ff = VIRIAL ? en * rr2 : 0.0;
+      if (CK != kSwNone && (CK >= 0 || a.coul_modify)) {
+        double sv, sd;
+        switch64<CK, VIRIAL>(a.coul_sw64, r2, rinv, sv, sd);
+        if (VIRIAL) ff = ff * sv - en * sd;
+        en *= sv;
+      }
+      Ec += en;
+      f += ff;
+    }
+    if ((TERMS & TERM_EWALD) && (code.y & kQEwald)) {
+      const double ar = a.alpha64 * (r2 * rinv), ee = qq * exp(-ar * ar);
+      double en;
+      if (!a.exact_erf) {
+        // A&S 7.1.26 (MathUtilities.cpp:39-49), as poly5
+        const double t = rcp_newton(1.0 + 0.3275911 * ar);
+        en = t * (0.254829592 +
+                  t * (-0.284496736 +
+                       t * (1.421413741 + t * (-1.453152027 + t * 1.061405429)))) * ee * rinv;
+      } else {
+        en = qq * erfc(ar) * rinv;
+      }
+      Ec += en;
+      if (VIRIAL) f += (en + a.a2pi64 * ee) * rr2;
+    }
+    if constexpr (VIRIAL) {
+      // addVirial(fij, d) with fij = d * f (each pair is listed once)
+      const double x = W.q.d[0][k], y = W.q.d[1][k], z = W.q.d[2][k];
+      const double fx = x * f, fy = y * f;
+      V[0] += x * fx; V[1] += y * fx; V[2] += z * fx;
+      V[3] += y * fy; V[4] += z * fy; V[5] += z * (z * f);
+    }
+    npairs++;
+  };
+
+  const int nitems = a.nclusters * a.splits;
+  const size_t rowcap = 4 * (size_t)a.cap;
+  for (int gw = blk.x * kE64Warps + wib; gw < nitems; gw += blk.n * kE64Warps) {
+    const int ci = gw / a.splits, sp = gw - ci * a.splits;
+    const int4 c4 = *reinterpret_cast<const int4 *>(a.jl_count + kRowParts * ci);
+    const int p1 = c4.x, p2 = p1 + c4.y, p3 = p2 + c4.z, cnt = p3 + c4.w;
+    const int t0 = (int)((long long)cnt * sp / a.splits);
+    const int t1 = (int)((long long)cnt * (sp + 1) / a.splits);
+    if (t1 <= t0) continue;
+    __syncwarp();  // the previous item's reads of the cluster are done
+    if (lane < 8) {
+      const int islot = 8 * ci + lane, oi = a.sorted[islot];
+      W.wi[lane] = a.xw[islot];
+      W.ti[lane] = (oi >= 0 ? __float_as_int(__ldg(&a.xlo[islot].w)) : 0) * a.ntypes;
+      W.oi[lane] = oi;
+    }
+    __syncwarp();
+    auto entry_at = [&](int idx) -> uint2 {
+      if (idx >= t1) return make_uint2(0u, 0u);  // mask 0: no entry
+      const int p = (idx >= p1) + (idx >= p2) + (idx >= p3);
+      const int off = idx - (p == 0 ? 0 : (p == 1 ? p1 : (p == 2 ? p2 : p3)));
+      return __ldg(a.jlanes + (size_t)(kRowParts * ci + p) * rowcap + off);
+    };
+    // the next step's entry and j record are loaded while this one runs
+    uint2 next = entry_at(t0 + lane);
+    double4 wnext = make_double4(0, 0, 0, 0);
+    int tnext = 0;
+    auto fetch = [&]() {
+      if (next.y & 0xFFu) {
+        const int js = (int)(next.x & kJSlotMask);
+        wnext = a.xw[js];
+        tnext = __float_as_int(__ldg(&a.xlo[js].w));
+      }
+    };
+    fetch();
+    for (int b0 = t0; b0 < t1; b0 += 32) {
+      const uint2 e = next;
+      const double4 wj = wnext;
+      const int tj = tnext;
+      next = entry_at(b0 + 32 + lane);
+      fetch();
+      const unsigned mi = e.y & 0xFFu, mm = (e.y >> 8) & 0xFFu;
+      // the j atom in the entry's image (d = xj + s L - xi)
+      const int sh = (int)(e.x >> kJSlotBits);
+      const double jx = wj.x + ((sh & 3) - 1) * a.box.e[0];
+      const double jy = wj.y + (((sh >> 2) & 3) - 1) * a.box.e[1];
+      const double jz = wj.z + (((sh >> 4) & 3) - 1) * a.box.e[2];
+      // accepted pairs of this lane and, when the terms' cutoffs differ or
+      // only the minimal image counts, each one's terms (4 bits a pair)
+      unsigned acc = 0u, terms = 0u;
+#pragma unroll
+      for (int il = 0; il < 8; il++) {
+        const double4 wi = W.wi[il];
+        const double dx = jx - wi.x, dy = jy - wi.y, dz = jz - wi.z;
+        const double r2 = dx * dx + dy * dy + dz * dz;
+        if (!((mi >> il) & 1u) || r2 > a.max_cut2 * (1.0 + kBand)) continue;
+        int flags = 0;
+        bool band = false;
+        if (a.same_cut) {
+          if (r2 <= a.max_cut2 * (1.0 - kBand)) flags = kAllTerms;
+          else band = true;
+        } else {
+          if (TERMS & TERM_LJ) {
+            if (r2 <= a.lj_cut2 * (1.0 - kBand)) flags |= kQLJ;
+            else band |= r2 <= a.lj_cut2 * (1.0 + kBand);
+          }
+          if (TERMS & TERM_COUL) {
+            if (r2 <= a.coul_cut2 * (1.0 - kBand)) flags |= kQCoul;
+            else band |= r2 <= a.coul_cut2 * (1.0 + kBand);
+          }
+          if (TERMS & TERM_EWALD) {
+            if (r2 <= a.ew_cut2 * (1.0 - kBand)) flags |= kQEwald;
+            else band |= r2 <= a.ew_cut2 * (1.0 + kBand);
+          }
+        }
+        if (band) {  // rare: the reference's own arithmetic decides
+          const double x = exact_r2(a, W.oi[il], a.sorted[e.x & kJSlotMask], dx, dy, dz);
+          if ((TERMS & TERM_LJ) && x <= a.lj_cut2) flags |= kQLJ;
+          if ((TERMS & TERM_COUL) && x <= a.coul_cut2) flags |= kQCoul;
+          if ((TERMS & TERM_EWALD) && x <= a.ew_cut2) flags |= kQEwald;
+        }
+        // boxes below twice the cutoff: cutoff terms take the minimal image
+        if ((TERMS & (TERM_LJ | TERM_COUL)) && a.minimal_image &&
+            !(fabs(dx) <= a.box.H2[0] && fabs(dy) <= a.box.H2[1] && fabs(dz) <= a.box.H2[2]))
+          flags &= ~(kQLJ | kQCoul);
+        if (flags) {
+          acc |= 1u << il;
+          terms |= (unsigned)flags << (4 * il);
+        }
+      }
+      // this lane's place in the queue: an exclusive scan of the counts
+      const int n = __popc(acc);
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(kAll, incl, o);
+        if (lane >= o) incl += t;
+      }
+      int at = queued + incl - n;
+      queued += __shfl_sync(kAll, incl, 31);
+      while (acc) {
+        const int il = __ffs(acc) - 1;
+        acc &= acc - 1u;
+        const double4 wi = W.wi[il];
+        const double dx = jx - wi.x, dy = jy - wi.y, dz = jz - wi.z;
+        W.q.r2[at] = dx * dx + dy * dy + dz * dz;
+        W.q.qq[at] = wi.w * wj.w;
+        if constexpr (VIRIAL) {
+          W.q.d[0][at] = dx;
+          W.q.d[1][at] = dy;
+          W.q.d[2][at] = dz;
+        }
+        W.q.code[at] = make_uint2((unsigned)(W.ti[il] + tj),
+                                  ((terms >> (4 * il)) & 7u) | (((mm >> il) & 1u) ? kQModified : 0));
+        at++;
+      }
+      __syncwarp();
+      while (queued >= 32) {
+        queued -= 32;
+        evaluate(queued + lane);
+      }
+      __syncwarp();  // the next step appends after the reads
+    }
+  }
+  if (lane < queued) evaluate(lane);
+  const int np = warp_sum(npairs);
+  const double dlj = warp_sum(Elj), dc = warp_sum(Ec);
+  if (VIRIAL)
+    for (int q = 0; q < 6; q++) V[q] = warp_sum(V[q]);
+  if (lane == 0) {
+    red_add(&a.acc[ACC_PAIRS], (long long)np);
+    if (TERMS & TERM_LJ) red_add(&a.acc[ACC_LJ], to_fixed(dlj, kEnergyScale));
+    if (TERMS & (TERM_COUL | TERM_EWALD))
+      red_add(&a.acc[ACC_COULOMB], to_fixed(dc, kEnergyScale));
+    if (VIRIAL) {
+      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+      for (int q = 0; q < 9; q++)
+        red_add(&a.acc[ACC_VIRIAL + q], to_fixed(V[map[q]], kEnergyScale));
+    }
+  }
+}
+
+extern __shared__ __align__(16) unsigned char e64_smem[];
+
+template <int TERMS, bool VIRIAL, int LJK, int CK>
+__global__ void __launch_bounds__(kE64Warps * 32, 2) k_pairs_e64(PairArgs<float> a) {
+  pairs_e64_body<TERMS, VIRIAL, LJK, CK>(a, own_blk(),
+                                         reinterpret_cast<E64Warp<VIRIAL> *>(e64_smem));
+}
+template <int TERMS, bool VIRIAL, int LJK, int CK>
+__global__ void __launch_bounds__(kE64Warps * 32, 2)
+    k_pairs_e64_batch(const PairArgs<float> *__restrict__ tab, const int *__restrict__ first,
+                      int nm) {
+  __shared__ __align__(16) unsigned char raw[sizeof(PairArgs<float>)];
+  const int m = batch_member(first, nm, blockIdx.x);
+  pairs_e64_body<TERMS, VIRIAL, LJK, CK>(batch_args_shared(tab, m, raw), batch_blk(first, m),
+                                         reinterpret_cast<E64Warp<VIRIAL> *>(e64_smem));
 }
 
 // Adds the forces accumulated by list slot into the atoms' forces and

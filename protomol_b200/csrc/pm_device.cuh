@@ -285,13 +285,8 @@ __device__ __forceinline__ void switch_eval_base(const SwitchDev<Real> &w, Real 
       const bool falling = cmp && !rising;
       Real sq = pm_sqrt(r2);
       Real sd = sq - (rising ? w.compoff : w.cutoff);
-      Real c;  // c[0] = sd^ordInt
-      if (sizeof(Real) == 8) {
-        c = (Real)pow((double)sd, (double)w.ord_int);
-      } else {
-        c = Real(1);
-        for (int i = 0; i < w.ord_int; i++) c *= sd;
-      }
+      Real c = Real(1);  // c[0] = sd^ordInt
+      for (int i = 0; i < w.ord_int; i++) c *= sd;
       for (int i = 0; i < w.ord_int + 1; i++) {
         Real cn = c * sd;                            // c[i+1]
         const Real rg = falling ? w.itrange[i] : w.irange[i];
