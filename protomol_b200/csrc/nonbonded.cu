@@ -1834,105 +1834,102 @@ int nb_debug_cells(System *s, double cellsize, int *cell_xyz, int *dims) {
 
 // --------------------------------------------------- NonbondedSimpleFull
 // Vacuum all pairs with exclusions (NonbondedSimpleFullSystemForce.h:125-150
-// with OneAtomPair<Vacuum, Universal, LennardJones|Coulomb>): a 2-D grid of
-// (128 i atoms) x (a chunk of j) blocks, j tiles staged in shared memory;
-// every i sees every j != i (forces for i only), energies halved.  The
-// exclusion table is consulted only for j inside i's partner-index range.
-constexpr int kSfTile = 128;
+// with OneAtomPair<Vacuum, Universal, LennardJones|Coulomb>) in FP64
+// (PMGPU_PREC_DOUBLE): a warp per atom (RowWarp), every i sees every j != i
+// (forces for i only), energies halved.  The exclusion table is consulted
+// only for j inside i's partner-index range.
+struct SfArgs {
+  int n, split;
+  const double *pos, *charge;
+  const int *type;
+  int ntypes;
+  const double4 *lj64;
+  const int2 *ex_range;
+  const int *ex_start, *ex_partner, *ex_class;
+  double csf;
+  long long *force, *acc;
+  int em;
+};
 
-template <typename Real, bool LJ, bool COUL>
-__global__ void __launch_bounds__(kSfTile)
-k_simplefull(int n, int jchunk, const double *__restrict__ pos,
-             const double *__restrict__ charge, const int *__restrict__ type, int ntypes,
-             const float4 *__restrict__ lj32, const double4 *__restrict__ lj64,
-             const int2 *__restrict__ ex_range, const int *__restrict__ ex_start,
-             const int *__restrict__ ex_partner, const int *__restrict__ ex_class, Real csf,
-             long long *__restrict__ force, long long *__restrict__ acc, int em) {
-  __shared__ double sx[kSfTile], sy[kSfTile], sz[kSfTile], sq[kSfTile];
-  __shared__ int st[kSfTile];
-  const int i = blockIdx.x * kSfTile + threadIdx.x;
-  const bool valid = i < n;
-  const int ii = valid ? i : 0;
-  const double xi = pos[3 * ii], yi = pos[3 * ii + 1], zi = pos[3 * ii + 2];
-  const double qi = charge[ii];
-  const int ti = type[ii];
-  const int2 er = ex_range[ii];
-  Real fx = 0, fy = 0, fz = 0;
-  double elj = 0, ec = 0;
-  double v[6] = {0, 0, 0, 0, 0, 0};
-  const int j0 = blockIdx.y * jchunk, j1 = min(n, j0 + jchunk);
-  for (int base = j0; base < j1; base += kSfTile) {
-    const int j = base + threadIdx.x;
-    if (j < j1) {
-      sx[threadIdx.x] = pos[3 * j]; sy[threadIdx.x] = pos[3 * j + 1];
-      sz[threadIdx.x] = pos[3 * j + 2]; sq[threadIdx.x] = charge[j];
-      st[threadIdx.x] = type[j];
-    }
-    __syncthreads();
-    const int lim = min(kSfTile, j1 - base);
-    if (valid) {
-      for (int k = 0; k < lim; k++) {
-        const int jj = base + k;
-        if (jj == i) continue;
-        int excl = PMGPU_EXCL_NONE;
-        if (jj >= er.x && jj <= er.y) {
-          excl = excl_class_of(ex_start, ex_partner, ex_class, i, jj);
-          if (excl == PMGPU_EXCL_FULL) continue;
-        }
-        const Real dx = (Real)(sx[k] - xi), dy = (Real)(sy[k] - yi), dz = (Real)(sz[k] - zi);
-        const Real r2 = dx * dx + dy * dy + dz * dz;
-        const Real rr2 = Real(1) / r2;
-        Real f = 0;
-        if (LJ) {
-          Real A, B;
-          if (sizeof(Real) == 4) {
-            const float4 p = __ldg(&lj32[ti * ntypes + st[k]]);
-            A = excl == PMGPU_EXCL_MODIFIED ? p.z : p.x;
-            B = excl == PMGPU_EXCL_MODIFIED ? p.w : p.y;
-          } else {
-            const double4 p = lj64[ti * ntypes + st[k]];
-            A = excl == PMGPU_EXCL_MODIFIED ? p.z : p.x;
-            B = excl == PMGPU_EXCL_MODIFIED ? p.w : p.y;
-          }
-          const Real r6 = rr2 * rr2 * rr2;
-          const Real r6B = B * r6, r12A = A * r6 * r6;
-          if (em) elj += (double)(r12A - r6B);
-          f += (Real(12) * r12A - Real(6) * r6B) * rr2;
-        }
-        if (COUL) {
-          Real en = (Real)(qi * sq[k]) * pm_sqrt(rr2);
-          if (excl == PMGPU_EXCL_MODIFIED) en *= csf;
-          if (em) ec += (double)en;
-          f += en * rr2;
-        }
-        fx -= dx * f; fy -= dy * f; fz -= dz * f;
-        if (em == 2) {
-          const double hf = 0.5 * (double)f;
-          v[0] += dx * dx * hf; v[1] += dx * dy * hf; v[2] += dx * dz * hf;
-          v[3] += dy * dy * hf; v[4] += dy * dz * hf; v[5] += dz * dz * hf;
-        }
+// The virial of a warp's pairs (upper triangle) into the accumulators.
+__device__ __forceinline__ void row_virial(long long *acc, double (&v)[6], double *sm) {
+  const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+  for (int q = 0; q < 6; q++) {
+    v[q] = row_block_sum(v[q], sm);
+    if (threadIdx.x == 0)
+      for (int k = 0; k < 9; k++)
+        if (map[k] == q) red_add(&acc[ACC_VIRIAL + k], to_fixed(v[q], kEnergyScale));
+  }
+}
+// The force on atom i, summed over its warp's lanes.
+__device__ __forceinline__ void row_force(long long *force, int n, int i, double fx, double fy,
+                                          double fz) {
+  fx = warp_sum(fx);
+  fy = warp_sum(fy);
+  fz = warp_sum(fz);
+  if ((threadIdx.x & 31) == 0) {
+    red_add(&force[i], to_fixed(fx, kForceScale));
+    red_add(&force[n + i], to_fixed(fy, kForceScale));
+    red_add(&force[2 * n + i], to_fixed(fz, kForceScale));
+  }
+}
+
+template <bool LJ, bool COUL>
+__global__ void __launch_bounds__(kRowThreads) k_simplefull(SfArgs a) {
+  __shared__ double sm[kRowThreads / 32];
+  RowWarp r;
+  double elj = 0, ec = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  if (row_warp(a.n, a.split, &r)) {
+    const int i = r.i;
+    const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
+    const double qi = a.charge[i];
+    const int ti = a.type[i];
+    const int2 er = a.ex_range[i];
+    double fx = 0, fy = 0, fz = 0;
+    for (int j = r.j0; j < a.n; j += r.dj) {
+      if (j == i) continue;
+      int excl = PMGPU_EXCL_NONE;
+      if (j >= er.x && j <= er.y) {
+        excl = excl_class_of(a.ex_start, a.ex_partner, a.ex_class, i, j);
+        if (excl == PMGPU_EXCL_FULL) continue;
+      }
+      const double dx = a.pos[3 * j] - xi, dy = a.pos[3 * j + 1] - yi, dz = a.pos[3 * j + 2] - zi;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const double rr2 = 1.0 / r2;
+      double f = 0;
+      if (LJ) {
+        const double4 p = a.lj64[ti * a.ntypes + a.type[j]];
+        const double A = excl == PMGPU_EXCL_MODIFIED ? p.z : p.x;
+        const double B = excl == PMGPU_EXCL_MODIFIED ? p.w : p.y;
+        const double r6 = rr2 * rr2 * rr2;
+        const double r6B = B * r6, r12A = A * r6 * r6;
+        if (a.em) elj += r12A - r6B;
+        f += (12.0 * r12A - 6.0 * r6B) * rr2;
+      }
+      if (COUL) {
+        double en = qi * a.charge[j] * sqrt(rr2);
+        if (excl == PMGPU_EXCL_MODIFIED) en *= a.csf;
+        if (a.em) ec += en;
+        f += en * rr2;
+      }
+      fx -= dx * f; fy -= dy * f; fz -= dz * f;
+      if (a.em == 2) {
+        const double hf = 0.5 * f;
+        v[0] += dx * dx * hf; v[1] += dx * dy * hf; v[2] += dx * dz * hf;
+        v[3] += dy * dy * hf; v[4] += dy * dz * hf; v[5] += dz * dz * hf;
       }
     }
-    __syncthreads();
+    __syncwarp();
+    row_force(a.force, a.n, i, fx, fy, fz);
   }
-  if (valid) {
-    red_add(&force[i], to_fixed((double)fx, kForceScale));
-    red_add(&force[n + i], to_fixed((double)fy, kForceScale));
-    red_add(&force[2 * n + i], to_fixed((double)fz, kForceScale));
+  if (!a.em) return;
+  elj = row_block_sum(elj, sm) * 0.5;
+  ec = row_block_sum(ec, sm) * 0.5;
+  if (threadIdx.x == 0) {
+    if (LJ) red_add(&a.acc[ACC_LJ], to_fixed(elj, kEnergyScale));
+    if (COUL) red_add(&a.acc[ACC_COULOMB], to_fixed(ec, kEnergyScale));
   }
-  if (!em) return;
-  elj = warp_sum(elj) * 0.5;
-  ec = warp_sum(ec) * 0.5;
-  if (em == 2)
-    for (int q = 0; q < 6; q++) v[q] = warp_sum(v[q]);
-  if ((threadIdx.x & 31) == 0) {
-    if (LJ) red_add(&acc[ACC_LJ], to_fixed(elj, kEnergyScale));
-    if (COUL) red_add(&acc[ACC_COULOMB], to_fixed(ec, kEnergyScale));
-    if (em == 2) {
-      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-      for (int q = 0; q < 9; q++) red_add(&acc[ACC_VIRIAL + q], to_fixed(v[map[q]], kEnergyScale));
-    }
-  }
+  if (a.em == 2) row_virial(a.acc, v, sm);
 }
 
 // NonbondedSimpleFull with switching functions: OneAtomPair /
@@ -1942,7 +1939,7 @@ k_simplefull(int n, int jchunk, const double *__restrict__ pos,
 // Same decomposition as k_simplefull: every i sees every j != i and keeps
 // only its own force; energies and virial are halved at the end.
 struct SfSwArgs {
-  int n, jchunk;
+  int n, split;
   const double *pos, *charge;
   const int *type, *mol;
   int ntypes;
@@ -1953,6 +1950,7 @@ struct SfSwArgs {
   Box box;
   SwitchDev<double> lj_sw, coul_sw;
   int lj, coul, modify;
+  int same_sw;    // both terms take one switch (the same constants)
   double rough2;  // the larger rough-test cutoff^2
   long long *force, *acc;
   int em;  // 0 forces, 1 + energies, 2 + virial
@@ -1980,120 +1978,94 @@ __device__ __forceinline__ void scpism_pair(double qq, double sai, double saj, d
   f = (rDiElec * drDiElec + rDist) * e * rDist;
 }
 
-__global__ void __launch_bounds__(kSfTile) k_simplefull_sw(SfSwArgs a) {
-  __shared__ double sx[kSfTile], sy[kSfTile], sz[kSfTile], sq[kSfTile];
-  __shared__ int st[kSfTile], sm[kSfTile];
-  const int i = blockIdx.x * kSfTile + threadIdx.x;
-  const bool valid = i < a.n;
-  const int ii = valid ? i : 0;
-  const double xi = a.pos[3 * ii], yi = a.pos[3 * ii + 1], zi = a.pos[3 * ii + 2];
-  const double qi = a.charge[ii];
-  const int ti = a.type[ii], mi = a.mol[ii];
-  const int2 er = a.ex_range[ii];
-  double fx = 0, fy = 0, fz = 0, elj = 0, ec = 0;
-  double v[6] = {0, 0, 0, 0, 0, 0};
-  const int j0 = blockIdx.y * a.jchunk, j1 = min(a.n, j0 + a.jchunk);
-  for (int base = j0; base < j1; base += kSfTile) {
-    const int j = base + threadIdx.x;
-    if (j < j1) {
-      sx[threadIdx.x] = a.pos[3 * j];
-      sy[threadIdx.x] = a.pos[3 * j + 1];
-      sz[threadIdx.x] = a.pos[3 * j + 2];
-      sq[threadIdx.x] = a.charge[j];
-      st[threadIdx.x] = a.type[j];
-      sm[threadIdx.x] = a.mol[j];
-    }
-    __syncthreads();
-    const int lim = min(kSfTile, j1 - base);
-    if (valid) {
-      for (int k = 0; k < lim; k++) {
-        const int jj = base + k;
-        if (jj == i) continue;
-        double dx, dy, dz;
-        // minimalDifference(x_i, x_j): d = x_j - x_i
-        const double r2 = box_mindiff(a.box, xi, yi, zi, sx[k], sy[k], sz[k], dx, dy, dz);
-        if (r2 > a.rough2) continue;
-        // the exclusion table only for atoms of one molecule
-        int excl = PMGPU_EXCL_NONE;
-        if (sm[k] == mi && jj >= er.x && jj <= er.y) {
-          excl = excl_class_of(a.ex_start, a.ex_partner, a.ex_class, i, jj);
-          if (excl == PMGPU_EXCL_FULL) continue;
+__global__ void __launch_bounds__(kRowThreads) k_simplefull_sw(SfSwArgs a) {
+  __shared__ double sm[kRowThreads / 32];
+  RowWarp r;
+  double elj = 0, ec = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  if (row_warp(a.n, a.split, &r)) {
+    const int i = r.i;
+    const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
+    const double qi = a.charge[i];
+    const double sai = a.scpism ? a.sqrtalpha[i] : 0.0;
+    const bool wi = a.water && a.water[i];
+    const int ti = a.type[i], mi = a.mol[i];
+    const int2 er = a.ex_range[i];
+    double fx = 0, fy = 0, fz = 0;
+    for (int j = r.j0; j < a.n; j += r.dj) {
+      if (j == i) continue;
+      double dx, dy, dz;
+      // minimalDifference(x_i, x_j): d = x_j - x_i
+      const double r2 = box_mindiff(a.box, xi, yi, zi, a.pos[3 * j], a.pos[3 * j + 1],
+                                    a.pos[3 * j + 2], dx, dy, dz);
+      if (r2 > a.rough2) continue;
+      // the exclusion table only for atoms of one molecule
+      int excl = PMGPU_EXCL_NONE;
+      if (j >= er.x && j <= er.y && a.mol[j] == mi) {
+        excl = excl_class_of(a.ex_start, a.ex_partner, a.ex_class, i, j);
+        if (excl == PMGPU_EXCL_FULL) continue;
+      }
+      const double rr2 = 1.0 / r2;
+      double f = 0, sv = 1.0, sd = 0.0;
+      if (a.lj) {
+        const double4 p = a.lj64[ti * a.ntypes + a.type[j]];
+        const double A = excl == PMGPU_EXCL_MODIFIED ? p.z : p.x;
+        const double B = excl == PMGPU_EXCL_MODIFIED ? p.w : p.y;
+        const double r6 = rr2 * rr2 * rr2;
+        const double r6B = B * r6, r12A = A * r6 * r6;
+        double e = r12A - r6B, ff = 12.0 * r12A * rr2 - 6.0 * r6B * rr2;
+        if (a.modify) {
+          switch_eval<double>(a.lj_sw, r2, sv, sd);
+          ff = ff * sv - e * sd;
+          e = e * sv;
         }
-        const double rr2 = 1.0 / r2;
-        double f = 0;
-        if (a.lj) {
-          const double4 p = a.lj64[ti * a.ntypes + st[k]];
-          const double A = excl == PMGPU_EXCL_MODIFIED ? p.z : p.x;
-          const double B = excl == PMGPU_EXCL_MODIFIED ? p.w : p.y;
-          const double r6 = rr2 * rr2 * rr2;
-          const double r6B = B * r6, r12A = A * r6 * r6;
-          double e = r12A - r6B, ff = 12.0 * r12A * rr2 - 6.0 * r6B * rr2;
-          if (a.modify) {
-            double sv, sd;
-            switch_eval<double>(a.lj_sw, r2, sv, sd);
-            ff = ff * sv - e * sd;
-            e = e * sv;
-          }
-          elj += e;
-          f += ff;
-        }
-        if (a.coul) {
-          double e, ff;
-          if (a.scpism) {
-            if (a.water && (a.water[i] || a.water[jj])) {
-              e = ff = 0.0;  // no contribution from water (CoulombSCPISMForce.h:38-40)
-            } else {
-              scpism_pair(qi * sq[k], a.sqrtalpha[i], a.sqrtalpha[jj], a.D, rr2, e, ff);
-              if (excl == PMGPU_EXCL_MODIFIED) {
-                e *= a.csf;
-                ff *= a.csf;
-              }
-            }
+        elj += e;
+        f += ff;
+      }
+      if (a.coul) {
+        double e, ff;
+        if (a.scpism) {
+          if (a.water && (wi || a.water[j])) {
+            e = ff = 0.0;  // no contribution from water (CoulombSCPISMForce.h:38-40)
           } else {
-            e = qi * sq[k] * sqrt(rr2);
-            if (excl == PMGPU_EXCL_MODIFIED) e *= a.csf;
-            ff = e * rr2;
+            scpism_pair(qi * a.charge[j], sai, a.sqrtalpha[j], a.D, rr2, e, ff);
+            if (excl == PMGPU_EXCL_MODIFIED) {
+              e *= a.csf;
+              ff *= a.csf;
+            }
           }
-          if (a.modify) {
-            double sv, sd;
-            switch_eval<double>(a.coul_sw, r2, sv, sd);
-            ff = ff * sv - e * sd;
-            e = e * sv;
-          }
-          ec += e;
-          f += ff;
+        } else {
+          e = qi * a.charge[j] * sqrt(rr2);
+          if (excl == PMGPU_EXCL_MODIFIED) e *= a.csf;
+          ff = e * rr2;
         }
-        fx -= dx * f;
-        fy -= dy * f;
-        fz -= dz * f;
-        if (a.em == 2) {
-          const double hf = 0.5 * f;
-          v[0] += dx * dx * hf; v[1] += dx * dy * hf; v[2] += dx * dz * hf;
-          v[3] += dy * dy * hf; v[4] += dy * dz * hf; v[5] += dz * dz * hf;
+        if (a.modify) {
+          if (!a.same_sw) switch_eval<double>(a.coul_sw, r2, sv, sd);
+          ff = ff * sv - e * sd;
+          e = e * sv;
         }
+        ec += e;
+        f += ff;
+      }
+      fx -= dx * f;
+      fy -= dy * f;
+      fz -= dz * f;
+      if (a.em == 2) {
+        const double hf = 0.5 * f;
+        v[0] += dx * dx * hf; v[1] += dx * dy * hf; v[2] += dx * dz * hf;
+        v[3] += dy * dy * hf; v[4] += dy * dz * hf; v[5] += dz * dz * hf;
       }
     }
-    __syncthreads();
-  }
-  if (valid) {
-    red_add(&a.force[i], to_fixed(fx, kForceScale));
-    red_add(&a.force[a.n + i], to_fixed(fy, kForceScale));
-    red_add(&a.force[2 * a.n + i], to_fixed(fz, kForceScale));
+    __syncwarp();
+    row_force(a.force, a.n, i, fx, fy, fz);
   }
   if (!a.em) return;
-  elj = warp_sum(elj) * 0.5;
-  ec = warp_sum(ec) * 0.5;
-  if (a.em == 2)
-    for (int q = 0; q < 6; q++) v[q] = warp_sum(v[q]);
-  if ((threadIdx.x & 31) == 0) {
+  elj = row_block_sum(elj, sm) * 0.5;
+  ec = row_block_sum(ec, sm) * 0.5;
+  if (threadIdx.x == 0) {
     if (a.lj) red_add(&a.acc[ACC_LJ], to_fixed(elj, kEnergyScale));
     if (a.coul) red_add(&a.acc[ACC_COULOMB], to_fixed(ec, kEnergyScale));
-    if (a.em == 2) {
-      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-      for (int q = 0; q < 9; q++)
-        red_add(&a.acc[ACC_VIRIAL + q], to_fixed(v[map[q]], kEnergyScale));
-    }
   }
+  if (a.em == 2) row_virial(a.acc, v, sm);
 }
 
 // The FP32 pass over each unordered pair once, as the reference visits
@@ -2340,13 +2312,9 @@ int nb_simplefull_sw(System *s, const SwitchParams *lj_sw, const SwitchParams *c
                      int em, int scpism, double dielectric) {
   const int n = s->n;
   if (n == 0 || !(lj_sw || coul_sw)) return PMGPU_OK;
-  const int iblocks = (n + kSfTile - 1) / kSfTile;
-  int chunks = std::max(1, std::min((296 + iblocks - 1) / iblocks, iblocks));
-  const int jchunk = ((n + chunks - 1) / chunks + kSfTile - 1) / kSfTile * kSfTile;
-  chunks = (n + jchunk - 1) / jchunk;
   SfSwArgs a;
   a.n = n;
-  a.jchunk = jchunk;
+  a.split = row_split(n);
   a.pos = s->d_pos;
   a.charge = s->d_charge;
   a.type = s->d_type;
@@ -2365,6 +2333,7 @@ int nb_simplefull_sw(System *s, const SwitchParams *lj_sw, const SwitchParams *c
   a.lj = lj_sw != nullptr;
   a.coul = coul_sw != nullptr;
   a.modify = (lj_sw && lj_sw->modify) || (coul_sw && coul_sw->modify);
+  a.same_sw = lj_sw && coul_sw && std::memcmp(lj_sw, coul_sw, sizeof(*lj_sw)) == 0;
   a.rough2 = std::max(lj_sw ? lj_sw->rough2 : 0.0, coul_sw ? coul_sw->rough2 : 0.0);
   a.force = s->d_force;
   a.acc = s->d_acc;
@@ -2373,15 +2342,15 @@ int nb_simplefull_sw(System *s, const SwitchParams *lj_sw, const SwitchParams *c
   a.D = dielectric;
   a.sqrtalpha = s->d_scp;  // plane 0 of the SCPISM data
   a.water = s->d_water;
-  k_simplefull_sw<<<dim3(iblocks, chunks), kSfTile, 0, s->stream>>>(a);
+  k_simplefull_sw<<<row_blocks(n, a.split), kRowThreads, 0, s->stream>>>(a);
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;
 }
 
 // ------------------------------------------------ SCPISM Born radii/self
 // BornRadii and BornSelf (force/born/BornRadii.h:33-77, force/born/
-// BornSelfForce.h:31-118) as two all-pairs passes in FP64, one thread per
-// atom visiting every other atom: the first forms each atom's Born radius
+// BornSelfForce.h:31-118) as two all-pairs passes in FP64, a warp per atom
+// visiting every other atom (RowWarp): the first forms each atom's Born radius
 // and from it the atom's BornSelf factor and self energy, the second the
 // pair forces (each atom keeps its own; energies and virial halved where a
 // pair is seen twice).  Pairs are those the reference's OneAtomPair with
@@ -2448,19 +2417,18 @@ __device__ __forceinline__ int born_excl(const BornArgs &a, int i, int j, int2 e
   return excl_class_of(a.ex_start, a.ex_partner, a.ex_class, i, j);
 }
 
-constexpr int kBornThreads = 128;
 constexpr double kBornPolarE = 0.80;  // the polar H+ exponent (BornRadii.h:51)
 
-__global__ void __launch_bounds__(kBornThreads) k_born_radii(BornArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n) return;
-  const int n = a.n;
+__global__ void __launch_bounds__(kRowThreads) k_born_radii(BornArgs a) {
+  RowWarp w;
+  if (!row_warp(a.n, 1, &w)) return;
+  const int i = w.i, n = a.n;
   const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
   const double eta = a.scp[3 * n + i], C = a.scp[4 * n + i];
   const int2 er = a.ex_range[i];
   const bool wi = a.water && a.water[i];
-  double R = a.scp[2 * n + i];  // preForce: the radius starts at zeta
-  for (int j = 0; j < n; j++) {
+  double R = 0.0;
+  for (int j = w.j0; j < n; j += w.dj) {
     if (j == i) continue;
     double dx, dy, dz;
     const double r2 = box_mindiff(a.box, xi, yi, zi, a.pos[3 * j], a.pos[3 * j + 1],
@@ -2474,6 +2442,9 @@ __global__ void __launch_bounds__(kBornThreads) k_born_radii(BornArgs a) {
     double gg;
     if (born_polar(a, i, j, gg)) R += gg * f * exp(-kBornPolarE * dist);
   }
+  __syncwarp();
+  R = a.scp[2 * n + i] + warp_sum(R);  // preForce: the radius starts at zeta
+  if ((threadIdx.x & 31) != 0) return;
   // BornSelfForce.h:76-88: the solvation factor, its derivative, the
   // atom's force factor and self energy
   const double D = a.D, K = (D - 1.0) / 2, alpha = a.scp[n + i], q = a.charge[i];
@@ -2484,18 +2455,19 @@ __global__ void __launch_bounds__(kBornThreads) k_born_radii(BornArgs a) {
   a.born_q[n + i] = 0.5 * q * q * rR * (rDs - 1);
 }
 
-__global__ void __launch_bounds__(kBornThreads) k_born_self(BornArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool valid = i < a.n;
+__global__ void __launch_bounds__(kRowThreads) k_born_self(BornArgs a) {
+  __shared__ double sm[kRowThreads / 32];
+  RowWarp w;
   const int n = a.n;
-  double fx = 0, fy = 0, fz = 0, e = 0;
-  double v[6] = {0, 0, 0, 0, 0, 0};
-  if (valid) {
+  double e = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  if (row_warp(n, 1, &w)) {
+    const int i = w.i;
+    double fx = 0, fy = 0, fz = 0;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
     const double eta = a.scp[3 * n + i], C = a.scp[4 * n + i], Qi = a.born_q[i];
     const int2 er = a.ex_range[i];
     bool used = false;
-    for (int j = 0; j < n; j++) {
+    for (int j = w.j0; j < n; j += w.dj) {
       if (j == i) continue;
       double dx, dy, dz;
       const double r2 = box_mindiff(a.box, xi, yi, zi, a.pos[3 * j], a.pos[3 * j + 1],
@@ -2524,23 +2496,13 @@ __global__ void __launch_bounds__(kBornThreads) k_born_self(BornArgs a) {
     }
     // the self energy of every atom that took part in a pair
     // (BornSelfForce.h:108-117, postProcess :128-135)
-    if (used) e = a.born_q[n + i];
-    red_add(&a.force[i], to_fixed(fx, kForceScale));
-    red_add(&a.force[n + i], to_fixed(fy, kForceScale));
-    red_add(&a.force[2 * n + i], to_fixed(fz, kForceScale));
+    if (__any_sync(0xffffffffu, used) && (threadIdx.x & 31) == 0) e = a.born_q[n + i];
+    row_force(a.force, n, i, fx, fy, fz);
   }
   if (!a.em) return;
-  e = warp_sum(e);
-  if (a.em == 2)
-    for (int q = 0; q < 6; q++) v[q] = warp_sum(v[q]);
-  if ((threadIdx.x & 31) == 0) {
-    red_add(&a.acc[ACC_COULOMB], to_fixed(e, kEnergyScale));
-    if (a.em == 2) {
-      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-      for (int q = 0; q < 9; q++)
-        red_add(&a.acc[ACC_VIRIAL + q], to_fixed(v[map[q]], kEnergyScale));
-    }
-  }
+  e = row_block_sum(e, sm);
+  if (threadIdx.x == 0) red_add(&a.acc[ACC_COULOMB], to_fixed(e, kEnergyScale));
+  if (a.em == 2) row_virial(a.acc, v, sm);
 }
 
 int nb_born(System *s, const Force &f, int em) {
@@ -2568,9 +2530,9 @@ int nb_born(System *s, const Force &f, int em) {
   a.force = s->d_force;
   a.acc = s->d_acc;
   a.em = em;
-  const int nb = (n + kBornThreads - 1) / kBornThreads;
-  k_born_radii<<<nb, kBornThreads, 0, s->stream>>>(a);
-  k_born_self<<<nb, kBornThreads, 0, s->stream>>>(a);
+  const int nb = row_blocks(n, 1);
+  k_born_radii<<<nb, kRowThreads, 0, s->stream>>>(a);
+  k_born_self<<<nb, kRowThreads, 0, s->stream>>>(a);
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;
 }
@@ -2579,18 +2541,6 @@ int nb_born(System *s, const Force &f, int em) {
 int nb_simplefull(System *s, int lj, int coul, int em) {
   const int n = s->n;
   if (n == 0 || !(lj || coul)) return PMGPU_OK;
-  // enough j chunks for ~2 blocks per SM
-  const int iblocks = (n + kSfTile - 1) / kSfTile;
-  int chunks = std::max(1, std::min((296 + iblocks - 1) / iblocks, iblocks));
-  const int jchunk = ((n + chunks - 1) / chunks + kSfTile - 1) / kSfTile * kSfTile;
-  chunks = (n + jchunk - 1) / jchunk;
-  const dim3 grid(iblocks, chunks);
-  auto go = [&](auto kern, auto csf) {
-    kern<<<grid, kSfTile, 0, s->stream>>>(n, jchunk, s->d_pos, s->d_charge, s->d_type,
-                                          s->ntypes, s->d_lj32, s->d_lj64, s->d_excl_range,
-                                          s->d_excl_start, s->d_excl_partner, s->d_excl_class,
-                                          csf, s->d_force, s->d_acc, em);
-  };
   if (s->precision == PMGPU_PREC_MIXED) {
     int tiles, blocks;
     long long items;
@@ -2624,10 +2574,13 @@ int nb_simplefull(System *s, int lj, int coul, int em) {
             k_simplefull_half<false, true, false, 2>);
     }
   } else {
-    const double csf = s->coulomb_scaling;
-    if (lj && coul) go(k_simplefull<double, true, true>, csf);
-    else if (lj) go(k_simplefull<double, true, false>, csf);
-    else go(k_simplefull<double, false, true>, csf);
+    const int split = row_split(n), nb = row_blocks(n, split);
+    const SfArgs a{n, split, s->d_pos, s->d_charge, s->d_type, s->ntypes, s->d_lj64,
+                   s->d_excl_range, s->d_excl_start, s->d_excl_partner, s->d_excl_class,
+                   s->coulomb_scaling, s->d_force, s->d_acc, em};
+    if (lj && coul) k_simplefull<true, true><<<nb, kRowThreads, 0, s->stream>>>(a);
+    else if (lj) k_simplefull<true, false><<<nb, kRowThreads, 0, s->stream>>>(a);
+    else k_simplefull<false, true><<<nb, kRowThreads, 0, s->stream>>>(a);
   }
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;
