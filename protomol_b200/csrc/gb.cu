@@ -5,9 +5,8 @@
 //   GBForce      (force/GB/GBForce.cpp:14-242): pair + self energies, forces
 // The reference stores six N x N scratch arrays (distij, L, U, expTerm,
 // filTerm, partialTerm, topology/Atom.h:35-157); here every pass recomputes
-// what it needs in registers.  Each pass is a thread-per-i kernel over a
-// 2-D grid (i blocks x j chunks) with j tiles in shared memory, and per-atom
-// sums reduced in int64 fixed point, so results are order independent.
+// what it needs in registers, and per-atom sums are reduced in int64 fixed
+// point, so results are order independent.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -18,17 +17,6 @@
 namespace pmgpu {
 
 constexpr double kGbScale = 1099511627776.0;  // 2^40 for per-atom GB sums
-constexpr int kGbTile = 64;
-
-// 2-D launch shape of the all-pairs passes: enough j chunks (whole tiles)
-// that about eight blocks land on every SM.
-static void gb_grid(int n, dim3 *grid, int *jchunk) {
-  const int iblocks = (n + kGbTile - 1) / kGbTile;
-  int chunks = std::max(1, std::min((148 * 8 + iblocks - 1) / iblocks, iblocks));
-  *jchunk = ((n + chunks - 1) / chunks + kGbTile - 1) / kGbTile * kGbTile;
-  chunks = (n + *jchunk - 1) / *jchunk;
-  *grid = dim3(iblocks, chunks);
-}
 
 struct GbArgs {
   int n;
@@ -75,42 +63,25 @@ __device__ __forceinline__ Real gb_burial_term(Real dist, Real oi, Real oj, Real
          ((sjoj * sjoj) / (Real(4) * dist)) * (iL * iL - iU * iU) + C;
 }
 
-template <typename Real>
-__global__ void __launch_bounds__(kGbTile) k_gb_burial(GbArgs a, int jchunk) {
-  __shared__ double sx[kGbTile], sy[kGbTile], sz[kGbTile], so[kGbTile], ss[kGbTile];
-  __shared__ int sw[kGbTile];
-  int i = blockIdx.x * kGbTile + threadIdx.x;
-  bool valid = i < a.n;
-  int ii = valid ? i : 0;
-  double xi = a.pos[3 * ii], yi = a.pos[3 * ii + 1], zi = a.pos[3 * ii + 2];
-  Real oi = (Real)(a.vdwr[ii] - a.offset[ii]);
-  int wi = a.water ? a.water[ii] : 0;
+// The FP64 passes (PMGPU_PREC_DOUBLE): a warp per atom i, lanes on j
+// (RowWarp).  Each atom's sums end in one fixed-point add per warp.
+__global__ void __launch_bounds__(kRowThreads) k_gb_burial(GbArgs a, int split) {
+  RowWarp r;
+  if (!row_warp(a.n, split, &r)) return;
+  const int i = r.i;
+  if (a.water && a.water[i]) return;
+  const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
+  const double oi = a.vdwr[i] - a.offset[i];
   double acc = 0.0;
-  int j0 = blockIdx.y * jchunk, j1 = min(a.n, j0 + jchunk);
-  for (int base = j0; base < j1; base += kGbTile) {
-    int j = base + threadIdx.x;
-    if (j < j1) {
-      sx[threadIdx.x] = a.pos[3 * j]; sy[threadIdx.x] = a.pos[3 * j + 1];
-      sz[threadIdx.x] = a.pos[3 * j + 2];
-      so[threadIdx.x] = a.vdwr[j] - a.offset[j];
-      ss[threadIdx.x] = a.scale[j];
-      sw[threadIdx.x] = a.water ? a.water[j] : 0;
-    }
-    __syncthreads();
-    int lim = min(kGbTile, j1 - base);
-    if (valid && !wi) {
-      Real part = 0;
-      for (int k = 0; k < lim; k++) {
-        if (base + k == i || sw[k]) continue;
-        Real dx = (Real)(sx[k] - xi), dy = (Real)(sy[k] - yi), dz = (Real)(sz[k] - zi);
-        Real dist = pm_sqrt(dx * dx + dy * dy + dz * dz);
-        part += gb_burial_term<Real>(dist, oi, (Real)so[k], (Real)ss[k]);
-      }
-      acc += (double)part;
-    }
-    __syncthreads();
+  for (int j = r.j0; j < a.n; j += r.dj) {
+    if (j == i || (a.water && a.water[j])) continue;
+    const double dx = a.pos[3 * j] - xi, dy = a.pos[3 * j + 1] - yi, dz = a.pos[3 * j + 2] - zi;
+    const double dist = sqrt(dx * dx + dy * dy + dz * dz);
+    acc += gb_burial_term<double>(dist, oi, a.vdwr[j] - a.offset[j], a.scale[j]);
   }
-  if (valid && !wi && acc != 0.0) red_add(&a.burial_fx[i], to_fixed(acc, kGbScale));
+  __syncwarp();
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0 && acc != 0.0) red_add(&a.burial_fx[i], to_fixed(acc, kGbScale));
 }
 
 // GBBornRadii::postProcess (GBBornRadii.cpp:145-173) and the GB self
@@ -155,43 +126,26 @@ __global__ void k_gb_radii(GbArgs a) {
   if ((threadIdx.x & 31) == 0) red_add(&a.acc[ACC_COULOMB], to_fixed(self, kEnergyScale));
 }
 
-template <typename Real>
-__global__ void __launch_bounds__(kGbTile) k_gb_partial(GbArgs a, int jchunk) {
-  __shared__ double sx[kGbTile], sy[kGbTile], sz[kGbTile], sb[kGbTile], sq[kGbTile];
-  int i = blockIdx.x * kGbTile + threadIdx.x;
-  bool valid = i < a.n;
-  int ii = valid ? i : 0;
-  double xi = a.pos[3 * ii], yi = a.pos[3 * ii + 1], zi = a.pos[3 * ii + 2];
-  Real bi = (Real)a.born[ii], qi = (Real)a.charge[ii];
+__global__ void __launch_bounds__(kRowThreads) k_gb_partial(GbArgs a, int split) {
+  RowWarp r;
+  if (!row_warp(a.n, split, &r)) return;
+  const int i = r.i;
+  const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
+  const double bi = a.born[i], qi = a.charge[i];
   double acc = 0.0;
-  int j0 = blockIdx.y * jchunk, j1 = min(a.n, j0 + jchunk);
-  for (int base = j0; base < j1; base += kGbTile) {
-    int j = base + threadIdx.x;
-    if (j < j1) {
-      sx[threadIdx.x] = a.pos[3 * j]; sy[threadIdx.x] = a.pos[3 * j + 1];
-      sz[threadIdx.x] = a.pos[3 * j + 2];
-      sb[threadIdx.x] = a.born[j];
-      sq[threadIdx.x] = a.charge[j];
-    }
-    __syncthreads();
-    int lim = min(kGbTile, j1 - base);
-    if (valid) {
-      Real part = 0;
-      for (int k = 0; k < lim; k++) {
-        if (base + k == i) continue;
-        Real dx = (Real)(sx[k] - xi), dy = (Real)(sy[k] - yi), dz = (Real)(sz[k] - zi);
-        Real r2 = dx * dx + dy * dy + dz * dz;
-        Real bj = (Real)sb[k];
-        Real ex = exp(-r2 / (Real(4) * bi * bj));
-        Real fil = pm_sqrt(r2 + bi * bj * ex);
-        Real p = qi * (Real)sq[k] * (Real(1) / (fil * fil)) * Real(0.5) * (Real(1) / fil) * ex;
-        part += p * (bj + r2 / (Real(4) * bi));  // aTerm, GBPartialSum.cpp:33
-      }
-      acc += (double)part;
-    }
-    __syncthreads();
+  for (int j = r.j0; j < a.n; j += r.dj) {
+    if (j == i) continue;
+    const double dx = a.pos[3 * j] - xi, dy = a.pos[3 * j + 1] - yi, dz = a.pos[3 * j + 2] - zi;
+    const double r2 = dx * dx + dy * dy + dz * dz;
+    const double bj = a.born[j];
+    const double ex = exp(-r2 / (4.0 * bi * bj));
+    const double fil = sqrt(r2 + bi * bj * ex);
+    const double p = qi * a.charge[j] * (1.0 / (fil * fil)) * 0.5 * (1.0 / fil) * ex;
+    acc += p * (bj + r2 / (4.0 * bi));  // aTerm, GBPartialSum.cpp:33
   }
-  if (valid && acc != 0.0) red_add(&a.partial_fx[i], to_fixed(acc, kGbScale));
+  __syncwarp();
+  acc = warp_sum(acc);
+  if ((threadIdx.x & 31) == 0 && acc != 0.0) red_add(&a.partial_fx[i], to_fixed(acc, kGbScale));
 }
 
 __global__ void k_gb_partial_fin(GbArgs a) {
@@ -227,79 +181,61 @@ __device__ __forceinline__ Real gb_dBT(Real dist, Real oi, Real oj, Real Sj) {
          Real(0.25) * ((sjoj * sjoj) / dist) * iL2 * iL * dL + dC;
 }
 
-template <typename Real>
-__global__ void __launch_bounds__(kGbTile) k_gb_force(GbArgs a, int jchunk) {
-  __shared__ double sx[kGbTile], sy[kGbTile], sz[kGbTile], sb[kGbTile], sq[kGbTile];
-  __shared__ double so[kGbTile], ss[kGbTile], sp[kGbTile], spart[kGbTile], sa[kGbTile];
-  int i = blockIdx.x * kGbTile + threadIdx.x;
-  bool valid = i < a.n;
-  int ii = valid ? i : 0;
-  double xi = a.pos[3 * ii], yi = a.pos[3 * ii + 1], zi = a.pos[3 * ii + 2];
-  Real bi = (Real)a.born[ii], qi = (Real)a.charge[ii];
-  Real oi = (Real)(a.vdwr[ii] - a.offset[ii]);
-  Real Si = (Real)a.scale[ii], dfac_i = (Real)a.psi[ii];
-  Real part_i = (Real)a.partial[ii];
-  const Real ace_i = a.ace ? (Real)a.ace[ii] : Real(0);
-  const Real d = (Real)a.dielec;
-  Real fx = 0, fy = 0, fz = 0;
+__global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
+  __shared__ double sm[kRowThreads / 32];
+  RowWarp r;
   double epair = 0.0;
-  int j0 = blockIdx.y * jchunk, j1 = min(a.n, j0 + jchunk);
-  for (int base = j0; base < j1; base += kGbTile) {
-    int j = base + threadIdx.x;
-    if (j < j1) {
-      sx[threadIdx.x] = a.pos[3 * j]; sy[threadIdx.x] = a.pos[3 * j + 1];
-      sz[threadIdx.x] = a.pos[3 * j + 2];
-      sb[threadIdx.x] = a.born[j]; sq[threadIdx.x] = a.charge[j];
-      so[threadIdx.x] = a.vdwr[j] - a.offset[j];
-      ss[threadIdx.x] = a.scale[j]; sp[threadIdx.x] = a.psi[j];
-      spart[threadIdx.x] = a.partial[j];
-      sa[threadIdx.x] = a.ace ? a.ace[j] : 0.0;
+  if (row_warp(a.n, split, &r)) {
+    const int i = r.i;
+    const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
+    const double bi = a.born[i], qi = a.charge[i];
+    const double oi = a.vdwr[i] - a.offset[i];
+    const double Si = a.scale[i], dfac_i = a.psi[i];
+    const double part_i = a.partial[i];
+    const double ace_i = a.ace ? a.ace[i] : 0.0;
+    const double d = a.dielec;
+    double fx = 0, fy = 0, fz = 0;
+    for (int j = r.j0; j < a.n; j += r.dj) {
+      if (j == i) continue;
+      const double dx = a.pos[3 * j] - xi, dy = a.pos[3 * j + 1] - yi, dz = a.pos[3 * j + 2] - zi;
+      const double r2 = dx * dx + dy * dy + dz * dz;
+      const double dist = sqrt(r2);
+      const double idist = 1.0 / dist;
+      const double bj = a.born[j], qj = a.charge[j];
+      const double oj = a.vdwr[j] - a.offset[j], Sj = a.scale[j];
+      const double ex = exp(-r2 / (4.0 * bi * bj));
+      const double fGB = sqrt(r2 + bi * bj * ex);
+      epair += -(qi * qj) / fGB;
+      const double bti = gb_dBT<double>(dist, oi, oj, Sj);
+      const double btj = gb_dBT<double>(dist, oj, oi, Si);
+      const double dRi = dfac_i * bti;
+      const double dRj = a.psi[j] * btj;
+      const double pref = qi * qj * (1.0 / (fGB * fGB)) * 0.5 * (1.0 / fGB);
+      // partialTerm[i][j] and [j][i] (GBPartialSum.cpp:33-41)
+      const double ptij = pref * ex * (bj + r2 / (4.0 * bi));
+      const double ptji = pref * ex * (bi + r2 / (4.0 * bj));
+      double f = -pref * ((2.0 * dist - 0.5 * ex * dist) + ex * dRi * (bj + r2 / (4.0 * bi)) +
+                          ex * dRj * (bi + r2 / (4.0 * bj))) * idist;
+      f -= 0.5 * qi * qi * dRi / (bi * bi) * idist;
+      f -= 0.5 * qj * qj * dRj / (bj * bj) * idist;
+      f -= (part_i - ptij) * (dRi * idist);
+      f -= (a.partial[j] - ptji) * (dRj * idist);
+      // GBForce scaled by the dielectric factor, plus GBACEForce
+      f = f * d + (ace_i * bti + (a.ace ? a.ace[j] : 0.0) * btj) * idist;
+      fx -= dx * f; fy -= dy * f; fz -= dz * f;
     }
-    __syncthreads();
-    int lim = min(kGbTile, j1 - base);
-    if (valid) {
-      Real ep = 0;
-      for (int k = 0; k < lim; k++) {
-        if (base + k == i) continue;
-        Real dx = (Real)(sx[k] - xi), dy = (Real)(sy[k] - yi), dz = (Real)(sz[k] - zi);
-        Real r2 = dx * dx + dy * dy + dz * dz;
-        Real dist = pm_sqrt(r2);
-        Real idist = Real(1) / dist;
-        Real bj = (Real)sb[k], qj = (Real)sq[k];
-        Real oj = (Real)so[k], Sj = (Real)ss[k];
-        Real ex = exp(-r2 / (Real(4) * bi * bj));
-        Real fGB = pm_sqrt(r2 + bi * bj * ex);
-        ep += -(qi * qj) / fGB;
-        const Real bti = gb_dBT<Real>(dist, oi, oj, Sj);
-        const Real btj = gb_dBT<Real>(dist, oj, oi, Si);
-        Real dRi = dfac_i * bti;
-        Real dRj = (Real)sp[k] * btj;
-        Real pref = qi * qj * (Real(1) / (fGB * fGB)) * Real(0.5) * (Real(1) / fGB);
-        // partialTerm[i][j] and [j][i] (GBPartialSum.cpp:33-41)
-        Real ptij = pref * ex * (bj + r2 / (Real(4) * bi));
-        Real ptji = pref * ex * (bi + r2 / (Real(4) * bj));
-        Real f = -pref * ((Real(2) * dist - Real(0.5) * ex * dist) +
-                          ex * dRi * (bj + r2 / (Real(4) * bi)) +
-                          ex * dRj * (bi + r2 / (Real(4) * bj))) * idist;
-        f -= Real(0.5) * qi * qi * dRi / (bi * bi) * idist;
-        f -= Real(0.5) * qj * qj * dRj / (bj * bj) * idist;
-        f -= (part_i - ptij) * (dRi * idist);
-        f -= ((Real)spart[k] - ptji) * (dRj * idist);
-        // GBForce scaled by the dielectric factor, plus GBACEForce
-        f = f * d + (ace_i * bti + (Real)sa[k] * btj) * idist;
-        fx -= dx * f; fy -= dy * f; fz -= dz * f;
-      }
-      epair += (double)ep;
+    __syncwarp();
+    fx = warp_sum(fx);
+    fy = warp_sum(fy);
+    fz = warp_sum(fz);
+    if ((threadIdx.x & 31) == 0) {
+      red_add(&a.force[i], to_fixed(fx, kForceScale));
+      red_add(&a.force[a.n + i], to_fixed(fy, kForceScale));
+      red_add(&a.force[2 * a.n + i], to_fixed(fz, kForceScale));
     }
-    __syncthreads();
   }
-  if (valid) {
-    red_add(&a.force[i], to_fixed((double)fx, kForceScale));
-    red_add(&a.force[a.n + i], to_fixed((double)fy, kForceScale));
-    red_add(&a.force[2 * a.n + i], to_fixed((double)fz, kForceScale));
-  }
-  epair = warp_sum(epair) * 0.5 * a.dielec;
-  if ((threadIdx.x & 31) == 0) red_add(&a.acc[ACC_COULOMB], to_fixed(epair, kEnergyScale));
+  epair = row_block_sum(epair, sm) * 0.5 * a.dielec;
+  if (threadIdx.x == 0) red_add(&a.acc[ACC_COULOMB], to_fixed(epair, kEnergyScale));
 }
 
 // ---------------------------------------------------------------------
@@ -659,6 +595,16 @@ static void gb_passes_f32(const GbArgs &a, cudaStream_t st) {
   k_gb_force_half<16><<<blocks2, 16 * 32, 0, st>>>(a, tiles, items2);
 }
 
+// The FP64 chain (the partial sums' FP64 form feeds the force pass).
+static void gb_passes_f64(const GbArgs &a, cudaStream_t st) {
+  const int split = row_split(a.n), nb = row_blocks(a.n, split), nf = (a.n + 127) / 128;
+  k_gb_burial<<<nb, kRowThreads, 0, st>>>(a, split);
+  k_gb_radii<<<nf, 128, 0, st>>>(a);
+  if (a.partial_pass) k_gb_partial<<<nb, kRowThreads, 0, st>>>(a, split);
+  k_gb_partial_fin<<<nf, 128, 0, st>>>(a);
+  k_gb_force<<<nb, kRowThreads, 0, st>>>(a, split);
+}
+
 int gb_init(System *s) {
   int n = std::max(1, s->n);
   if (!s->d_gb_vdwr) return fail(PMGPU_ERR_ARG, "GB force needs gb_vdwr/gb_scale/gb_offset");
@@ -714,18 +660,11 @@ int gb_forces(System *s, const Force *gb, const Force *ace) {
   a.rec = s->d_rec;
   a.gst = s->d_gb_gst;
   a.grad = s->d_gb_grad;
-  dim3 grid;
-  int jchunk;
-  gb_grid(n, &grid, &jchunk);
   cudaStream_t st = s->stream;
   if (s->precision == PMGPU_PREC_MIXED) {
     gb_passes_f32(a, st);
   } else {
-    k_gb_burial<double><<<grid, kGbTile, 0, st>>>(a, jchunk);
-    k_gb_radii<<<(n + 127) / 128, 128, 0, st>>>(a);
-    if (a.partial_pass) k_gb_partial<double><<<grid, kGbTile, 0, st>>>(a, jchunk);
-    k_gb_partial_fin<<<(n + 127) / 128, 128, 0, st>>>(a);
-    k_gb_force<double><<<grid, kGbTile, 0, st>>>(a, jchunk);
+    gb_passes_f64(a, st);
   }
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;
@@ -875,19 +814,12 @@ extern "C" int pmgpu_gb_forces_noalloc(int n_atoms, const double *pos, const dou
   PM_CUDA(cudaMemsetAsync(a.burial_fx, 0, sizeof(long long) * (5 * (size_t)n + kGbStaticAccWords),
                           st));
 
-  dim3 grid;
-  int jchunk;
-  gb_grid(n, &grid, &jchunk);
   if (precision == PMGPU_PREC_MIXED) {
     launch_stage_pairs(n, pos, charge, nullptr, rec, st);
     k_gb_static<<<(n + 127) / 128, 128, 0, st>>>(n, gb_vdwr, gb_scale, gb_offset, water, gst);
     gb_passes_f32(a, st);
   } else {
-    k_gb_burial<double><<<grid, kGbTile, 0, st>>>(a, jchunk);
-    k_gb_radii<<<(n + 127) / 128, 128, 0, st>>>(a);
-    k_gb_partial<double><<<grid, kGbTile, 0, st>>>(a, jchunk);
-    k_gb_partial_fin<<<(n + 127) / 128, 128, 0, st>>>(a);
-    k_gb_force<double><<<grid, kGbTile, 0, st>>>(a, jchunk);
+    gb_passes_f64(a, st);
   }
   k_gb_static_out<<<(n + 255) / 256, 256, 0, st>>>(n, a.force, a.acc, forces, energy);
   PM_CUDA(cudaGetLastError());
