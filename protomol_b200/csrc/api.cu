@@ -263,7 +263,7 @@ static int system_free(System *s) {
                   s->d_improper_params,
                   s->d_gb_vdwr, s->d_gb_scale, s->d_gb_offset, s->d_water, s->d_gb_born,
                   s->d_gb_psi, s->d_gb_partial, s->d_gb_fixed, s->d_gb_ace, s->d_pos, s->d_vel,
-                  s->d_force, s->d_acc, s->d_status, s->d_pairbuf, s->d_paircount,
+                  s->d_force, s->d_pairbuf, s->d_paircount,
                   s->d_stage, s->d_snap, s->d_step, s->d_sf_tile, s->d_gb_gst, s->d_gb_grad,
                   s->d_rec, s->d_scp, s->d_scp_i, s->d_born_q,
                   s->d_sf_bits};
@@ -272,7 +272,6 @@ static int system_free(System *s) {
   for (void *p : ptrs) dev_free(s, p);
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->h_acc) cudaFreeHost(s->h_acc);
-  if (s->h_status) cudaFreeHost(s->h_status);
   if (s->h_stage) cudaFreeHost(s->h_stage);
   prof_collect(s);
   for (cudaEvent_t e : s->prof.pool) cudaEventDestroy(e);
@@ -610,10 +609,8 @@ static void constant_terms(System *s, int only, double *energies, double *virial
 // were not computed (recorded as zeros).
 int read_results(System *s, int only, double *energies, double *virial, int add,
                  int energies_valid) {
-  PM_CUDA(cudaMemcpyAsync(s->h_acc, s->d_acc, sizeof(long long) * ACC_COUNT,
+  PM_CUDA(cudaMemcpyAsync(s->h_acc, s->d_acc, sizeof(long long) * (ACC_COUNT + 1),
                           cudaMemcpyDeviceToHost, s->stream));
-  PM_CUDA(cudaMemcpyAsync(s->h_status, s->d_status, sizeof(int), cudaMemcpyDeviceToHost,
-                          s->stream));
   PM_CUDA(cudaStreamSynchronize(s->stream));
   prof_collect(s);
   return take_results(s, only, energies, virial, add, energies_valid);
@@ -723,11 +720,6 @@ static int fp32_peak(int device, double *tflops) {
   cudaEventDestroy(e1);
   cudaFree(sink);
   *tflops = best;
-  return PMGPU_OK;
-}
-
-int begin_eval(System *s) {
-  PM_CUDA(cudaMemsetAsync(s->d_acc, 0, sizeof(long long) * ACC_COUNT, s->stream));
   return PMGPU_OK;
 }
 
@@ -932,13 +924,13 @@ int pmgpu_system_create(pmgpu_context *ctx, const pmgpu_topology *t, int precisi
   }
   PM_CHECK(upload(s.get(), &s->d_pos, (const double *)nullptr, 3 * nn));
   PM_CHECK(upload(s.get(), &s->d_vel, (const double *)nullptr, 3 * nn));
-  PM_CHECK(upload(s.get(), &s->d_force, (const long long *)nullptr, 3 * nn));
-  PM_CHECK(upload(s.get(), &s->d_acc, (const long long *)nullptr, ACC_COUNT));
-  PM_CHECK(upload(s.get(), &s->d_status, (const int *)nullptr, 1));
+  PM_CHECK(upload(s.get(), &s->d_force, (const long long *)nullptr, 3 * nn + ACC_COUNT + 1));
+  s->d_acc = s->d_force + 3 * (size_t)n;
+  s->d_status = reinterpret_cast<int *>(s->d_acc + ACC_COUNT);
   PM_CHECK(upload(s.get(), &s->d_step, (const unsigned long long *)nullptr, 2));  // step, blocks done
   PM_CHECK(upload(s.get(), &s->d_stage, (const double *)nullptr, 3 * nn));
-  PM_CUDA(cudaMallocHost(&s->h_acc, sizeof(long long) * ACC_COUNT));
-  PM_CUDA(cudaMallocHost(&s->h_status, sizeof(int)));
+  PM_CUDA(cudaMallocHost(&s->h_acc, sizeof(long long) * (ACC_COUNT + 1)));
+  s->h_status = reinterpret_cast<int *>(s->h_acc + ACC_COUNT);
   PM_CUDA(cudaMallocHost(&s->h_stage, sizeof(double) * 3 * nn));
   PM_CUDA(cudaStreamSynchronize(s->stream));
   s->h_charge.assign(t->charge, t->charge + n);
@@ -955,6 +947,18 @@ int pmgpu_system_destroy(pmgpu_system *h) {
 }
 
 static System *sysp(pmgpu_system *h) { return reinterpret_cast<System *>(h); }
+
+// Whether every value is finite, in a form the host compiler vectorises: an
+// exponent field of all ones plus one carries into the sign bit.
+static bool all_finite(const double *x, size_t count) {
+  uint64_t carry = 0;
+  for (size_t k = 0; k < count; k++) {
+    uint64_t b;
+    std::memcpy(&b, x + k, sizeof(b));
+    carry |= (b & 0x7ff0000000000000ull) + 0x0010000000000000ull;
+  }
+  return !(carry >> 63);
+}
 
 static int copy_in(System *s, double *dst, const double *src) {
   if (!src) return fail(PMGPU_ERR_ARG, "null host array");
@@ -978,7 +982,7 @@ static int copy_out(System *s, double *dst, const double *src) {
 int pmgpu_system_set_positions(pmgpu_system *h, const double *pos) {
   if (!h) return fail(PMGPU_ERR_ARG, "null system");
   System *s = sysp(h);
-  if (pos)
+  if (pos && !all_finite(pos, 3 * (size_t)s->n))
     for (size_t k = 0; k < 3 * (size_t)s->n; k++)
       if (!std::isfinite(pos[k]))
         return fail(PMGPU_ERR_NAN, "non-finite position of atom " + std::to_string(k / 3));
@@ -1416,8 +1420,7 @@ int pmgpu_evaluate(pmgpu_system *h, double *energies, double *virial) {
   // MD steps (the pair kernel's specialised form), forces only
   const int mode = virial ? PAIR_VIRIAL : (energies ? PAIR_ENERGY : PAIR_FORCE);
   int r = with_overflow_retry([&]() {
-    PM_CHECK(zero_forces(s));
-    PM_CHECK(begin_eval(s));
+    PM_CHECK(zero_eval(s));
     PM_CHECK(evaluate_forces(s, -1, mode));
     return read_results(s, -1, energies, virial, 0, mode != PAIR_FORCE);
   });
@@ -1436,8 +1439,7 @@ int pmgpu_force_evaluate(pmgpu_system *h, int id, const double *pos, double *for
   s->forces_valid = 0;
   const int mode = virial ? PAIR_VIRIAL : (energies ? PAIR_ENERGY : PAIR_FORCE);
   PM_CHECK(with_overflow_retry([&]() {
-    PM_CHECK(zero_forces(s));
-    PM_CHECK(begin_eval(s));
+    PM_CHECK(zero_eval(s));
     PM_CHECK(evaluate_forces(s, id, mode));
     return read_results(s, id, energies, virial, 1, mode != PAIR_FORCE);
   }));
@@ -1457,7 +1459,7 @@ static int one_step(System *s, const pmgpu_integrator *it, int phase, int mode) 
   PM_CHECK(ri);
   // the update (which also advances the step counter of the Langevin noise)
   s->kernels += s->n > 0;
-  if (s->n == 0) PM_CHECK(begin_eval(s));
+  if (s->n == 0) PM_CHECK(zero_eval(s));
   return evaluate_forces(s, -1, mode, mode != PAIR_FORCE);
 }
 
@@ -1568,8 +1570,7 @@ static int run_enqueue(System *s, const pmgpu_integrator *it, long n_steps) {
   const bool lang = it->kind == PMGPU_INT_LANGEVIN_LEAPFROG;
   PM_CHECK(set_device_step(s));
   if (!s->forces_valid) {
-    PM_CHECK(zero_forces(s));
-    PM_CHECK(begin_eval(s));
+    PM_CHECK(zero_eval(s));
     PM_CHECK(evaluate_forces(s, -1, PAIR_FORCE, 0));
   }
   for (long k = 0; k < n_steps;) {
@@ -1882,8 +1883,7 @@ int pmgpu_debug_pair_set(pmgpu_system *h, int id, int *pairs, long long cap,
   }
   if (!s->d_paircount) PM_CHECK(dev_alloc(s, &s->d_paircount, sizeof(long long)));
   PM_CUDA(cudaMemsetAsync(s->d_paircount, 0, sizeof(long long), s->stream));
-  PM_CHECK(zero_forces(s));
-  PM_CHECK(begin_eval(s));
+  PM_CHECK(zero_eval(s));
   PM_CHECK(nb_prepare(s, &s->lists[f.list_index], 0));
   PM_CHECK(nb_build(s, &s->lists[f.list_index]));
   PM_CHECK(nb_pair_forces(s, &s->lists[f.list_index], f.terms, PAIR_RECORD, 1));

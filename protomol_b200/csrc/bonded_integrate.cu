@@ -1,6 +1,7 @@
 // Harmonic bonds and angles (FP64), the device-resident leapfrog and
 // Langevin-leapfrog updates (FP64), and fixed-point force conversion.
 #include <cmath>
+#include <cstring>
 
 #include "pm_device.cuh"
 
@@ -352,11 +353,12 @@ int bonded_all(System *s, int bonds, int angles, int dihedrals, int impropers, i
   return PMGPU_OK;
 }
 
-int zero_forces(System *s) {
+int zero_eval(System *s) {
   // a slot buffer still pending holds stale pair forces: fold (and clear) it
   // before the forces are zeroed, so the next pair launch starts from zero
   PM_CHECK(fold_pending_slots(s));
-  PM_CUDA(cudaMemsetAsync(s->d_force, 0, sizeof(long long) * 3 * (size_t)s->n, s->stream));
+  PM_CUDA(cudaMemsetAsync(s->d_force, 0, sizeof(long long) * (3 * (size_t)s->n + ACC_COUNT),
+                          s->stream));
   return PMGPU_OK;
 }
 
@@ -685,21 +687,17 @@ int forces_to_host(System *s, double *out, int add) {
   if (n == 0) return PMGPU_OK;
   // pair forces a force-only step left in a slot buffer belong to d_force
   PM_CHECK(fold_pending_slots(s));
-  double *d_tmp = nullptr;
-  PM_CUDA(cudaMallocAsync(&d_tmp, sizeof(double) * 3 * n, s->stream));
-  k_forces_to_aos<<<(n + 255) / 256, 256, 0, s->stream>>>(n, s->d_force, d_tmp);
-  std::vector<double> h(3 * (size_t)n);
-  cudaError_t e1 = cudaMemcpyAsync(h.data(), d_tmp, sizeof(double) * 3 * n,
-                                   cudaMemcpyDeviceToHost, s->stream);
-  cudaFreeAsync(d_tmp, s->stream);
-  cudaError_t e2 = cudaStreamSynchronize(s->stream);
-  if (e1 != cudaSuccess || e2 != cudaSuccess)
-    return fail(PMGPU_ERR_CUDA, std::string("force download: ") +
-                                    cudaGetErrorString(e1 != cudaSuccess ? e1 : e2));
+  // through the system's own staging buffers: no allocation, and a copy into
+  // pinned memory
+  k_forces_to_aos<<<(n + 255) / 256, 256, 0, s->stream>>>(n, s->d_force, s->d_stage);
+  PM_CUDA(cudaGetLastError());
+  PM_CUDA(cudaMemcpyAsync(s->h_stage, s->d_stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost,
+                          s->stream));
+  PM_CUDA(cudaStreamSynchronize(s->stream));
   if (add)
-    for (size_t k = 0; k < h.size(); k++) out[k] += h[k];
+    for (size_t k = 0; k < 3 * (size_t)n; k++) out[k] += s->h_stage[k];
   else
-    for (size_t k = 0; k < h.size(); k++) out[k] = h[k];
+    std::memcpy(out, s->h_stage, sizeof(double) * 3 * (size_t)n);
   return PMGPU_OK;
 }
 

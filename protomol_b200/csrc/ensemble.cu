@@ -193,8 +193,7 @@ int ensure_forces(pmgpu_ensemble *e) {
     if (s->forces_valid) continue;
     int r = PMGPU_OK;
     for (int attempt = 0; attempt < 3; attempt++) {
-      PM_CHECK(zero_forces(s));
-      PM_CHECK(begin_eval(s));
+      PM_CHECK(zero_eval(s));
       PM_CHECK(evaluate_forces(s, -1, PAIR_FORCE, 1));
       r = read_results(s, -1, nullptr, nullptr, 0, 0);
       if (r != PMGPU_ERR_OVERFLOW) break;

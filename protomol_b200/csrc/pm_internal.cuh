@@ -331,7 +331,10 @@ struct System {
   double *d_pos = nullptr;   // 3n AoS
   double *d_vel = nullptr;   // 3n AoS
   long long *d_force = nullptr;  // 3 planes of n, fixed point
-  long long *d_acc = nullptr;    // ACC_COUNT fixed point accumulators
+  // ACC_COUNT fixed point accumulators and the status word, after the forces
+  // in one allocation: an evaluation clears forces and accumulators with one
+  // fill and reads accumulators and status with one copy
+  long long *d_acc = nullptr;
   int *d_status = nullptr;
   // simple-full tile masks: per tile pair (I <= J) of 32-atom tiles the
   // index of its masks or -1; per (masks, lane) the bits of excluded (x)
@@ -344,8 +347,8 @@ struct System {
   int rec_fresh = 0;
   // GB FP32 records: static (k_gb_static) and per evaluation (k_gb_radii)
   float4 *d_gb_gst = nullptr, *d_gb_grad = nullptr;
-  long long *h_acc = nullptr;    // pinned mirror
-  int *h_status = nullptr;       // pinned mirror
+  long long *h_acc = nullptr;    // pinned mirror of accumulators and status
+  int *h_status = nullptr;       // (into h_acc)
   // forces and lists
   std::vector<Force> forces;
   std::vector<NeighborList> lists;
@@ -464,7 +467,6 @@ void switch_setup(const pmgpu_switch *in, SwitchParams *o);
 // positions into the zeroed forces and accumulators; fold = 0 leaves the
 // pair forces of a force-only MD step in the list's slot buffer
 int evaluate_forces(System *s, int only, int mode, int fold = 1);
-int begin_eval(System *s);
 // reads the accumulators and the status word after an evaluation or a
 // segment (overflow: the lists grow and PMGPU_ERR_OVERFLOW is returned)
 int read_results(System *s, int only, double *energies, double *virial, int add,
@@ -555,7 +557,8 @@ int gb_forces(System *s, const Force *gb, const Force *ace);
 // one launch; *launched = 1 when there was any term
 int bonded_all(System *s, int bonds, int angles, int dihedrals, int impropers, int em,
                int *launched);
-int zero_forces(System *s);
+// clears the forces and accumulators for an evaluation
+int zero_eval(System *s);
 // zero_acc: the update launch also clears the energy accumulators (the
 // start of a force evaluation); list: the pair list whose rebuild decision
 // the update takes from the drifted positions (or null)
