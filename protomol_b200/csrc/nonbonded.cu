@@ -1323,8 +1323,23 @@ static int jl_splits(int nclusters) {
   return (int)std::max(1LL, std::min(8LL, (want + nclusters / 2) / std::max(1, nclusters)));
 }
 
+// Raises a kernel's dynamic shared memory (once above 48 KB it must be).
+template <typename K>
+static cudaError_t raise_smem(K kern, size_t bytes) {
+  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+}
+
+template <int TERMS, typename SPEC, bool SMEM_LJ, bool TAB>
+static void launch_jl(const PairArgs<float> &a, int nb, cudaStream_t st) {
+  const size_t bytes = sizeof(JlSmem<SMEM_LJ, TAB>);
+  auto kern = k_pairs_jl<TERMS, SPEC, SMEM_LJ, TAB>;
+  // (a failed launch is found by the caller's cudaGetLastError)
+  if (raise_smem(kern, bytes) == cudaSuccess) kern<<<nb, kJlWarps * 32, bytes, st>>>(a);
+}
+
 // The specialised force-only FP32 kernels: j atoms on the lanes
-// (k_pairs_jl), the LJ table in shared memory when it is small.
+// (k_pairs_jl), a cluster's LJ parameters in shared memory when the types
+// are few.
 template <typename Real, int TERMS, typename SPEC>
 static void launch_force_spec(PairArgs<Real> &a, cudaStream_t st) {
   if constexpr (sizeof(Real) == 4) {
@@ -1335,13 +1350,9 @@ static void launch_force_spec(PairArgs<Real> &a, cudaStream_t st) {
     // the Ewald force table for the LJ + Ewald real form when the list has one
     constexpr bool kTab = TERMS == (TERM_LJ | TERM_EWALD) && SPEC::exact == 0;
     const bool tab = kTab && a.ewtab != nullptr;
-    if (a.ntypes <= kJlMaxTypes) {
-      if (tab) k_pairs_jl<TERMS, SPEC, true, kTab><<<nb, kJlWarps * 32, 0, st>>>(a);
-      else k_pairs_jl<TERMS, SPEC, true, false><<<nb, kJlWarps * 32, 0, st>>>(a);
-    } else {
-      if (tab) k_pairs_jl<TERMS, SPEC, false, kTab><<<nb, kJlWarps * 32, 0, st>>>(a);
-      else k_pairs_jl<TERMS, SPEC, false, false><<<nb, kJlWarps * 32, 0, st>>>(a);
-    }
+    if (tab && a.ntypes <= kJlMaxTypes) launch_jl<TERMS, SPEC, kTab, kTab>(a, nb, st);
+    else if (tab) launch_jl<TERMS, SPEC, false, kTab>(a, nb, st);
+    else launch_jl<TERMS, SPEC, false, false>(a, nb, st);
   } else {
     launch_pairs_spec<Real, TERMS, SPEC>(a, st, PAIR_FORCE);
   }
@@ -1393,11 +1404,6 @@ static int e64_blocks(const PairArgs<float> &a) {
 }
 template <bool VIRIAL>
 static size_t e64_smem_bytes() { return kE64Warps * sizeof(E64Warp<VIRIAL>); }
-template <bool VIRIAL, typename K>
-static cudaError_t e64_raise_smem(K kern) {
-  return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)e64_smem_bytes<VIRIAL>());
-}
 
 template <bool VIRIAL>
 static cudaError_t launch_e64(PairArgs<float> a, int form, cudaStream_t st) {
@@ -1406,7 +1412,7 @@ static cudaError_t launch_e64(PairArgs<float> a, int form, cudaStream_t st) {
   cudaError_t err = cudaSuccess;
   if (nb)
     e64_kernel<VIRIAL>(a.mask, form, [&](auto kern, auto) {
-      err = e64_raise_smem<VIRIAL>(kern);
+      err = raise_smem(kern, e64_smem_bytes<VIRIAL>());
       if (err == cudaSuccess)
         kern<<<nb, kE64Warps * 32, e64_smem_bytes<VIRIAL>(), st>>>(a);
     });
@@ -1643,7 +1649,7 @@ static int generic_batch(BatchTable<PairArgs<float>> &t, int terms, cudaStream_t
 static int e64_batch(BatchTable<PairArgs<float>> &t, int terms, int form, cudaStream_t st) {
   if (!t.members() || !t.total()) return 0;
   e64_kernel<false>(terms, form, [&](auto, auto kern) {
-    if (e64_raise_smem<false>(kern) == cudaSuccess)
+    if (raise_smem(kern, e64_smem_bytes<false>()) == cudaSuccess)
       kern<<<t.total(), kE64Warps * 32, e64_smem_bytes<false>(), st>>>(t.d, t.d_first,
                                                                        t.members());
   });
@@ -1653,14 +1659,16 @@ static int e64_batch(BatchTable<PairArgs<float>> &t, int terms, int form, cudaSt
 template <int TERMS, typename SPEC>
 static void jl_batch(NbBatch *b, BatchTable<PairArgs<float>> &t, cudaStream_t st) {
   constexpr bool kTab = TERMS == (TERM_LJ | TERM_EWALD) && SPEC::exact == 0;
-  const int g = t.total(), nm = t.members(), T = kJlWarps * 32;
-  if (kTab && b->tab) {
-    if (b->smem_lj) k_pairs_jl_batch<TERMS, SPEC, true, kTab><<<g, T, 0, st>>>(t.d, t.d_first, nm);
-    else k_pairs_jl_batch<TERMS, SPEC, false, kTab><<<g, T, 0, st>>>(t.d, t.d_first, nm);
-  } else {
-    if (b->smem_lj) k_pairs_jl_batch<TERMS, SPEC, true, false><<<g, T, 0, st>>>(t.d, t.d_first, nm);
-    else k_pairs_jl_batch<TERMS, SPEC, false, false><<<g, T, 0, st>>>(t.d, t.d_first, nm);
-  }
+  auto go = [&](auto kern, size_t bytes) {
+    if (raise_smem(kern, bytes) == cudaSuccess)
+      kern<<<t.total(), kJlWarps * 32, bytes, st>>>(t.d, t.d_first, t.members());
+  };
+  if (kTab && b->tab && b->smem_lj)
+    go(k_pairs_jl_batch<TERMS, SPEC, kTab, kTab>, sizeof(JlSmem<kTab, kTab>));
+  else if (kTab && b->tab)
+    go(k_pairs_jl_batch<TERMS, SPEC, false, kTab>, sizeof(JlSmem<false, kTab>));
+  else
+    go(k_pairs_jl_batch<TERMS, SPEC, false, false>, sizeof(JlSmem<false, false>));
 }
 
 // The pair forces of every member: force-only (the inner MD steps; the

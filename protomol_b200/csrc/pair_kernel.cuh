@@ -664,18 +664,17 @@ __global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE, SPE
 // of the cutoff take the reference's exact FP64 test after the batch's
 // pairs (rare), so the accepted set is the reference's.
 constexpr int kJlWarps = 8;
-constexpr int kJlMaxTypes = 16;  // LJ tables staged in shared memory up to this many types
+constexpr int kJlMaxTypes = 16;  // a cluster's LJ pairs staged in shared memory up to this many types
 constexpr int kJlMaxSplits = 16;  // warps one i cluster's tiles may be divided over
 constexpr float kEwTabMin = 1.0f / (1 << -kEwTabLoExp);  // the table's lowest r^2
 
 // The eight pairs of one lane's j atom with the cluster's i atoms (mi: the
 // pairs of the list's interaction mask).
-template <int TERMS, typename SPEC, bool MOD, bool SMEM_LJ, bool TAB>
-__device__ __forceinline__ void jl_pairs8(const PairArgs<float> &a, const float4 *s_lj,
-                                          const float4 *s_ew,
+template <int TERMS, typename SPEC, bool MOD, bool TAB>
+__device__ __forceinline__ void jl_pairs8(const PairArgs<float> &a, const float4 *s_ew,
                                           const float4 *xi, const int *ti, float rjx, float rjy,
                                           float rjz, float qj, int tj, unsigned mi, unsigned mm,
-                                          float (&fi)[8][3], float &fjx, float &fjy, float &fjz,
+                                          float2 (&fi)[4][3], float &fjx, float &fjy, float &fjz,
                                           unsigned &band, int &npairs) {
 #pragma unroll
   for (int il = 0; il < 8; il++) {
@@ -688,7 +687,7 @@ __device__ __forceinline__ void jl_pairs8(const PairArgs<float> &a, const float4
     band |= (on && !act && r2 <= a.max_hi) ? (1u << il) : 0u;
     npairs += act;
     const float rr = act ? r2 : 1.f;
-    const float4 p = SMEM_LJ ? s_lj[ti[il] + tj] : __ldg(a.lj32 + ti[il] + tj);
+    const float4 p = __ldg(a.lj32 + ti[il] + tj);
     float f;
     if constexpr (TAB)
       f = pair_force_tab<SPEC, MOD>(a, p, rr, x.w * qj, MOD && ((mm >> il) & 1u), s_ew);
@@ -698,9 +697,13 @@ __device__ __forceinline__ void jl_pairs8(const PairArgs<float> &a, const float4
     fjx = fmaf(dx, f, fjx);
     fjy = fmaf(dy, f, fjy);
     fjz = fmaf(dz, f, fjz);
-    fi[il][0] = fmaf(-dx, f, fi[il][0]);
-    fi[il][1] = fmaf(-dy, f, fi[il][1]);
-    fi[il][2] = fmaf(-dz, f, fi[il][2]);
+    float2 *fp = fi[il >> 1];
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      const float d = c == 0 ? dx : (c == 1 ? dy : dz);
+      if (il & 1) fp[c].y = fmaf(-d, f, fp[c].y);
+      else fp[c].x = fmaf(-d, f, fp[c].x);
+    }
   }
 }
 
@@ -710,6 +713,112 @@ struct JlStage {
   double4 w[32];
   int t[32];
 };
+
+// A warp's shared memory: its cluster's atoms from the reference point, one
+// by one (xi: position, charge) and by twos for the packed pair arithmetic
+// (xy: x0, x1, y0, y1; zq: z0, z1, q0, q1; ljp[k][t]: jl_lj_pair of the two
+// atoms with j type t), and the j-atom records of two warp steps.
+template <bool LJP>
+struct JlWarp {
+  float4 xi[8], xy[4], zq[4];
+  float4 ljp[LJP ? 4 : 1][LJP ? kJlMaxTypes : 1];
+  double wc[4];  // reference point (FP64)
+  int ti[8];     // i type * ntypes
+  int oi[8];     // i atom (-1: padding)
+  JlStage js[2];
+};
+template <bool SMEM_LJ, bool TAB>
+struct JlSmem {
+  float4 ew[TAB ? kEwTabN : 1];
+  JlWarp<SMEM_LJ && TAB> w[kJlWarps];
+};
+
+// 12 A and -6 B of two i atoms against one j type, times the C2 switch's
+// factor s1.
+__device__ __forceinline__ float4 jl_lj_pair(const float4 &p0, const float4 &p1, float s1) {
+  const float a = 12.f * s1, b = -6.f * s1;
+  return make_float4(a * p0.x, a * p1.x, b * p0.y, b * p1.y);
+}
+
+// The unmodified pairs of one lane's j atom with the cluster's 8 i atoms,
+// LJ C2 + Ewald table form, two i atoms at a time in packed FP32 (fma, mul
+// and add on register pairs: one issue slot for two results).  The kernel
+// is issue-bound, and packing halves the distance, Lennard-Jones, switch
+// and force-sum instructions; the reciprocal, the cutoff test and the table
+// lookup stay scalar.  A pair's distance bits less the table's first
+// (u) give the cutoff test, the table's range test and its index at once;
+// pairs outside read the table's last interval and are dropped by a select.
+// Warp instructions of a launch 33.2 -> 25.3 M on 23,550 atoms, 46.4 -> 40.4
+// us (caches warm); 49,998 atoms 83.6 -> 70.7 us.  What is left is the
+// per-entry work (decode, FP64 image shift, staging, three 64-bit force
+// atomics) and the latency of 24 warps an SM.
+// (d = xi - xj here.)  fj gets the sum of f d, i.e. minus the force on j.
+template <bool SMEM_LJ>
+__device__ __forceinline__ void jl_pairs8_x2(const PairArgs<float> &a, const float4 *s_ew,
+                                             const JlWarp<SMEM_LJ> &W, float rjx, float rjy,
+                                             float rjz, float qj, int tj, unsigned mi,
+                                             unsigned umax, float2 (&fi)[4][3], float2 (&fj)[3],
+                                             bool &band) {
+  constexpr unsigned kBase = kEwTabBase << (23 - kEwTabSubBits);
+  const float2 nx = make_float2(-rjx, -rjx), ny = make_float2(-rjy, -rjy),
+               nz = make_float2(-rjz, -rjz), q2 = make_float2(qj, qj);
+  const float2 ncut = make_float2(-a.lj_sw.cutoff2, -a.lj_sw.cutoff2),
+               s2 = make_float2(a.lj_sw.s2, a.lj_sw.s2), m3 = make_float2(-1.f / 3.f, -1.f / 3.f);
+#pragma unroll
+  for (int k = 0; k < 4; k++) {
+    const float4 xy = W.xy[k], zq = W.zq[k];
+    const float2 dx = add2(make_float2(xy.x, xy.y), nx),
+                 dy = add2(make_float2(xy.z, xy.w), ny),
+                 dz = add2(make_float2(zq.x, zq.y), nz);
+    const float2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+    // LJ times the switch's factor s1: 12 A r^-12 and -6 B r^-6
+    float4 ab;
+    if constexpr (SMEM_LJ) {
+      ab = W.ljp[k][tj];
+    } else {
+      const float4 p0 = __ldg(a.lj32 + W.ti[2 * k] + tj), p1 = __ldg(a.lj32 + W.ti[2 * k + 1] + tj);
+      ab = jl_lj_pair(p0, p1, a.lj_sw.s1);
+    }
+    const float2 i2 = make_float2(rcp_fast(r2.x), rcp_fast(r2.y));
+    const float2 r6 = mul2(mul2(i2, i2), i2);
+    const float2 nb = mul2(make_float2(ab.z, ab.w), r6);
+    const float2 a12 = mul2(mul2(make_float2(ab.x, ab.y), r6), r6);
+    const float2 sum = add2(a12, nb);
+    // C2 switch on r^2 clamped into [rs^2, rc^2] (switch_fast), with
+    // c = r^2 - rc^2 and w = rc^2 - 3 rs^2 + 2 r^2
+    const float2 rc = make_float2(fminf(fmaxf(r2.x, a.lj_sw.switchon2), a.lj_sw.cutoff2),
+                                  fminf(fmaxf(r2.y, a.lj_sw.switchon2), a.lj_sw.cutoff2));
+    const float2 c = add2(rc, ncut);
+    const float2 cw = mul2(c, add2(add2(rc, rc), s2));
+    // (s1 is in the parameters; the derivative's factor s3 is 4 s1, and
+    // sum + nb is 12 times the energy)
+    const float2 der = mul2(m3, fma2(c, c, cw));
+    const float2 lj = fma2(mul2(sum, i2), mul2(c, cw),
+                                 mul2(add2(sum, nb), der));
+    const float2 qq = mul2(make_float2(zq.z, zq.w), q2);
+    float2 f;
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      const float rr = h ? r2.y : r2.x;
+      const unsigned u = __float_as_uint(rr) - kBase;
+      const bool on = (mi >> (2 * k + h)) & 1u;
+      const bool act = on && u <= umax;
+      band |= on && !act && rr <= a.max_hi;
+      const float4 t4 = s_ew[min(u >> (23 - kEwTabSubBits), (unsigned)kEwTabN - 1u)];
+      const float t =
+          __uint_as_float(((u << kEwTabSubBits) & 0x007FFFFFu) | 0x3F800000u) - 1.f;
+      const float g = fmaf(t, fmaf(t, fmaf(t, t4.w, t4.z), t4.y), t4.x);
+      const float v = fmaf(h ? qq.y : qq.x, g, h ? lj.y : lj.x);
+      (h ? f.y : f.x) = act ? v : 0.f;
+    }
+    fj[0] = fma2(dx, f, fj[0]);
+    fj[1] = fma2(dy, f, fj[1]);
+    fj[2] = fma2(dz, f, fj[2]);
+    fi[k][0] = fma2(dx, f, fi[k][0]);
+    fi[k][1] = fma2(dy, f, fi[k][1]);
+    fi[k][2] = fma2(dz, f, fi[k][2]);
+  }
+}
 
 __device__ __forceinline__ void cp_async16(void *smem, const void *gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
@@ -727,22 +836,22 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
+extern __shared__ __align__(16) unsigned char jl_smem[];
+
 template <int TERMS, typename SPEC, bool SMEM_LJ, bool TAB>
 __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk) {
   constexpr unsigned kAll = 0xffffffffu;
-  __shared__ float4 s_lj[SMEM_LJ ? kJlMaxTypes * kJlMaxTypes : 1];
-  __shared__ float4 s_ew[TAB ? kEwTabN : 1];
-  __shared__ float4 s_xi[kJlWarps][8];   // i atoms from the reference point, charge
-  __shared__ int s_ti[kJlWarps][8];      // i type * ntypes
-  __shared__ int s_oi[kJlWarps][8];      // i atom (-1: padding)
-  __shared__ double s_wc[kJlWarps][3];   // reference point (FP64)
-  __shared__ JlStage s_js[kJlWarps][2];  // j-atom records of two warp steps
-  if (SMEM_LJ)
-    for (int k = threadIdx.x; k < a.ntypes * a.ntypes; k += blockDim.x) s_lj[k] = a.lj32[k];
-  if (TAB)
-    for (int k = threadIdx.x; k < kEwTabN; k += blockDim.x) s_ew[k] = __ldg(a.ewtab + k);
-  if (SMEM_LJ || TAB) __syncthreads();
+  JlSmem<SMEM_LJ, TAB> &S = *reinterpret_cast<JlSmem<SMEM_LJ, TAB> *>(jl_smem);
+  const float4 *s_ew = S.ew;
+  if (TAB) {
+    for (int k = threadIdx.x; k < kEwTabN; k += blockDim.x) S.ew[k] = __ldg(a.ewtab + k);
+    __syncthreads();
+  }
+  // the largest accepted r^2, as table position (see jl_pairs8_x2)
+  const unsigned umax =
+      __float_as_uint(a.max_lo) - (kEwTabBase << (23 - kEwTabSubBits));
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  auto &W = S.w[wib];
   int npairs = 0;
   const int nitems = a.nclusters * a.splits;
   const size_t rowcap = 4 * (size_t)a.cap;  // entries per row
@@ -760,18 +869,34 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
       const double4 w0 = a.xw[8 * ci];  // a cluster with entries has an atom in its first slot
       const double4 wi = a.xw[islot];
       const int oi = a.sorted[islot];
-      s_xi[wib][lane] = make_float4((float)(wi.x - w0.x), (float)(wi.y - w0.y),
-                                    (float)(wi.z - w0.z), (float)wi.w);
-      s_ti[wib][lane] = (oi >= 0 ? __float_as_int(__ldg(&a.xlo[islot].w)) : 0) * a.ntypes;
-      s_oi[wib][lane] = oi;
-      if (lane < 3) s_wc[wib][lane] = lane == 0 ? w0.x : (lane == 1 ? w0.y : w0.z);
+      const float4 x = make_float4((float)(wi.x - w0.x), (float)(wi.y - w0.y),
+                                   (float)(wi.z - w0.z), (float)wi.w);
+      W.xi[lane] = x;
+      if (TAB) {
+        float *xy = &W.xy[lane >> 1].x + (lane & 1), *zq = &W.zq[lane >> 1].x + (lane & 1);
+        xy[0] = x.x;
+        xy[2] = x.y;
+        zq[0] = x.z;
+        zq[2] = x.w;
+      }
+      W.ti[lane] = (oi >= 0 ? __float_as_int(__ldg(&a.xlo[islot].w)) : 0) * a.ntypes;
+      W.oi[lane] = oi;
+      if (lane < 3) W.wc[lane] = lane == 0 ? w0.x : (lane == 1 ? w0.y : w0.z);
     }
     __syncwarp();
-    const float4 *xi = s_xi[wib];
-    const int *ti = s_ti[wib];
-    float fi[8][3];
+    if constexpr (TAB && SMEM_LJ) {
+      for (int k = lane; k < 4 * a.ntypes; k += 32) {
+        const int c = k / a.ntypes, t = k - c * a.ntypes;
+        const float4 p0 = __ldg(a.lj32 + W.ti[2 * c] + t), p1 = __ldg(a.lj32 + W.ti[2 * c + 1] + t);
+        W.ljp[c][t] = jl_lj_pair(p0, p1, a.lj_sw.s1);
+      }
+      __syncwarp();
+    }
+    const float4 *xi = W.xi;
+    const int *ti = W.ti;
+    float2 fi[4][3];
 #pragma unroll
-    for (int k = 0; k < 8; k++) fi[k][0] = fi[k][1] = fi[k][2] = 0.f;
+    for (int k = 0; k < 4; k++) fi[k][0] = fi[k][1] = fi[k][2] = make_float2(0.f, 0.f);
     // Software pipeline over the warp steps (32 entries each): the entries
     // of step k + 2 are loaded into registers and the j atoms' records of
     // step k + 1 are copied into this lane's shared-memory slot (cp.async)
@@ -787,7 +912,7 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
     auto stage = [&](uint2 e, int buf) {
       if (e.y & 0xFFu) {
         const int js = (int)(e.x & kJSlotMask);
-        JlStage &g = s_js[wib][buf];
+        JlStage &g = W.js[buf];
         cp_async16(&g.w[lane], &a.xw[js]);
         cp_async16(reinterpret_cast<char *>(&g.w[lane]) + 16,
                    reinterpret_cast<const char *>(&a.xw[js]) + 16);
@@ -806,7 +931,7 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
       int tj = 0;
       float rjx = 0.f, rjy = 0.f, rjz = 0.f, qj = 0.f;
       if (mi) {
-        const JlStage &g = s_js[wib][k & 1];
+        const JlStage &g = W.js[k & 1];
         const double4 wj = g.w[lane];
         // the j atom in the entry's image (d = xj + s L - xi), from the
         // reference point; the image offsets are exact (-L, 0 or L)
@@ -815,9 +940,9 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
         const double ox = sx == 1 ? 0.0 : (sx == 0 ? -a.box.e[0] : a.box.e[0]);
         const double oy = sy == 1 ? 0.0 : (sy == 0 ? -a.box.e[1] : a.box.e[1]);
         const double oz = sz == 1 ? 0.0 : (sz == 0 ? -a.box.e[2] : a.box.e[2]);
-        rjx = (float)((wj.x + ox) - s_wc[wib][0]);
-        rjy = (float)((wj.y + oy) - s_wc[wib][1]);
-        rjz = (float)((wj.z + oz) - s_wc[wib][2]);
+        rjx = (float)((wj.x + ox) - W.wc[0]);
+        rjy = (float)((wj.y + oy) - W.wc[1]);
+        rjz = (float)((wj.z + oz) - W.wc[2]);
         qj = (float)wj.w;
         tj = g.t[lane];
       }
@@ -827,14 +952,32 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
       unsigned band = 0u;
       // modified (scaled 1-4) pairs are rare: batches without any take the
       // path without their selects
-      if (__any_sync(kAll, mm != 0u))
-        jl_pairs8<TERMS, SPEC, true, SMEM_LJ, TAB>(a, s_lj, s_ew, xi, ti, rjx, rjy, rjz, qj, tj,
-                                                   mi, mm, fi,
-                                              fjx, fjy, fjz, band, npairs);
-      else
-        jl_pairs8<TERMS, SPEC, false, SMEM_LJ, TAB>(a, s_lj, s_ew, xi, ti, rjx, rjy, rjz, qj, tj,
-                                                    mi, mm,
-                                               fi, fjx, fjy, fjz, band, npairs);
+      const bool mod = __any_sync(kAll, mm != 0u);
+      if (TAB && !mod && !a.count_pairs) {
+        float2 fj[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+        bool any = false;
+        if constexpr (TAB)
+          jl_pairs8_x2<SMEM_LJ>(a, s_ew, W, rjx, rjy, rjz, qj, tj, mi, umax, fi, fj, any);
+        fjx = -(fj[0].x + fj[0].y);
+        fjy = -(fj[1].x + fj[1].y);
+        fjz = -(fj[2].x + fj[2].y);
+        // which pairs need the exact test (the packed arithmetic's rounding)
+        if (any)
+          for (int il = 0; il < 8; il++) {
+            const float4 x = xi[il];
+            const float dx = x.x - rjx, dy = x.y - rjy, dz = x.z - rjz;
+            const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
+            const bool act =
+                __float_as_uint(r2) - (kEwTabBase << (23 - kEwTabSubBits)) <= umax;
+            if (((mi >> il) & 1u) && !act && r2 <= a.max_hi) band |= 1u << il;
+          }
+      } else if (mod) {
+        jl_pairs8<TERMS, SPEC, true, TAB>(a, s_ew, xi, ti, rjx, rjy, rjz, qj, tj, mi, mm, fi, fjx,
+                                          fjy, fjz, band, npairs);
+      } else {
+        jl_pairs8<TERMS, SPEC, false, TAB>(a, s_ew, xi, ti, rjx, rjy, rjz, qj, tj, mi, mm, fi,
+                                           fjx, fjy, fjz, band, npairs);
+      }
       // pairs within the rounding band of the cutoff: the exact FP64 test
       // (rare; their i forces go out as atomics, so this path keeps none of
       // the register-held sums live)
@@ -846,9 +989,9 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
           const float4 x = xi[il];
           const float dx = rjx - x.x, dy = rjy - x.y, dz = rjz - x.z;
           const float r2 = dx * dx + dy * dy + dz * dz;
-          if (exact_r2(a, s_oi[wib][il], oj, (double)dx, (double)dy, (double)dz) > a.max_cut2)
+          if (exact_r2(a, W.oi[il], oj, (double)dx, (double)dy, (double)dz) > a.max_cut2)
             continue;
-          const float4 p = SMEM_LJ ? s_lj[ti[il] + tj] : __ldg(a.lj32 + ti[il] + tj);
+          const float4 p = __ldg(a.lj32 + ti[il] + tj);
           const float f = pair_force_p<float, TERMS, SPEC, true>(a, p, r2, x.w * qj,
                                                                  (mm >> il) & 1u);
           fjx = fmaf(dx, f, fjx);
@@ -876,11 +1019,11 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
     for (int c = 0; c < 3; c++) {
       float v[8];
 #pragma unroll
-      for (int k = 0; k < 8; k++) v[k] = fi[k][c];
+      for (int k = 0; k < 8; k++) v[k] = k & 1 ? fi[k >> 1][c].y : fi[k >> 1][c].x;
       sum[c] = warp_tsum8(v, lane);
     }
     const int il = (lane >> 2) & 7, comp = lane & 3;
-    if (comp < 3 && s_oi[wib][il] >= 0)
+    if (comp < 3 && W.oi[il] >= 0)
       red_add(&a.fslot[(size_t)comp * a.ns + 8 * ci + il],
               fixed_force(comp == 0 ? sum[0] : (comp == 1 ? sum[1] : sum[2])));
   }

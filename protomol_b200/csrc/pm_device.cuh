@@ -153,6 +153,13 @@ __device__ __forceinline__ float rcp_nr(float x) {
   return fmaf(y, fmaf(-x, y, 1.0f), y);
 }
 
+// 1/x, the hardware estimate (one unit in the last place).
+__device__ __forceinline__ float rcp_fast(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Sums v[0..7] over the 32 lanes of a warp by a transposed butterfly
 // (9 shuffles): each exchange step hands half of the remaining slots to the
 // partner lane, so lane l ends with the total of slot (l >> 2) & 7, as do
@@ -172,6 +179,22 @@ __device__ __forceinline__ float warp_tsum8(const float (&v)[8], int lane) {
   return c;
 }
 
+// ------------------------------------------------------- packed FP32
+// Two FP32 values in a register pair: add, mul and fma issue once for both
+// (each result rounded as the scalar instruction rounds it).
+__device__ __forceinline__ float2 f2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) { return __fadd2_rn(a, b); }
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// Records by twos: element k is half k & 1 of pair k >> 1, and two fields
+// share a float4 (a0, a1, b0, b1), so one 16-byte load reads both fields of
+// two elements.
+__device__ __forceinline__ void put_pair(float4 *row, int k, float a, float b) {
+  float *p = &row[k >> 1].x + (k & 1);
+  p[0] = a;
+  p[2] = b;
+}
 // The work items of a launch dealt to the blocks round-robin (block b
 // takes items b, b + G, b + 2G, ... of G blocks), so every SM gets the same
 // number of items and the same mix of cheap and dear ones; inside a block
