@@ -482,14 +482,19 @@ __device__ __forceinline__ int clampi(int v, int lo, int hi) { return v < lo ? l
 // the radius.  Each unordered pair is listed once: j clusters of a later i
 // cluster are taken in every image, those of the same i cluster in the
 // zero image (pairs with the i atom before the j atom) and in one half of
-// the other images.  Candidates are tested four at a time: lane
-// (i atom l & 7, candidate l >> 3) tests its i atom against the
-// candidate's 4 j atoms, pairs beyond the reach or with padding are masked
-// off, and ExclusionTable::check (topology/ExclusionTable.h:116-130;
-// consulted for same-molecule minimal-image pairs as in
+// the other images.  Candidates queue in shared memory and are tested eight
+// at a time, one j atom per lane against the cluster's 8 i atoms (packed
+// FP32, two i atoms per instruction): a lane ends with its j atom's byte of
+// the interaction mask, which is the j-lane entry, and the four lanes of a
+// candidate form the tile's mask.  Pairs beyond the reach or with padding
+// are masked off, and ExclusionTable::check (topology/ExclusionTable.h:
+// 116-130; consulted for same-molecule minimal-image pairs as in
 // OneAtomPairTwo.h:47-53) clears fully excluded pairs and marks modified
-// ones.  Tiles are appended in a fixed order (range, cluster index), so
-// the list is deterministic.
+// ones.  Tiles and entries are appended in a fixed order (range, cluster
+// index), so the list is deterministic.  Against four candidates at a time
+// with a pair per lane, staged through shared memory, and the entries made
+// from the tiles in a second pass: 23,550 atoms 75 -> 43 us, 49,998 atoms
+// 142 -> 78 us, 501 atoms 30 -> 16 us a build; integer issue bounds it.
 struct BuildArgs {
   TileBuildArgs a;
   int *rebuild;
@@ -521,10 +526,12 @@ __device__ __forceinline__ void build_body(const BuildArgs &B, Blk blk) {
   int *__restrict__ status = B.status;
   if (!*rebuild) return;
   constexpr unsigned kAll = 0xffffffffu;
-  // this warp's staging of candidate j clusters (up to 32 of them)
-  __shared__ float4 st_x[kBuildWarps][128];
-  __shared__ int4 st_o[kBuildWarps][32], st_m[kBuildWarps][32];
-  __shared__ int st_h[kBuildWarps][32], st_c[kBuildWarps][32];
+  // this warp's candidate queue (j cluster, image; a ring: up to 7 left over
+  // and 32 new) and the cluster's atoms by twos: x0, x1, y0, y1 and z0, z1,
+  // molecules
+  constexpr int kRing = 64;
+  __shared__ int2 ring[kBuildWarps][kRing];
+  __shared__ float4 s_xy[kBuildWarps][4], s_zm[kBuildWarps][4];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   // the warps of the (resident) grid take the rows one at a time from a
   // counter, so the rows' unequal costs spread over the SMs; the output
@@ -560,83 +567,90 @@ __device__ __forceinline__ void build_body(const BuildArgs &B, Blk blk) {
     }
     continue;
   }
-  const int il = lane & 7, cq = lane >> 3;
-  const int islot = 8 * ci + il;
-  const int oi = sorted[islot];
-  const bool ilive = oi >= 0;
-  const float4 pi = xhi[islot];
-  const int mi = mol_s[islot];
+  bool live_i = false;
+  if (lane < 8) {
+    const float4 x = xhi[8 * ci + lane];
+    live_i = sorted[8 * ci + lane] >= 0;
+    put_pair(s_xy[wib], lane, x.x, x.y);
+    put_pair(s_zm[wib], lane, x.z, __int_as_float(mol_s[8 * ci + lane]));
+  }
+  const unsigned imask = __ballot_sync(kAll, live_i) & 0xFFu;
+  __syncwarp();
   const float R = a.cull, R2 = a.cull * a.cull;
   uint2 *row = tiles + (size_t)rw * a.cap;
   unsigned *rowmod = tmod + (size_t)rw * a.cap;
-  int count = 0;
+  uint2 *erow = jlanes + (size_t)rw * 4 * a.cap;
+  int count = 0, ne = 0;      // tiles, entries
+  unsigned head = 0, tail = 0;  // of the ring
 
-  // the candidate test of up to four staged j clusters (lane (il, cq)
-  // tests its i atom against the 4 atoms of staged candidate bq[cq])
-  auto test4 = [&](const int (&bq)[4], int ng) {
-    const int myb = cq == 0 ? bq[0] : (cq == 1 ? bq[1] : (cq == 2 ? bq[2] : bq[3]));
-    const bool cval = cq < ng;
-    const int hj = st_h[wib][myb], code = st_c[wib][myb];
-    const int sx = (code & 3) - 1, sy = ((code >> 2) & 3) - 1, sz = ((code >> 4) & 3) - 1;
-    const float S[3] = {sx * a.L[0], sy * a.L[1], sz * a.L[2]};
-    const bool diag = code == kZeroShift && (hj >> 1) == ci;
-    const int4 o4 = st_o[wib][myb], m4 = st_m[wib][myb];
-    const int oj[4] = {o4.x, o4.y, o4.z, o4.w};
-    const int mj[4] = {m4.x, m4.y, m4.z, m4.w};
-    bool pass[4], same = false;
-    float dd[4][3];
+  // the queue's next (up to) eight candidates, four lanes each
+  auto test8 = [&]() {
+    const bool val = (unsigned)(lane >> 2) < tail - head;
+    const int2 cand = ring[wib][(head + (lane >> 2)) & (kRing - 1)];
+    const int h = val ? cand.x : 0, code = val ? cand.y : kZeroShift;
+    const int jslot = 4 * h + (lane & 3);
+    const float4 pj = xhi[jslot];
+    const int mj = mol_s[jslot], oj = sorted[jslot];  // oj -1: padding
+    const float jx = pj.x + ((code & 3) - 1) * a.L[0], jy = pj.y + (((code >> 2) & 3) - 1) * a.L[1],
+                jz = pj.z + (((code >> 4) & 3) - 1) * a.L[2];
+    unsigned m = 0u, eq = 0u;
 #pragma unroll
-    for (int jl = 0; jl < 4; jl++) {
-      const float4 pj = st_x[wib][4 * myb + jl];
-      dd[jl][0] = pj.x + S[0] - pi.x;
-      dd[jl][1] = pj.y + S[1] - pi.y;
-      dd[jl][2] = pj.z + S[2] - pi.z;
-      const float r2 = dd[jl][0] * dd[jl][0] + dd[jl][1] * dd[jl][1] + dd[jl][2] * dd[jl][2];
-      pass[jl] = cval && ilive && oj[jl] >= 0 && r2 < a.reach2 && (!diag || islot < 4 * hj + jl);
-      same = same || (pass[jl] && mj[jl] == mi);
+    for (int k = 0; k < 4; k++) {
+      const float4 xy = s_xy[wib][k], zm = s_zm[wib][k];
+      const float2 dx = add2(make_float2(xy.x, xy.y), f2(-jx)),
+                   dy = add2(make_float2(xy.z, xy.w), f2(-jy)),
+                   dz = add2(make_float2(zm.x, zm.y), f2(-jz));
+      const float2 r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+      m |= (r2.x < a.reach2 ? 1u : 0u) << (2 * k) | (r2.y < a.reach2 ? 2u : 0u) << (2 * k);
+      eq |= (__float_as_int(zm.z) == mj ? 1u : 0u) << (2 * k) |
+            (__float_as_int(zm.w) == mj ? 2u : 0u) << (2 * k);
     }
-    unsigned mb[4] = {0u, 0u, 0u, 0u};
-    // same-molecule pairs (few tiles): ExclusionTable lookup
-    if (__any_sync(kAll, same)) {
-#pragma unroll
-      for (int jl = 0; jl < 4; jl++) {
-        bool mod = false;
-        if (pass[jl] && mj[jl] == mi) {
-          const bool minimal = !a.periodic || (fabsf(dd[jl][0]) <= a.H2[0] &&
-                                               fabsf(dd[jl][1]) <= a.H2[1] &&
-                                               fabsf(dd[jl][2]) <= a.H2[2]);
-          if (minimal) {
-            const int cls = excl_class_of(a.excl_start, a.excl_partner, a.excl_class, oi, oj[jl]);
-            if (cls == PMGPU_EXCL_FULL) pass[jl] = false;
-            else if (cls == PMGPU_EXCL_MODIFIED) mod = true;
-          }
-        }
-        mb[jl] = __ballot_sync(kAll, mod);
+    m &= val && oj >= 0 ? imask : 0u;
+    // the cluster's own atoms in the zero image: the i atom before the j atom
+    if (code == kZeroShift && (h >> 1) == ci) m &= (1u << (jslot & 7)) - 1u;
+    eq &= m;
+    unsigned mod = 0u;
+    // same-molecule pairs (few): ExclusionTable lookup
+    if (__any_sync(kAll, eq != 0u)) {
+      while (eq) {
+        const int il = __ffs(eq) - 1;
+        eq &= eq - 1u;
+        const float *xy = &s_xy[wib][il >> 1].x + (il & 1), *zm = &s_zm[wib][il >> 1].x + (il & 1);
+        const bool minimal = !a.periodic || (fabsf(jx - xy[0]) <= a.H2[0] &&
+                                             fabsf(jy - xy[2]) <= a.H2[1] &&
+                                             fabsf(jz - zm[0]) <= a.H2[2]);
+        if (!minimal) continue;
+        const int cls = excl_class_of(a.excl_start, a.excl_partner, a.excl_class,
+                                      sorted[8 * ci + il], oj);
+        if (cls == PMGPU_EXCL_FULL) m &= ~(1u << il);
+        else if (cls == PMGPU_EXCL_MODIFIED) mod |= 1u << il;
       }
     }
-    unsigned pb[4];
-#pragma unroll
-    for (int jl = 0; jl < 4; jl++) pb[jl] = __ballot_sync(kAll, pass[jl]);
-    // lane q < 4 assembles candidate q's masks (bit il + 8 jl) and writes it
-    const int q = lane & 3, sh = 8 * q;
-    const unsigned im = ((pb[0] >> sh) & 0xFFu) | (((pb[1] >> sh) & 0xFFu) << 8) |
-                        (((pb[2] >> sh) & 0xFFu) << 16) | (((pb[3] >> sh) & 0xFFu) << 24);
-    const unsigned mm = ((mb[0] >> sh) & 0xFFu) | (((mb[1] >> sh) & 0xFFu) << 8) |
-                        (((mb[2] >> sh) & 0xFFu) << 16) | (((mb[3] >> sh) & 0xFFu) << 24);
-    const bool wr = lane < ng && im != 0u;
-    const unsigned wm = __ballot_sync(kAll, wr);
-    if (wr) {
-      const int idx = count + __popc(wm & ((1u << lane) - 1u));
-      const int bsel = q == 0 ? bq[0] : (q == 1 ? bq[1] : (q == 2 ? bq[2] : bq[3]));
-      if (idx < a.limit) {
-        row[idx] = make_uint2((uint32_t)st_h[wib][bsel] |
-                                  ((uint32_t)st_c[wib][bsel] << kShiftBits) |
-                                  (mm ? kModFlag : 0u),
-                              im);
-        if (mm) rowmod[idx] = mm;
-      }
+    // the candidate's tile mask (bit il + 8 jl) from its four lanes
+    unsigned tm = 0u, t = m << (8 * (lane & 3));
+    t |= __shfl_xor_sync(kAll, t, 1);
+    t |= __shfl_xor_sync(kAll, t, 2);
+    if (__any_sync(kAll, mod != 0u)) {
+      tm = mod << (8 * (lane & 3));
+      tm |= __shfl_xor_sync(kAll, tm, 1);
+      tm |= __shfl_xor_sync(kAll, tm, 2);
     }
-    count += __popc(wm);
+    const bool first = (lane & 3) == 0;
+    const unsigned tb = __ballot_sync(kAll, first && t != 0u);
+    // tiles past the limit are counted, not written, and leave no entries
+    const int tidx = count + __popc(tb & ((1u << (lane & ~3)) - 1u));
+    const bool fits = tidx < a.limit;
+    if (first && t != 0u && fits) {
+      row[tidx] = make_uint2((uint32_t)h | ((uint32_t)code << kShiftBits) | (tm ? kModFlag : 0u), t);
+      if (tm) rowmod[tidx] = tm;
+    }
+    const unsigned eb = __ballot_sync(kAll, m != 0u && fits);
+    if (m != 0u && fits)
+      erow[ne + __popc(eb & ((1u << lane) - 1u))] =
+          make_uint2((uint32_t)jslot | ((uint32_t)code << kJSlotBits), m | (mod << 8));
+    count += __popc(tb);
+    ne += __popc(eb);
+    head += min(tail - head, 8u);
   };
 
   const int ux0 = (int)floorf((ilo[0] - R - a.lo[0]) / a.cs[0]);
@@ -767,38 +781,17 @@ __device__ __forceinline__ void build_body(const BuildArgs &B, Blk blk) {
           cand = jl4.w > 0.f && g2 <= R2;
         }
       }
-      unsigned cm = __ballot_sync(kAll, cand);
+      const unsigned cm = __ballot_sync(kAll, cand);
       if (!cm) continue;
-      // every candidate's lane stages its 4 atoms, cluster and image
-      if (cand) {
-        const float4 *xs = xhi + 4 * h;
-        st_x[wib][4 * lane] = xs[0];
-        st_x[wib][4 * lane + 1] = xs[1];
-        st_x[wib][4 * lane + 2] = xs[2];
-        st_x[wib][4 * lane + 3] = xs[3];
-        st_o[wib][lane] = *reinterpret_cast<const int4 *>(sorted + 4 * h);
-        st_m[wib][lane] = *reinterpret_cast<const int4 *>(mol_s + 4 * h);
-        st_h[wib][lane] = h;
-        st_c[wib][lane] = code;
-      }
+      if (cand)
+        ring[wib][(tail + __popc(cm & ((1u << lane) - 1u))) & (kRing - 1)] = make_int2(h, code);
+      tail += __popc(cm);
       __syncwarp();
-      while (cm) {
-        // the next (up to) four candidates, in ascending order
-        int bq[4];
-        int ng = 0;
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-          bq[q] = cm ? __ffs(cm) - 1 : 0;
-          if (cm) {
-            cm &= cm - 1;
-            ng = q + 1;
-          }
-        }
-        test4(bq, ng);
-      }
-      __syncwarp();  // the next batch overwrites the staging
+      while (tail - head >= 8u) test8();
+      __syncwarp();  // the next batch may overwrite what was read
     }
   }
+  if (tail != head) test8();
   if (lane == 0) {
     if (count > a.limit) {
       // the row keeps its first limit tiles; the host grows the capacity to
@@ -807,45 +800,9 @@ __device__ __forceinline__ void build_body(const BuildArgs &B, Blk blk) {
       atomicMax(rebuild + 2, count);
     }
     tile_count[rw] = min(count, a.limit);
+    jl_count[rw] = ne;
   }
-  // the row's j-lane entries, in tile order, from the tiles just written
-  // (visible to the warp after the __syncwarp)
-  __syncwarp();
-  {
-    const int nt = min(count, a.limit);
-    uint2 *erow = jlanes + (size_t)rw * 4 * a.cap;
-    int ne = 0;
-    for (int k0 = 0; k0 < nt; k0 += 32) {
-      const int k = k0 + lane;
-      uint2 t = make_uint2(0u, 0u);
-      unsigned tz = 0u;
-      if (k < nt) {
-        t = row[k];
-        if (t.x & kModFlag) tz = rowmod[k];
-      }
-      int nb = 0;
-#pragma unroll
-      for (int q = 0; q < 4; q++) nb += ((t.y >> (8 * q)) & 0xFFu) != 0u;
-      int incl = nb;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(kAll, incl, o);
-        if (lane >= o) incl += v;
-      }
-      int at = ne + incl - nb;
-      const uint32_t hj = t.x & kJMask, sh = (t.x >> kShiftBits) & kShiftMask;
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        const uint32_t mb = (t.y >> (8 * q)) & 0xFFu;
-        if (mb)
-          erow[at++] = make_uint2((4u * hj + q) | (sh << kJSlotBits),
-                                  mb | (((tz >> (8 * q)) & 0xFFu) << 8));
-      }
-      ne += __shfl_sync(kAll, incl, 31);
-    }
-    if (lane == 0) jl_count[rw] = ne;
-  }
-  __syncwarp();  // the next row reuses the staging
+  __syncwarp();  // the next row reuses the queue and the cluster's atoms
   }  // rows
   // the last warp of the launch to finish sets the counters back to zero
   if (lane == 0) {
