@@ -1226,9 +1226,14 @@ static int spec_kind(const SwitchParams &sw) {
 }
 
 // Warps per i cluster of the tile kernel: about four waves of the
-// force-only kernel's resident warps (40 per SM), at most 8 per cluster, so blocks that finish early are refilled and the
-// tail stays short.  The split depends only on the system, so every launch
-// of a system sums its forces in the same order.
+// force-only kernel's resident warps (40 per SM), at most kPairMaxSplits per
+// cluster, so blocks that finish early are refilled and the tail stays
+// short.  A small box has few clusters and each warp's tiles are one serial
+// chain (FP64 or run-time switches), so it takes many: with 8 at most, 648
+// atoms in FP64 left five warps an SM (38 us a launch; 12.8 us with 32), and
+// the generic members of a 24-box ensemble took 46 instead of 34 us.  The split depends only on the
+// system, so every launch of a system sums its forces in the same order.
+constexpr int kPairMaxSplits = 32;
 static int pair_splits(int nclusters) {
   static int sms = 0;
   if (!sms) {
@@ -1239,7 +1244,7 @@ static int pair_splits(int nclusters) {
       sms = 148;
   }
   const long long want = 4LL * sms * 40;
-  return (int)std::max(1LL, std::min(8LL, (want + nclusters / 2) / std::max(1, nclusters)));
+  return (int)std::max(1LL, std::min((long long)kPairMaxSplits, (want + nclusters / 2) / std::max(1, nclusters)));
 }
 
 template <typename Real, int TERMS, typename SPEC>
