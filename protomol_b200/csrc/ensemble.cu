@@ -252,11 +252,16 @@ int ens_step(pmgpu_ensemble *e, int phase, int mode) {
     PM_CHECK(pme_batch_correction(e->pme, em, e->side2, &kc));
   PM_CHECK(bd_batch_bonded(e->bd, em, e->side2, &kc));
   PM_CHECK(nb_batch_list(e->nb, e->st, &kc));
+  // the members without a specialised pair kernel on the third stream
+  PM_CUDA(cudaEventRecord(e->ev_fork, e->st));
+  PM_CUDA(cudaStreamWaitEvent(e->side2, e->ev_fork, 0));
+  PM_CHECK(nb_batch_generic(e->nb, e->side2, &kc));
   PM_CHECK(nb_batch_pairs(e->nb, mode, e->st, &kc));
   PM_CUDA(cudaEventRecord(e->ev_join, e->side));
   PM_CUDA(cudaStreamWaitEvent(e->st, e->ev_join, 0));
   PM_CUDA(cudaEventRecord(e->ev_join2, e->side2));
   PM_CUDA(cudaStreamWaitEvent(e->st, e->ev_join2, 0));
+  if (mode != PAIR_FORCE) PM_CHECK(nb_batch_fold(e->nb, e->st, &kc));
   return PMGPU_OK;
 }
 

@@ -1633,10 +1633,10 @@ static void jl_batch(NbBatch *b, BatchTable<PairArgs<float>> &t, cudaStream_t st
     go(k_pairs_jl_batch<TERMS, SPEC, false, false>, sizeof(JlSmem<false, false>));
 }
 
-// The pair forces of every member: force-only (the inner MD steps; the
-// slot-ordered forces stay for the next update kernel) or with energies
-// (the last step; the slot forces are folded in), as nb_pair_forces does
-// for each member.
+// The pair forces of every member, as nb_pair_forces gives each: force-only
+// (the inner MD steps; the slot-ordered forces stay for the next update
+// kernel) or with energies (the last step; nb_batch_fold then adds the slot
+// forces).
 static int jl_form(NbBatch *b, BatchTable<PairArgs<float>> &t, cudaStream_t st) {
   if (!t.members() || !t.total()) return 0;
   switch (b->form) {
@@ -1653,17 +1653,32 @@ static int jl_form(NbBatch *b, BatchTable<PairArgs<float>> &t, cudaStream_t st) 
   return 1;
 }
 
+// Small boxes without the specialised form take the generic kernel, whose
+// few long chains leave most of the device idle: launched on a stream beside
+// the others' force-only kernel (the two write different members' slots).
+int nb_batch_generic(NbBatch *b, cudaStream_t st, long long *launched) {
+  *launched += generic_batch(b->gforce, b->terms, st);
+  PM_CUDA(cudaGetLastError());
+  return PMGPU_OK;
+}
+
 int nb_batch_pairs(NbBatch *b, int mode, cudaStream_t st, long long *launched) {
   *launched += jl_form(b, b->jl, st);
-  *launched += generic_batch(b->gforce, b->terms, st);
   if (mode != PAIR_FORCE) {
     *launched += e64_batch(b->energy, b->terms, b->form, st);
     *launched += e64_batch(b->genergy, b->terms, PMGPU_PAIRK_GENERIC, st);
-    if (b->slots.total()) {
-      k_slot_forces_batch<<<b->slots.total(), 256, 0, st>>>(b->slots.d, b->slots.d_first,
-                                                           b->slots.members());
-      *launched += 1;
-    }
+  }
+  PM_CUDA(cudaGetLastError());
+  return PMGPU_OK;
+}
+
+// The slot-ordered forces of every member into its atoms' forces (energy
+// steps, after every pair launch).
+int nb_batch_fold(NbBatch *b, cudaStream_t st, long long *launched) {
+  if (b->slots.total()) {
+    k_slot_forces_batch<<<b->slots.total(), 256, 0, st>>>(b->slots.d, b->slots.d_first,
+                                                         b->slots.members());
+    *launched += 1;
   }
   PM_CUDA(cudaGetLastError());
   return PMGPU_OK;

@@ -490,7 +490,9 @@ int nb_batch_time_jl(NbBatch *b, System *const *m, int n, const int *splits, int
                      cudaStream_t st, double *ms);
 void nb_batch_member_info(NbBatch *b, int k, int *splits, int *clusters);
 int nb_batch_list(NbBatch *b, cudaStream_t st, long long *launched);
+int nb_batch_generic(NbBatch *b, cudaStream_t st, long long *launched);
 int nb_batch_pairs(NbBatch *b, int mode, cudaStream_t st, long long *launched);
+int nb_batch_fold(NbBatch *b, cudaStream_t st, long long *launched);
 void nb_batch_mark(NbBatch *b, System *const *m, int n, int mode);
 PmeBatch *pme_batch_new();
 void pme_batch_free(PmeBatch *b);
