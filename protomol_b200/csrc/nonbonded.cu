@@ -911,6 +911,9 @@ int nb_list_init(System *s, NeighborList *nl, double cutoff, double skin, double
   PM_CHECK(dev_alloc(s, &nl->d_sorted, sizeof(int) * ns));
   PM_CHECK(dev_alloc(s, &nl->d_slot_of, sizeof(int) * std::max(1, s->n)));
   PM_CUDA(cudaMemsetAsync(nl->d_sorted, 0xff, sizeof(int) * ns, s->stream));
+  // no slot: a first build whose column buckets overflow places only some of
+  // the atoms, and the steps until the host sees the flag read every atom's
+  PM_CUDA(cudaMemsetAsync(nl->d_slot_of, 0xff, sizeof(int) * std::max(1, s->n), s->stream));
   PM_CHECK(dev_alloc(s, &nl->d_offset, sizeof(double) * 3 * nn));
   PM_CHECK(dev_alloc(s, &nl->d_xbuild, sizeof(double) * 3 * nn));
   PM_CHECK(dev_alloc(s, &nl->d_xhi, sizeof(float4) * ns));

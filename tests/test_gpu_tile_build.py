@@ -8,7 +8,7 @@ import pytest
 
 import fixtures as F
 import oracle
-from protomol_b200 import ForceFactory, GpuSystem, systems
+from protomol_b200 import ForceFactory, GpuSystem, LeapfrogIntegrator, systems
 
 pytestmark = pytest.mark.gpu
 
@@ -51,3 +51,26 @@ def test_pair_set_and_forces(ctx, kind, n, edge, rc):
         force.evaluate(s.pos, f, energies)
         assert F.rms_rel(f, fo) <= 1e-5 or np.abs(f - fo).max() <= 4 * 2.0 ** -32
     gs.close()
+
+
+def test_column_overflow_in_recycled_memory(ctx):
+    """A first build that drops atoms (column buckets of 32) in memory another
+    system left full of other values: the dropped atoms have no slot, and the
+    repeated segment equals the one that never overflowed."""
+    big = systems.tip3p_box(4000, 49.5, seed=5, jitter=0.2)
+    out = []
+    for cap in (None, 32, 32):
+        other = GpuSystem(ctx, big, "mixed")
+        ForceFactory(other, 8.0).make(LINE.format(on=7.0, rc=8.0))
+        other.evaluate()
+        other.close()
+        s = systems.tip3p_box(216, 18.62, seed=5, jitter=0.2)
+        gs = GpuSystem(ctx, s, "mixed")
+        ForceFactory(gs, 8.0).make(LINE.format(on=7.0, rc=8.0))
+        if cap:
+            gs.set_column_capacity(cap)
+        LeapfrogIntegrator(0.5).run(gs, 20)
+        out.append((gs.positions(), gs.velocities()))
+        gs.close()
+    for got in out[1:]:
+        assert np.array_equal(got[0], out[0][0]) and np.array_equal(got[1], out[0][1])
