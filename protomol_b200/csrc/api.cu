@@ -269,6 +269,8 @@ static int system_free(System *s) {
                   s->d_sf_bits};
   for (auto &g : s->graphs)
     if (g.exec) cudaGraphExecDestroy(g.exec);
+  for (auto &g : s->evals)
+    if (g.exec) cudaGraphExecDestroy(g.exec);
   for (void *p : ptrs) dev_free(s, p);
   if (s->stream) cudaStreamSynchronize(s->stream);
   if (s->h_acc) cudaFreeHost(s->h_acc);
@@ -1411,6 +1413,97 @@ int pmgpu_force_set_enabled(pmgpu_system *h, int id, int enabled) {
   return PMGPU_OK;
 }
 
+// One evaluation's work on the system's stream: the staged positions to the
+// device (with_pos), clear, evaluate, accumulators and status to the host,
+// the forces to the staging buffer (with_forces).
+static int eval_enqueue(System *s, int only, int mode, int with_pos, int with_forces) {
+  if (with_pos && s->n)
+    PM_CUDA(cudaMemcpyAsync(s->d_pos, s->h_stage, sizeof(double) * 3 * (size_t)s->n,
+                            cudaMemcpyHostToDevice, s->stream));
+  PM_CHECK(zero_eval(s));
+  PM_CHECK(evaluate_forces(s, only, mode));
+  PM_CUDA(cudaMemcpyAsync(s->h_acc, s->d_acc, sizeof(long long) * (ACC_COUNT + 1),
+                          cudaMemcpyDeviceToHost, s->stream));
+  if (with_forces) PM_CHECK(forces_enqueue(s));
+  return PMGPU_OK;
+}
+
+// eval_enqueue and the wait for it.  An evaluation is 10 to 20 short
+// launches on three streams, which cost the host about 3 us each, more than
+// most of them run; the third evaluation of a kind captures them into a
+// graph and later ones replay it in one launch (the first two, which a
+// program that evaluates once or twice ends with, stay eager).  A kind is
+// the call's form and what the launches' arguments depend on; new buffers
+// or forces change graph_version.  One call, eager and replayed: 648 atoms
+// cutoff 97 and 78 us, 501 atoms with PME 146 and 123, a 544-atom polymer in
+// FP64 502 and 380, 49,998 atoms with PME about 700 and 690.
+constexpr int kEvalEager = 2;
+constexpr size_t kEvalKinds = 16;
+static int eval_run(System *s, int only, int mode, int with_pos, int with_forces) {
+  PM_CHECK(fold_pending_slots(s));
+  s->rec_fresh = 0;
+  unsigned long long key = (unsigned)(only + 1) | (unsigned long long)mode << 32 |
+                           (unsigned long long)(with_pos != 0) << 36 |
+                           (unsigned long long)(with_forces != 0) << 37 |
+                           (unsigned long long)(s->count_pairs != 0) << 38;
+  for (size_t k = 0; k < s->lists.size() && k < 16; k++)
+    if (s->lists[k].built) key |= 1ull << (40 + k);
+  System::EvalGraph *g = nullptr;
+  if (s->n && s->lists.size() <= 16 && !s->prof.enabled && !s->graphs_disabled) {
+    for (auto &e : s->evals)
+      if (e.key == key) g = &e;
+    if (!g && s->evals.size() < kEvalKinds) {
+      s->evals.emplace_back();
+      g = &s->evals.back();
+      g->key = key;
+    }
+  }
+  if (g && g->version != s->graph_version) {
+    if (g->exec) cudaGraphExecDestroy(g->exec);
+    g->exec = nullptr;
+    g->version = s->graph_version;
+    g->uses = 0;
+  }
+  if (g && !g->exec && g->uses++ >= kEvalEager) {
+    const long long k0 = s->kernels;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+      const int r = eval_enqueue(s, only, mode, with_pos, with_forces);
+      const cudaError_t ec = cudaStreamEndCapture(s->stream, &graph);
+      if (r != PMGPU_OK || ec != cudaSuccess || !graph ||
+          cudaGraphInstantiate(&g->exec, graph, cudaGraphInstantiateFlagUseNodePriority) !=
+              cudaSuccess)
+        g->exec = nullptr;
+      if (graph) cudaGraphDestroy(graph);
+      g->kernels = s->kernels - k0;
+      s->kernels = k0;
+      g->forms.clear();
+      for (auto &nl : s->lists) g->forms.push_back(nl.last_form);
+      // nothing has run yet: the lists are as they were
+      for (size_t k = 0; k < s->lists.size(); k++) s->lists[k].built = (key >> (40 + k)) & 1;
+    }
+    if (!g->exec) {
+      cudaGetLastError();
+      s->graphs_disabled = 1;
+    }
+  }
+  if (g && g->exec) {
+    PM_CUDA(cudaGraphLaunch(g->exec, s->stream));
+    s->kernels += g->kernels;
+    // the host state eval_enqueue leaves
+    for (auto &f : s->forces)
+      if ((only >= 0 ? f.id == only : f.enabled) && f.list_index >= 0) {
+        s->lists[f.list_index].built = 1;
+        s->lists[f.list_index].last_form = g->forms[f.list_index];
+      }
+  } else {
+    PM_CHECK(eval_enqueue(s, only, mode, with_pos, with_forces));
+  }
+  PM_CUDA(cudaStreamSynchronize(s->stream));
+  prof_collect(s);
+  return PMGPU_OK;
+}
+
 int pmgpu_evaluate(pmgpu_system *h, double *energies, double *virial) {
   if (!h) return fail(PMGPU_ERR_ARG, "null system");
   System *s = sysp(h);
@@ -1420,9 +1513,8 @@ int pmgpu_evaluate(pmgpu_system *h, double *energies, double *virial) {
   // MD steps (the pair kernel's specialised form), forces only
   const int mode = virial ? PAIR_VIRIAL : (energies ? PAIR_ENERGY : PAIR_FORCE);
   int r = with_overflow_retry([&]() {
-    PM_CHECK(zero_eval(s));
-    PM_CHECK(evaluate_forces(s, -1, mode));
-    return read_results(s, -1, energies, virial, 0, mode != PAIR_FORCE);
+    PM_CHECK(eval_run(s, -1, mode, 0, 0));
+    return take_results(s, -1, energies, virial, 0, mode != PAIR_FORCE);
   });
   s->forces_valid = (r == PMGPU_OK);
   return r;
@@ -1435,15 +1527,16 @@ int pmgpu_force_evaluate(pmgpu_system *h, int id, const double *pos, double *for
   PM_CHECK(run_finish(s));
   PM_CUDA(cudaSetDevice(s->device));
   if (id < 0 || id >= (int)s->forces.size()) return fail(PMGPU_ERR_ARG, "no such force");
-  if (pos) PM_CHECK(copy_in(s, s->d_pos, pos));
+  if (pos) std::memcpy(s->h_stage, pos, sizeof(double) * 3 * (size_t)s->n);
   s->forces_valid = 0;
   const int mode = virial ? PAIR_VIRIAL : (energies ? PAIR_ENERGY : PAIR_FORCE);
+  int staged = pos != nullptr;
   PM_CHECK(with_overflow_retry([&]() {
-    PM_CHECK(zero_eval(s));
-    PM_CHECK(evaluate_forces(s, id, mode));
-    return read_results(s, id, energies, virial, 1, mode != PAIR_FORCE);
+    PM_CHECK(eval_run(s, id, mode, staged, forces != nullptr));
+    staged = 0;  // on the device now; the forces have taken the staging buffer
+    return take_results(s, id, energies, virial, 1, mode != PAIR_FORCE);
   }));
-  if (forces) PM_CHECK(forces_to_host(s, forces, 1));
+  if (forces) forces_take(s, forces, 1);
   return PMGPU_OK;
 }
 

@@ -682,22 +682,32 @@ __global__ void k_forces_to_aos(int n, const long long *__restrict__ force,
   for (int c = 0; c < 3; c++) out[3 * i + c] = (double)force[c * n + i] * (1.0 / kForceScale);
 }
 
-int forces_to_host(System *s, double *out, int add) {
-  int n = s->n;
+int forces_enqueue(System *s) {
+  const int n = s->n;
   if (n == 0) return PMGPU_OK;
-  // pair forces a force-only step left in a slot buffer belong to d_force
-  PM_CHECK(fold_pending_slots(s));
   // through the system's own staging buffers: no allocation, and a copy into
   // pinned memory
   k_forces_to_aos<<<(n + 255) / 256, 256, 0, s->stream>>>(n, s->d_force, s->d_stage);
   PM_CUDA(cudaGetLastError());
   PM_CUDA(cudaMemcpyAsync(s->h_stage, s->d_stage, sizeof(double) * 3 * n, cudaMemcpyDeviceToHost,
                           s->stream));
-  PM_CUDA(cudaStreamSynchronize(s->stream));
+  return PMGPU_OK;
+}
+
+void forces_take(System *s, double *out, int add) {
+  const size_t n3 = 3 * (size_t)s->n;
   if (add)
-    for (size_t k = 0; k < 3 * (size_t)n; k++) out[k] += s->h_stage[k];
+    for (size_t k = 0; k < n3; k++) out[k] += s->h_stage[k];
   else
-    std::memcpy(out, s->h_stage, sizeof(double) * 3 * (size_t)n);
+    std::memcpy(out, s->h_stage, sizeof(double) * n3);
+}
+
+int forces_to_host(System *s, double *out, int add) {
+  // pair forces a force-only step left in a slot buffer belong to d_force
+  PM_CHECK(fold_pending_slots(s));
+  PM_CHECK(forces_enqueue(s));
+  PM_CUDA(cudaStreamSynchronize(s->stream));
+  forces_take(s, out, add);
   return PMGPU_OK;
 }
 

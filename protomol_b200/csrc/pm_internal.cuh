@@ -366,6 +366,17 @@ struct System {
     cudaGraphExec_t exec = nullptr;
     long long kernels = 0;  // own kernels per replay
   } graphs[2];
+  // captured evaluations (eval_run in api.cu): one per kind of call, the
+  // whole of it as one graph launch
+  struct EvalGraph {
+    int version = -1;
+    unsigned long long key = 0;
+    int uses = 0;  // eager evaluations of this kind so far
+    cudaGraphExec_t exec = nullptr;
+    long long kernels = 0;
+    std::vector<int> forms;  // pair-kernel form of each list it leaves
+  };
+  std::vector<EvalGraph> evals;
   struct PendingRun {
     int active = 0;
     pmgpu_integrator integ{};
@@ -571,6 +582,10 @@ int update_args(System *s, const pmgpu_integrator *it, int phase, int zero_acc,
                 NeighborList *list, UpdateArgs *out);
 int update_blocks(const System *s);
 int set_device_step(System *s);
+// the forces into the pinned staging buffer (enqueued); then from there
+// into out, once the stream is done
+int forces_enqueue(System *s);
+void forces_take(System *s, double *out, int add);
 int forces_to_host(System *s, double *out, int add);
 
 }  // namespace pmgpu
