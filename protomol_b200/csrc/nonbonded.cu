@@ -1228,6 +1228,18 @@ static int spec_kind(const SwitchParams &sw) {
   return -2;
 }
 
+static int sm_count() {
+  static int sms = 0;
+  if (!sms) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        sms <= 0)
+      sms = 148;
+  }
+  return sms;
+}
+
 // Warps per i cluster of the tile kernel: about four waves of the
 // force-only kernel's resident warps (40 per SM), at most kPairMaxSplits per
 // cluster, so blocks that finish early are refilled and the tail stays
@@ -1238,15 +1250,7 @@ static int spec_kind(const SwitchParams &sw) {
 // system, so every launch of a system sums its forces in the same order.
 constexpr int kPairMaxSplits = 32;
 static int pair_splits(int nclusters) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        sms <= 0)
-      sms = 148;
-  }
-  const long long want = 4LL * sms * 40;
+  const long long want = 4LL * sm_count() * 40;
   return (int)std::max(1LL, std::min((long long)kPairMaxSplits, (want + nclusters / 2) / std::max(1, nclusters)));
 }
 
@@ -1265,28 +1269,44 @@ static void launch_pairs_spec(PairArgs<Real> &a, cudaStream_t st, int mode) {
   }
 }
 
-// Work items per i cluster of the j-lane force-only kernel: about three
-// waves of its resident warps (3 blocks of 8 warps per SM), at most 8 per
-// cluster.  Depends only on the system, so every launch of a system sums
-// its forces in the same order.
+// Warps per i cluster of the j-lane force-only kernel, from the warps that
+// are resident at once (3 blocks of 8 per SM).  A cluster's split costs its
+// staging and its i forces once more, so a small system takes as many (at
+// most 6) as three quarters of that wave hold, which leaves room for the
+// PME kernels beside it, one of two waves' clusters takes 1 and the others
+// 2.  50-step segments with 1 | 2 | 3 | 4 | 6 | 8 warps a cluster, us:
+//   1,000 waters (418 clusters)  2779 | 2151 | 2088 | 2067 | 2060 | 2141
+//   1,667 (682)                  2928 | 2292 | 2207 | 2203 | 2377 | 2389
+//   3,000 (1,213)                3287 | 2608 | 2768 | 2715 | 2713 | 2766
+//   7,850 (3,116)                4375 | 4255 | 4376 | 4446 | 4693 | 5060
+//   16,666 (6,534)               7166 | 7193 | 7537 | 7796 | 8530 | 9311
+//   20,000 (7,816)               8401 | 8626
+// and 24 boxes of 100 to 1,000 waters as one ensemble: 4440 us with 8 each,
+// 4270 by this rule.  Depends only on the system, so every launch of a
+// system sums its forces in the same order.
 static int jl_splits(int nclusters) {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        sms <= 0)
-      sms = 148;
-  }
+  const int wave = 3 * sm_count() * kJlWarps;
   static int forced = -1;
   if (forced < 0) {
     const char *e = std::getenv("PMGPU_JL_SPLITS");
     forced = e ? std::max(0, std::atoi(e)) : 0;
   }
   if (forced) return std::min(forced, kJlMaxSplits);
-  const long long want = 3LL * sms * 3 * kJlWarps;
-  return (int)std::max(1LL, std::min(8LL, (want + nclusters / 2) / std::max(1, nclusters)));
+  if (nclusters >= 2 * wave) return 1;
+  return std::max(2, std::min(6, wave * 3 / 4 / std::max(1, nclusters)));
 }
+
+// Warps per i cluster of the FP64 energy kernel: two and a quarter waves of
+// its resident warps (2 blocks of 8 per SM), 2 to 12.  Its warps are chains of FP64 latency, so a
+// small system wants more than the force kernel does: one call on 648 atoms
+// with 2 | 4 | 8 | 12 | 16 warps a cluster 94 | 81 | 80 | 72 | 72 us; a large
+// one pays for each split's half-full last queue: 12,000 atoms, 2 | 3 | 4 | 8:
+// 376 | 354 | 362 | 383 us; 49,998 atoms, 2 | 3 | 4: 715 | 722 | 731 us.
+static int e64_splits(int nclusters) {
+  const int want = 2 * sm_count() * kE64Warps * 9 / 4;
+  return std::max(2, std::min(12, want / std::max(1, nclusters)));
+}
+static_assert(kJlMaxSplits >= 12, "splits of a row");
 
 // Raises a kernel's dynamic shared memory (once above 48 KB it must be).
 template <typename K>
@@ -1363,7 +1383,7 @@ static void e64_kernel(int mask, int form, F go) {
     go(k_pairs_e64<LE, VIRIAL, -1, -1>, k_pairs_e64_batch<LE, VIRIAL, -1, -1>);
 }
 
-// The energy launch's shape: work items as the force-only kernel's.
+// The energy launch's shape.
 static int e64_blocks(const PairArgs<float> &a) {
   return (int)(((long long)a.nclusters * a.splits + kE64Warps - 1) / kE64Warps);
 }
@@ -1372,7 +1392,7 @@ static size_t e64_smem_bytes() { return kE64Warps * sizeof(E64Warp<VIRIAL>); }
 
 template <bool VIRIAL>
 static cudaError_t launch_e64(PairArgs<float> a, int form, cudaStream_t st) {
-  a.splits = jl_splits(a.nclusters);
+  a.splits = e64_splits(a.nclusters);
   const int nb = e64_blocks(a);
   cudaError_t err = cudaSuccess;
   if (nb)
@@ -1561,7 +1581,7 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
     // the energy kernel of a special form compiles its switches in, so the
     // members without one take a table of their own
     PairArgs<float> ea = a;
-    ea.splits = jl_splits(a.nclusters);
+    ea.splits = e64_splits(a.nclusters);
     (form != PMGPU_PAIRK_GENERIC ? b->energy : b->genergy).add(ea, e64_blocks(ea));
     b->slots.add(SlotArgs{nl->ns_max, s->n, nl->d_sorted, nl->d_fslot, s->d_force},
                  (nl->ns_max + 255) / 256);
