@@ -1561,16 +1561,66 @@ static bool same_integrator(const pmgpu_integrator &a, const pmgpu_integrator &b
          a.temperature == b.temperature && a.gamma_ps == b.gamma_ps && a.seed == b.seed;
 }
 
-// Replays (capturing on first use) a CUDA graph of g inner steps.  *used is
-// 0 when capture is not possible, in which case the caller runs eagerly.
-static int run_graph(System *s, const pmgpu_integrator *it, long g, int *used) {
+// The closing half kick of a run, which also takes the slot forces a
+// force-only evaluation may have left (a run of zero steps).
+static int closing_kick(System *s, const pmgpu_integrator *it) {
+  prof_begin(s, PMGPU_PHASE_INTEGRATE);
+  const int r = integrate_kick_drift(s, it, it->kind == PMGPU_INT_LANGEVIN_LEAPFROG ? 5 : 2, 0,
+                                     s->lists.size() == 1 ? &s->lists[0] : nullptr);
+  prof_end(s);
+  PM_CHECK(r);
+  s->kernels += s->n > 0;
+  return PMGPU_OK;
+}
+
+// The parts of a run that are captured: kGraphSteps inner steps, one inner
+// step, the first step (its own kick) and the last step (energies) with the
+// closing kick.
+enum { RUN_MANY, RUN_ONE, RUN_FIRST, RUN_LAST };
+static int run_part(System *s, const pmgpu_integrator *it, int part) {
+  const bool lang = it->kind == PMGPU_INT_LANGEVIN_LEAPFROG;
+  const int inner = lang ? 4 : 1;
+  switch (part) {
+    case RUN_FIRST: return one_step(s, it, lang ? 3 : 0, PAIR_FORCE);
+    case RUN_LAST:
+      PM_CHECK(one_step(s, it, inner, PAIR_ENERGY));
+      return closing_kick(s, it);
+    default:
+      for (long k = 0; k < (part == RUN_MANY ? kGraphSteps : 1); k++)
+        PM_CHECK(one_step(s, it, inner, PAIR_FORCE));
+      return PMGPU_OK;
+  }
+}
+
+// Replays a CUDA graph of a part.  The inner steps are captured at their
+// first use; the first and the last step, of which a run has one each, at
+// the third run with the same integrator: eager, their 17 launches each cost
+// the host more than the device takes (501 to 5,001 atoms with PME, a run of
+// 2 steps 172 to 190 us, replayed 111 to 137; 50 steps of 5,001 atoms
+// 2223 -> 2200 us, of a 2,000-atom polymer 2662 -> 2634).  *used is 0 when
+// the part is to run eagerly (too few uses, a list not built yet, or no
+// capture).
+static int run_graph(System *s, const pmgpu_integrator *it, int part, int *used) {
   *used = 0;
-  System::StepGraph &sg = s->graphs[g == 1 ? 1 : 0];
-  const int phase = it->kind == PMGPU_INT_LANGEVIN_LEAPFROG ? 4 : 1;
-  if (!(sg.exec && sg.version == s->graph_version && sg.steps == g &&
+  if (s->prof.enabled || s->graphs_disabled) return PMGPU_OK;
+  System::StepGraph &sg = s->graphs[part];
+  if (!(sg.version == s->graph_version && sg.count_pairs == s->count_pairs &&
         same_integrator(sg.key, *it))) {
     if (sg.exec) cudaGraphExecDestroy(sg.exec);
     sg.exec = nullptr;
+    sg.version = s->graph_version;
+    sg.count_pairs = s->count_pairs;
+    sg.key = *it;
+    sg.uses = 0;
+  }
+  std::vector<int> in_use(s->lists.size(), 0);
+  for (auto &f : s->forces)
+    if (f.enabled && f.list_index >= 0) in_use[f.list_index] = 1;
+  // the captured launches of a list that is not built would always build it
+  for (size_t k = 0; k < s->lists.size(); k++)
+    if (in_use[k] && !s->lists[k].built) return PMGPU_OK;
+  if (!sg.exec && part >= RUN_FIRST && sg.uses++ < kEvalEager) return PMGPU_OK;
+  if (!sg.exec) {
     long long k0 = s->kernels;
     cudaGraph_t graph = nullptr;
     if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
@@ -1578,8 +1628,7 @@ static int run_graph(System *s, const pmgpu_integrator *it, long g, int *used) {
       s->graphs_disabled = 1;
       return PMGPU_OK;
     }
-    int r = PMGPU_OK;
-    for (long k = 0; k < g && r == PMGPU_OK; k++) r = one_step(s, it, phase, PAIR_FORCE);
+    const int r = run_part(s, it, part);
     cudaError_t ec = cudaStreamEndCapture(s->stream, &graph);
     const long long per_launch = s->kernels - k0;
     s->kernels = k0;
@@ -1600,13 +1649,20 @@ static int run_graph(System *s, const pmgpu_integrator *it, long g, int *used) {
       return PMGPU_OK;
     }
     cudaGraphDestroy(graph);
-    sg.version = s->graph_version;
-    sg.steps = g;
-    sg.key = *it;
     sg.kernels = per_launch;
+    sg.lists.clear();
+    for (auto &nl : s->lists) sg.lists.push_back({nl.slot_pending, nl.last_form});
+    sg.rec_fresh = s->rec_fresh;
   }
   PM_CUDA(cudaGraphLaunch(sg.exec, s->stream));
   s->kernels += sg.kernels;
+  // the host state the part leaves
+  for (size_t k = 0; k < s->lists.size(); k++) {
+    if (!in_use[k]) continue;
+    s->lists[k].slot_pending = sg.lists[k].slot_pending;
+    s->lists[k].last_form = sg.lists[k].last_form;
+  }
+  s->rec_fresh = sg.rec_fresh;
   *used = 1;
   return PMGPU_OK;
 }
@@ -1667,33 +1723,26 @@ static int run_enqueue(System *s, const pmgpu_integrator *it, long n_steps) {
     PM_CHECK(evaluate_forces(s, -1, PAIR_FORCE, 0));
   }
   for (long k = 0; k < n_steps;) {
-    // Inner steps (not the first, not the last) replay a captured graph
-    // of several steps when possible; the rest run eagerly.
-    const long inner_left = (n_steps - 1) - k;
-    if (k > 0 && inner_left > 0 && !s->prof.enabled && !s->graphs_disabled) {
-      const long g = inner_left >= kGraphSteps ? kGraphSteps : 1;
-      int used = 0;
-      PM_CHECK(run_graph(s, it, g, &used));
-      if (used) {
-        s->step += g;
-        k += g;
-        continue;
-      }
+    // every part replays a captured graph when possible, else runs eagerly
+    const long left = n_steps - k;
+    const bool inner = k > 0 && left > 1;
+    const int part = inner ? (left > kGraphSteps ? RUN_MANY : RUN_ONE)
+                           : (left == 1 ? RUN_LAST : RUN_FIRST);
+    int used = 0;
+    if (n_steps > 1) PM_CHECK(run_graph(s, it, part, &used));
+    if (used) {
+      const long g = part == RUN_MANY ? kGraphSteps : 1;
+      s->step += g;
+      k += g;
+      if (part == RUN_LAST) return PMGPU_OK;
+      continue;
     }
     int phase = lang ? (k == 0 ? 3 : 4) : (k == 0 ? 0 : 1);
-    PM_CHECK(one_step(s, it, phase, k + 1 == n_steps ? PAIR_ENERGY : PAIR_FORCE));
+    PM_CHECK(one_step(s, it, phase, left == 1 ? PAIR_ENERGY : PAIR_FORCE));
     s->step++;
     k++;
   }
-  prof_begin(s, PMGPU_PHASE_INTEGRATE);
-  // the closing half kick also takes the slot forces a force-only
-  // evaluation may have left (a run of zero steps)
-  int ri = integrate_kick_drift(s, it, lang ? 5 : 2, 0,
-                                s->lists.size() == 1 ? &s->lists[0] : nullptr);
-  prof_end(s);
-  PM_CHECK(ri);
-  s->kernels += s->n > 0;
-  return PMGPU_OK;
+  return closing_kick(s, it);
 }
 
 static int run_start(System *s, const pmgpu_integrator *it, long n_steps) {

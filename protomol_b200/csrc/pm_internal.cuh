@@ -356,16 +356,23 @@ struct System {
   int forces_valid = 0;   // resident forces correspond to resident positions
   uint64_t step = 0;      // RNG counter (host mirror of *d_step)
   unsigned long long *d_step = nullptr;
-  // captured multi-step graphs of pmgpu_run (invalidated by graph_version)
+  // captured steps of pmgpu_run (run_graph in api.cu; invalidated by
+  // graph_version): several inner steps, one, a run's first and its last
   int graph_version = 0;
   int graphs_disabled = 0;
   struct StepGraph {
     int version = -1;
-    long steps = 0;
+    int count_pairs = 0;
     pmgpu_integrator key{};
+    int uses = 0;  // eager steps of this kind so far
     cudaGraphExec_t exec = nullptr;
     long long kernels = 0;  // own kernels per replay
-  } graphs[2];
+    struct ListState {
+      int slot_pending, last_form;
+    };
+    std::vector<ListState> lists;  // the host state it leaves
+    int rec_fresh = 0;
+  } graphs[4];
   // captured evaluations (eval_run in api.cu): one per kind of call, the
   // whole of it as one graph launch
   struct EvalGraph {
