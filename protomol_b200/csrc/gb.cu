@@ -566,6 +566,376 @@ k_gb_force_half(GbArgs a, int tiles, long long items) {
   if (lane == 0 && epair != 0.0) red_add(&a.acc[ACC_COULOMB], to_fixed(epair, kEnergyScale));
 }
 
+// ------------------------------------------- large molecules, packed FP32
+// The three passes with two j atoms per instruction (packed FP32): a work
+// item is a whole 32 x 32 tile pair, lane l holds atom 32 I + l and the j
+// atoms sit in the warp's shared memory by twos.  The main loop has no
+// branches: the Born terms take the far series for every pair, near pairs
+// (any lane, either direction) contribute nothing there and go into a mask,
+// and a loop after the item's 32 j atoms adds the closed form of each lane's
+// near pairs, j side by atomics.  In the passes above a near pair of one
+// lane sends the whole warp through the closed form of both directions: a
+// fifth of the pairs of a compact 8,191-atom molecule.  8,191 atoms, the
+// passes above and these: force 194 -> 141 us, burial 110 -> 86, partial
+// 80 -> 61, the evaluation 414 -> 301; FP32 issue bounds them.
+//
+// For molecules that give every warp several items (gb_packed): with fewer
+// the passes are bound by the latency of an item, which the finer items
+// above shorten (2,000 atoms, packed: force 19.2 against 18.2 us, burial
+// 13.4 against 12.9, partial 9.3 against 8.9).
+// Distance vectors and squared distances of a lane's atom to pair m.
+struct GbPair2 {
+  float2 dx, dy, dz, r2;
+};
+__device__ __forceinline__ GbPair2 gb_pair2(float4 xyh, float2 zh, float4 xyl, float2 zl,
+                                            const float4 &hi, const float4 &li) {
+  GbPair2 p;
+  p.dx = add2(add2(make_float2(xyh.x, xyh.y), f2(-hi.x)),
+              add2(make_float2(xyl.x, xyl.y), f2(-li.x)));
+  p.dy = add2(add2(make_float2(xyh.z, xyh.w), f2(-hi.y)),
+              add2(make_float2(xyl.z, xyl.w), f2(-li.y)));
+  p.dz = add2(add2(zh, f2(-hi.z)), add2(zl, f2(-li.z)));
+  p.r2 = fma2(p.dz, p.dz, fma2(p.dy, p.dy, mul2(p.dx, p.dx)));
+  return p;
+}
+
+// gb_far of both directions of a pair: dist beyond rho~ + S rho~ of the
+// partner and beyond 4 S rho~ of it, for either atom as the partner.
+__device__ __forceinline__ float gb_far_from(float oi, float soi, float oj, float soj) {
+  return fmaxf(fmaxf(oi + soj, soj * (1.0f / kGbFarT)), fmaxf(oj + soi, soi * (1.0f / kGbFarT)));
+}
+
+__device__ __forceinline__ float2 gb_series_term2(float2 u) {
+  float2 p = fma2(f2(16.0f / 17.0f), u, f2(14.0f / 15.0f));
+  p = fma2(p, u, f2(12.0f / 13.0f));
+  p = fma2(p, u, f2(10.0f / 11.0f));
+  p = fma2(p, u, f2(8.0f / 9.0f));
+  p = fma2(p, u, f2(6.0f / 7.0f));
+  p = fma2(p, u, f2(4.0f / 5.0f));
+  return fma2(p, u, f2(2.0f / 3.0f));
+}
+__device__ __forceinline__ float2 gb_series_dbt2(float2 u) {
+  float2 p = fma2(f2(144.0f / 17.0f), u, f2(112.0f / 15.0f));
+  p = fma2(p, u, f2(84.0f / 13.0f));
+  p = fma2(p, u, f2(60.0f / 11.0f));
+  p = fma2(p, u, f2(40.0f / 9.0f));
+  p = fma2(p, u, f2(24.0f / 7.0f));
+  p = fma2(p, u, f2(12.0f / 5.0f));
+  return fma2(p, u, f2(4.0f / 3.0f));
+}
+
+// The pairs of one lane's i atom with a tile's j atoms that count: i and j
+// atoms that exist, each unordered pair once (j after i on the diagonal).
+__device__ __forceinline__ unsigned half_mask(int n, int i, int I, int J, int lane) {
+  const int jn = n - 32 * J;
+  unsigned m = i < n ? (jn >= 32 ? ~0u : (1u << jn) - 1u) : 0u;
+  if (I == J) m &= ~((2u << lane) - 1u);
+  return m;
+}
+
+// Burial sums, both directions per pair.  Water atoms neither receive nor
+// give burial.
+struct GbBurialWarp {
+  float4 xyh[16], zho[16], xyl[16], zls[16];  // x y | z rho~ | x y (low) | z (low) S rho~
+  float ioj[32];                              // 1 / rho~
+};
+
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+k_gb_burial_packed(GbArgs a, int tiles, long long items) {
+  __shared__ GbBurialWarp warps[WARPS];
+  const int lane = threadIdx.x & 31;
+  GbBurialWarp &W = warps[threadIdx.x >> 5];
+  __shared__ int counter;
+  if (threadIdx.x == 0) counter = 0;
+  __syncthreads();
+  const BlockItems queue{&counter};
+  for (long long w = queue.next(lane); w < items; w = queue.next(lane)) {
+    int I, J;
+    tile_pair_of(w, tiles, &I, &J);
+    const int i = I * 32 + lane;
+    const int ii = i < a.n ? i : 0;
+    const float4 hi = a.rec[ii], li = a.rec[a.n + ii], gi = a.gst[ii];
+    float wj;
+    {
+      const int j = J * 32 + lane;
+      const int jj = j < a.n ? j : 0;
+      const float4 g = a.gst[jj], h = a.rec[jj], l = a.rec[a.n + jj];
+      put_pair(W.xyh, lane, h.x, h.y);
+      put_pair(W.zho, lane, h.z, g.x);
+      put_pair(W.xyl, lane, l.x, l.y);
+      put_pair(W.zls, lane, l.z, g.y);
+      W.ioj[lane] = g.z;
+      wj = g.w;
+    }
+    __syncwarp();
+    unsigned use = half_mask(a.n, i, I, J, lane) & ~__ballot_sync(0xffffffffu, wj != 0.0f);
+    if (gi.w != 0.0f) use = 0u;
+    unsigned near = 0u;
+    float2 own = f2(0.f);
+#pragma unroll 1
+    for (int g = 0; g < 4; g++) {
+      float gb[8];
+      const unsigned gu = use >> (8 * g);
+      unsigned gn = 0u;
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const int m = g * 4 + p;
+        const float4 zo = W.zho[m], zs = W.zls[m];
+        const GbPair2 q = gb_pair2(W.xyh[m], make_float2(zo.x, zo.y), W.xyl[m],
+                                   make_float2(zs.x, zs.y), hi, li);
+        const float2 sj = make_float2(zs.z, zs.w);
+        const float2 id = rsqrt_nr2(q.r2), d = mul2(q.r2, id);
+        const float2 tj = mul2(sj, id), ti = mul2(f2(gi.y), id);
+        const float2 uj = mul2(tj, tj), ui = mul2(ti, ti);
+        const float2 tij = mul2(mul2(id, mul2(tj, uj)), gb_series_term2(uj));
+        const float2 tji = mul2(mul2(id, mul2(ti, ui)), gb_series_term2(ui));
+        const bool ux = (gu >> (2 * p)) & 1u, uy = (gu >> (2 * p + 1)) & 1u;
+        const bool fx = ux && d.x >= gb_far_from(gi.x, gi.y, zo.z, sj.x);
+        const bool fy = uy && d.y >= gb_far_from(gi.x, gi.y, zo.w, sj.y);
+        gn |= (ux && !fx ? 1u << (2 * p) : 0u) | (uy && !fy ? 2u << (2 * p) : 0u);
+        own = add2(own, make_float2(fx ? tij.x : 0.f, fy ? tij.y : 0.f));
+        gb[2 * p] = fx ? tji.x : 0.f;
+        gb[2 * p + 1] = fy ? tji.y : 0.f;
+      }
+      near |= gn << (8 * g);
+      const float sb = warp_tsum8(gb, lane);
+      const int jt = J * 32 + g * 8 + (lane >> 2);
+      if ((lane & 3) == 0 && jt < a.n) red_add(&a.burial_fx[jt], to_fixed((double)sb, kGbScale));
+    }
+    float bsum = own.x + own.y;
+    while (near) {
+      const int k = __ffs(near) - 1, m = k >> 1;
+      near &= near - 1u;
+      const float *xh = &W.xyh[m].x + (k & 1), *zo = &W.zho[m].x + (k & 1),
+                  *xl = &W.xyl[m].x + (k & 1), *zs = &W.zls[m].x + (k & 1);
+      const float dx = (xh[0] - hi.x) + (xl[0] - li.x), dy = (xh[2] - hi.y) + (xl[2] - li.y),
+                  dz = (zo[0] - hi.z) + (zs[0] - li.z);
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      const float id = rsqrt_nr(r2), d = r2 * id;
+      bsum += gb_burial_term_f32(d, id, gi.x, gi.z, zs[2]);
+      red_add(&a.burial_fx[J * 32 + k],
+              to_fixed((double)gb_burial_term_f32(d, id, zo[2], W.ioj[k], gi.y), kGbScale));
+    }
+    if (use) red_add(&a.burial_fx[i], to_fixed((double)bsum, kGbScale));
+    __syncwarp();
+  }
+}
+
+// Partial sums: partialTerm[i][j] adds to i in the lane and
+// partialTerm[j][i] to j.
+struct GbPartialWarp {
+  float4 xyh[16], zhq[16], xyl[16], zlr[16];  // x y | z q | x y (low) | z (low) R
+  float2 ir[16];                              // 1 / R
+};
+
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+k_gb_partial_packed(GbArgs a, int tiles, long long items) {
+  constexpr float kLog2e = 1.4426950408889634f;
+  __shared__ GbPartialWarp warps[WARPS];
+  const int lane = threadIdx.x & 31;
+  GbPartialWarp &W = warps[threadIdx.x >> 5];
+  __shared__ int counter;
+  if (threadIdx.x == 0) counter = 0;
+  __syncthreads();
+  const BlockItems queue{&counter};
+  for (long long w = queue.next(lane); w < items; w = queue.next(lane)) {
+    int I, J;
+    tile_pair_of(w, tiles, &I, &J);
+    const int i = I * 32 + lane;
+    const int ii = i < a.n ? i : 0;
+    const float4 hi = a.rec[ii], li = a.rec[a.n + ii], ri = a.grad[ii];
+    {
+      const int j = J * 32 + lane;
+      const int jj = j < a.n ? j : 0;
+      const float4 h = a.rec[jj], l = a.rec[a.n + jj], r = a.grad[jj];
+      put_pair(W.xyh, lane, h.x, h.y);
+      put_pair(W.zhq, lane, h.z, h.w);
+      put_pair(W.xyl, lane, l.x, l.y);
+      put_pair(W.zlr, lane, l.z, r.x);
+      (&W.ir[0].x)[lane] = r.y;
+    }
+    __syncwarp();
+    const unsigned use = half_mask(a.n, i, I, J, lane);
+    const float q4bi = 0.25f * ri.y;
+    float2 own = f2(0.f);
+#pragma unroll 1
+    for (int g = 0; g < 4; g++) {
+      float gp[8];
+      const unsigned gu = use >> (8 * g);
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const int m = g * 4 + p;
+        const float4 zq = W.zhq[m], zr = W.zlr[m];
+        const float2 r2 = gb_pair2(W.xyh[m], make_float2(zq.x, zq.y), W.xyl[m],
+                                   make_float2(zr.x, zr.y), hi, li).r2;
+        const float2 rj = make_float2(zr.z, zr.w), ir = W.ir[m];
+        const float2 x = mul2(r2, f2(q4bi));
+        const float2 y = mul2(mul2(x, ir), f2(-kLog2e));
+        const float2 ex = make_float2(exp2f_fast(y.x), exp2f_fast(y.y));
+        const float2 fi = rsqrt_nr2(fma2(mul2(f2(ri.x), rj), ex, r2));
+        const float2 pp = mul2(mul2(mul2(f2(0.5f * hi.w), make_float2(zq.z, zq.w)),
+                                    mul2(fi, mul2(fi, fi))), ex);
+        // aTerm of both directions (GBPartialSum.cpp:33)
+        const float2 pij = mul2(pp, add2(rj, x));
+        const float2 pji = mul2(pp, fma2(mul2(r2, f2(0.25f)), ir, f2(ri.x)));
+        const bool ux = (gu >> (2 * p)) & 1u, uy = (gu >> (2 * p + 1)) & 1u;
+        own = add2(own, make_float2(ux ? pij.x : 0.f, uy ? pij.y : 0.f));
+        gp[2 * p] = ux ? pji.x : 0.f;
+        gp[2 * p + 1] = uy ? pji.y : 0.f;
+      }
+      const float sp = warp_tsum8(gp, lane);
+      const int jt = J * 32 + g * 8 + (lane >> 2);
+      if ((lane & 3) == 0 && jt < a.n) red_add(&a.partial_fx[jt], to_fixed((double)sp, kGbScale));
+    }
+    if (use) red_add(&a.partial_fx[i], to_fixed((double)(own.x + own.y), kGbScale));
+    __syncwarp();
+  }
+}
+
+// Forces and pair energy (the grouping of k_gb_force_half).
+struct GbForceWarp {
+  float4 xyh[16], zhq[16], xyl[16], zlr[16];  // x y | z q | x y (low) | z (low) R
+  float4 rd[16], os[16];                      // 1 / R, D | rho~, S rho~
+};
+
+template <int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, 1)
+k_gb_force_packed(GbArgs a, int tiles, long long items) {
+  constexpr float kLog2e = 1.4426950408889634f;
+  __shared__ GbForceWarp warps[WARPS];
+  const int lane = threadIdx.x & 31;
+  GbForceWarp &W = warps[threadIdx.x >> 5];
+  __shared__ int counter;
+  if (threadIdx.x == 0) counter = 0;
+  __syncthreads();
+  const BlockItems queue{&counter};
+  const double d = a.dielec;
+  const float qd = 0.5f * (float)d;
+  double epair = 0.0;
+  for (long long w = queue.next(lane); w < items; w = queue.next(lane)) {
+    int I, J;
+    tile_pair_of(w, tiles, &I, &J);
+    const int i = I * 32 + lane;
+    const int ii = i < a.n ? i : 0;
+    const float4 hi = a.rec[ii], li = a.rec[a.n + ii], gi = a.gst[ii], ri = a.grad[ii];
+    // D_i scaled by the dielectric factor, less the ACE factor A_i
+    const float Di = (float)(d * ((double)ri.w + (double)a.partial_fx[ii] * (1.0 / kGbScale)) *
+                                 (double)ri.z -
+                             (a.ace ? a.ace[ii] : 0.0));
+    {
+      const int j = J * 32 + lane;
+      const int jj = j < a.n ? j : 0;
+      const float4 h = a.rec[jj], l = a.rec[a.n + jj], g = a.gst[jj], r = a.grad[jj];
+      const double Dj =
+          d * ((double)r.w + (double)a.partial_fx[jj] * (1.0 / kGbScale)) * (double)r.z -
+          (a.ace ? a.ace[jj] : 0.0);
+      put_pair(W.xyh, lane, h.x, h.y);
+      put_pair(W.zhq, lane, h.z, h.w);
+      put_pair(W.xyl, lane, l.x, l.y);
+      put_pair(W.zlr, lane, l.z, r.x);
+      put_pair(W.rd, lane, r.y, (float)Dj);
+      put_pair(W.os, lane, g.x, g.y);
+    }
+    __syncwarp();
+    const unsigned use = half_mask(a.n, i, I, J, lane);
+    const float ei = -0.25f * ri.y * kLog2e;
+    unsigned near = 0u;
+    float2 sx = f2(0.f), sy = f2(0.f), sz = f2(0.f), se = f2(0.f);
+#pragma unroll 1
+    for (int g = 0; g < 4; g++) {
+      float gx[8], gy[8], gz[8];
+      const unsigned gu = use >> (8 * g);
+      unsigned gn = 0u;
+#pragma unroll
+      for (int p = 0; p < 4; p++) {
+        const int m = g * 4 + p;
+        const float4 zq = W.zhq[m], zr = W.zlr[m], rd = W.rd[m], os = W.os[m];
+        const GbPair2 q = gb_pair2(W.xyh[m], make_float2(zq.x, zq.y), W.xyl[m],
+                                   make_float2(zr.x, zr.y), hi, li);
+        const float2 id = rsqrt_nr2(q.r2), dist = mul2(q.r2, id);
+        const float2 y = mul2(mul2(q.r2, f2(ei)), make_float2(rd.x, rd.y));
+        const float2 ex = make_float2(exp2f_fast(y.x), exp2f_fast(y.y));
+        const float2 ig =
+            rsqrt_nr2(fma2(mul2(f2(ri.x), make_float2(zr.z, zr.w)), ex, q.r2));
+        const float2 qq = mul2(f2(hi.w), make_float2(zq.z, zq.w));
+        // the far series of both directions, 1/d^3 (D_i .. + D_j ..)
+        const float2 sj = make_float2(os.z, os.w);
+        const float2 tj = mul2(sj, id), ti = mul2(f2(gi.y), id);
+        const float2 uj = mul2(tj, tj), ui = mul2(ti, ti);
+        const float2 bi = mul2(mul2(mul2(tj, uj), f2(-Di)), gb_series_dbt2(uj));
+        const float2 bj = mul2(mul2(ti, ui), mul2(make_float2(rd.z, rd.w), gb_series_dbt2(ui)));
+        const float2 id3 = mul2(mul2(id, id), id);
+        const float2 bt = mul2(id3, fma2(bj, f2(-1.0f), bi));
+        const bool ux = (gu >> (2 * p)) & 1u, uy = (gu >> (2 * p + 1)) & 1u;
+        const bool fx = dist.x >= gb_far_from(gi.x, gi.y, os.x, sj.x);
+        const bool fy = dist.y >= gb_far_from(gi.x, gi.y, os.y, sj.y);
+        gn |= (ux && !fx ? 1u << (2 * p) : 0u) | (uy && !fy ? 2u << (2 * p) : 0u);
+        const float2 pref = mul2(mul2(qq, f2(qd)), mul2(ig, mul2(ig, ig)));
+        // minus the force over the distance
+        const float2 fs = fma2(pref, fma2(ex, f2(-0.5f), f2(2.0f)),
+                               make_float2(fx ? bt.x : 0.f, fy ? bt.y : 0.f));
+        const float2 e = mul2(qq, ig);
+        const float2 f = make_float2(ux ? fs.x : 0.f, uy ? fs.y : 0.f);
+        se = add2(se, make_float2(ux ? e.x : 0.f, uy ? e.y : 0.f));
+        const float2 x = mul2(q.dx, f), v = mul2(q.dy, f), z = mul2(q.dz, f);
+        sx = add2(sx, x);
+        sy = add2(sy, v);
+        sz = add2(sz, z);
+        gx[2 * p] = x.x; gx[2 * p + 1] = x.y;
+        gy[2 * p] = v.x; gy[2 * p + 1] = v.y;
+        gz[2 * p] = z.x; gz[2 * p + 1] = z.y;
+      }
+      near |= gn << (8 * g);
+      const float tx = warp_tsum8(gx, lane), ty = warp_tsum8(gy, lane),
+                  tz = warp_tsum8(gz, lane);
+      // lane l ends with the totals of j atom l >> 2 and adds component l & 3
+      const int jt = J * 32 + g * 8 + (lane >> 2), c = lane & 3;
+      if (c < 3 && jt < a.n)
+        red_add(&a.force[(size_t)c * a.n + jt],
+                to_fixed(-(double)(c == 0 ? tx : (c == 1 ? ty : tz)), kForceScale));
+    }
+    float ax = sx.x + sx.y, ay = sy.x + sy.y, az = sz.x + sz.y;
+    while (near) {
+      const int k = __ffs(near) - 1, m = k >> 1;
+      near &= near - 1u;
+      const float *xh = &W.xyh[m].x + (k & 1), *zq = &W.zhq[m].x + (k & 1),
+                  *xl = &W.xyl[m].x + (k & 1), *zr = &W.zlr[m].x + (k & 1),
+                  *rd = &W.rd[m].x + (k & 1), *os = &W.os[m].x + (k & 1);
+      const float dx = (xh[0] - hi.x) + (xl[0] - li.x), dy = (xh[2] - hi.y) + (xl[2] - li.y),
+                  dz = (zq[0] - hi.z) + (zr[0] - li.z);
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      const float id = rsqrt_nr(r2), dist = r2 * id;
+      const float f = id * (Di * gb_dBT_f32(dist, id, gi.x, os[2]) +
+                            rd[2] * gb_dBT_f32(dist, id, os[0], gi.y));
+      ax += dx * f;
+      ay += dy * f;
+      az += dz * f;
+      long long *fj = a.force + J * 32 + k;
+      red_add(fj, to_fixed(-(double)(dx * f), kForceScale));
+      red_add(fj + a.n, to_fixed(-(double)(dy * f), kForceScale));
+      red_add(fj + 2 * (size_t)a.n, to_fixed(-(double)(dz * f), kForceScale));
+    }
+    if (use) {
+      red_add(&a.force[i], to_fixed((double)ax, kForceScale));
+      red_add(&a.force[a.n + i], to_fixed((double)ay, kForceScale));
+      red_add(&a.force[2 * a.n + i], to_fixed((double)az, kForceScale));
+    }
+    epair -= (double)(se.x + se.y);
+    __syncwarp();
+  }
+  epair = warp_sum(epair) * d;
+  if (lane == 0 && epair != 0.0) red_add(&a.acc[ACC_COULOMB], to_fixed(epair, kEnergyScale));
+}
+
+// Whether a molecule gives every warp of the packed passes two and a half
+// items (from 3,457 atoms on 148 SMs).  One evaluation, the passes above and
+// these: 3,000 atoms 79.5 and 80.6 us, 3,600 104.6 and 92.9, 4,352 128.8 and
+// 107.3.
+constexpr int kGbWarps = 16;
+static bool gb_packed(long long items, int blocks) { return 2 * items >= 5LL * blocks * kGbWarps; }
+
 // Static FP32 record of the GB passes: (rho~ = vdwr - offset, S rho~,
 // 1 / rho~, 1 for water else 0).
 __global__ void k_gb_static(int n, const double *__restrict__ vdwr,
@@ -588,6 +958,14 @@ static void gb_passes_f32(const GbArgs &a, cudaStream_t st) {
   long long items, items2;
   halfpairs_grid(a.n, 1, &tiles, &items, &blocks);
   halfpairs_grid(a.n, 2, &tiles, &items2, &blocks2);
+  if (gb_packed(items, blocks)) {
+    k_gb_burial_packed<24><<<blocks, 24 * 32, 0, st>>>(a, tiles, items);
+    k_gb_radii<<<(a.n + 31) / 32, 32, 0, st>>>(a);
+    if (a.partial_pass)
+      k_gb_partial_packed<kGbWarps><<<blocks, kGbWarps * 32, 0, st>>>(a, tiles, items);
+    k_gb_force_packed<kGbWarps><<<blocks, kGbWarps * 32, 0, st>>>(a, tiles, items);
+    return;
+  }
   k_gb_burial_half<32><<<blocks2, 32 * 32, 0, st>>>(a, tiles, items2);
   // one-warp blocks: they fit beside a resident simple-full block
   k_gb_radii<<<(a.n + 31) / 32, 32, 0, st>>>(a);

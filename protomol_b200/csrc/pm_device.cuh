@@ -160,6 +160,13 @@ __device__ __forceinline__ float rcp_fast(float x) {
   return y;
 }
 
+// 2^x by the hardware estimate (as __expf takes it).
+__device__ __forceinline__ float exp2f_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
 // Sums v[0..7] over the 32 lanes of a warp by a transposed butterfly
 // (9 shuffles): each exchange step hands half of the remaining slots to the
 // partner lane, so lane l ends with the total of slot (l >> 2) & 7, as do
@@ -195,6 +202,12 @@ __device__ __forceinline__ void put_pair(float4 *row, int k, float a, float b) {
   p[0] = a;
   p[2] = b;
 }
+// rsqrt_nr of both
+__device__ __forceinline__ float2 rsqrt_nr2(float2 x) {
+  const float2 y = make_float2(rsqrtf(x.x), rsqrtf(x.y));
+  return mul2(y, fma2(mul2(x, f2(-0.5f)), mul2(y, y), f2(1.5f)));
+}
+
 // The work items of a launch dealt to the blocks round-robin (block b
 // takes items b, b + G, b + 2G, ... of G blocks), so every SM gets the same
 // number of items and the same mix of cheap and dear ones; inside a block
