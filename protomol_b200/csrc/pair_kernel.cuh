@@ -749,7 +749,8 @@ __device__ __forceinline__ float4 jl_lj_pair(const float4 &p0, const float4 &p1,
 // (u) give the cutoff test, the table's range test and its index at once;
 // pairs outside read the table's last interval and are dropped by a select.
 // Warp instructions of a launch 33.2 -> 25.3 M on 23,550 atoms, 46.4 -> 40.4
-// us (caches warm); 49,998 atoms 83.6 -> 70.7 us.  What is left is the
+// us (caches warm; 22.5 M with the two warps a cluster it takes now);
+// 49,998 atoms 83.6 -> 70.7 us.  What is left is the
 // per-entry work (decode, FP64 image shift, staging, three 64-bit force
 // atomics) and the latency of 24 warps an SM.
 // (d = xi - xj here.)  fj gets the sum of f d, i.e. minus the force on j.
