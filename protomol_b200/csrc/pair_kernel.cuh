@@ -954,27 +954,30 @@ __device__ __forceinline__ void pairs_jl_body(const PairArgs<float> &a, Blk blk)
       // modified (scaled 1-4) pairs are rare: batches without any take the
       // path without their selects
       const bool mod = __any_sync(kAll, mm != 0u);
-      if (TAB && !mod && !a.count_pairs) {
+      if (mod) {
+        jl_pairs8<TERMS, SPEC, true, TAB>(a, s_ew, xi, ti, rjx, rjy, rjz, qj, tj, mi, mm, fi, fjx,
+                                          fjy, fjz, band, npairs);
+      } else if constexpr (TAB) {
         float2 fj[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
         bool any = false;
-        if constexpr (TAB)
-          jl_pairs8_x2<SMEM_LJ>(a, s_ew, W, rjx, rjy, rjz, qj, tj, mi, umax, fi, fj, any);
+        jl_pairs8_x2<SMEM_LJ>(a, s_ew, W, rjx, rjy, rjz, qj, tj, mi, umax, fi, fj, any);
         fjx = -(fj[0].x + fj[0].y);
         fjy = -(fj[1].x + fj[1].y);
         fjz = -(fj[2].x + fj[2].y);
-        // which pairs need the exact test (the packed arithmetic's rounding)
-        if (any)
+        // which pairs need the exact test and, when pairs are counted, which
+        // were accepted (the packed arithmetic's rounding): counting must not
+        // change the arithmetic of the forces
+        if (any || a.count_pairs)
           for (int il = 0; il < 8; il++) {
             const float4 x = xi[il];
             const float dx = x.x - rjx, dy = x.y - rjy, dz = x.z - rjz;
             const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
             const bool act =
                 __float_as_uint(r2) - (kEwTabBase << (23 - kEwTabSubBits)) <= umax;
-            if (((mi >> il) & 1u) && !act && r2 <= a.max_hi) band |= 1u << il;
+            if (!((mi >> il) & 1u)) continue;
+            npairs += act;
+            if (!act && r2 <= a.max_hi) band |= 1u << il;
           }
-      } else if (mod) {
-        jl_pairs8<TERMS, SPEC, true, TAB>(a, s_ew, xi, ti, rjx, rjy, rjz, qj, tj, mi, mm, fi, fjx,
-                                          fjy, fjz, band, npairs);
       } else {
         jl_pairs8<TERMS, SPEC, false, TAB>(a, s_ew, xi, ti, rjx, rjy, rjz, qj, tj, mi, mm, fi,
                                            fjx, fjy, fjz, band, npairs);
