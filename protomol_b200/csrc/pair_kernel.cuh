@@ -351,6 +351,38 @@ __device__ __forceinline__ long long fixed_force(float v) {
 }
 __device__ __forceinline__ long long fixed_force(double v) { return to_fixed(v, kForceScale); }
 
+// The energies and virial of a block's pairs into the accumulators: v holds
+// a lane's LJ energy, Coulomb (and Ewald) energy and the virial's upper
+// triangle.  Summed over the block in FP64 and rounded to fixed point once a
+// block (once a warp would leave an error growing with the splits).  Every
+// thread of the block calls it.
+template <int TERMS, bool VIRIAL, int WARPS>
+__device__ __forceinline__ void block_energies(long long *acc, const double (&v)[8]) {
+  constexpr int N = VIRIAL ? 8 : 2;
+  __shared__ double s_e[WARPS][N];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const double t = warp_sum(v[q]);
+    if (lane == 0) s_e[wib][q] = t;
+  }
+  __syncthreads();
+  const int q = threadIdx.x;
+  if (q >= N) return;
+  double t = 0.0;
+  for (int w = 0; w < WARPS; w++) t += s_e[w][q];
+  const long long fixed = to_fixed(t, kEnergyScale);
+  if (q == 0) {
+    if (TERMS & TERM_LJ) red_add(&acc[ACC_LJ], fixed);
+  } else if (q == 1) {
+    if (TERMS & (TERM_COUL | TERM_EWALD)) red_add(&acc[ACC_COULOMB], fixed);
+  } else {
+    const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
+    for (int k = 0; k < 9; k++)
+      if (map[k] == q - 2) red_add(&acc[ACC_VIRIAL + k], fixed);
+  }
+}
+
 // One warp per (8-atom i cluster, contiguous share of its tiles).  Lane
 // l holds pair (i atom l & 7, j atom l >> 3) of every 8 x 4 tile, so a
 // tile's 32 pairs are evaluated at once with no compaction.  The list holds
@@ -381,22 +413,21 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   double Elj = 0, Ec = 0;
   Real vxx = 0, vxy = 0, vxz = 0, vyy = 0, vyz = 0, vzz = 0;
   int npairs = 0;
-  // work items (i cluster, share of its tiles); the warps of a smaller
-  // grid stride over them
-  const int nitems = a.nclusters * a.splits;
-  for (int gw = blk.x * kPairWarps + (threadIdx.x >> 5); gw < nitems;
-       gw += blk.n * kPairWarps) {
-  const int ci = gw / a.splits, sp = gw - ci * a.splits;
+  // this warp's work item (i cluster, share of its tiles)
+  const int wib = threadIdx.x >> 5, gw = blk.x * kPairWarps + wib;
+  const bool item = gw < a.nclusters * a.splits;
+  const int ci = item ? gw / a.splits : 0, sp = gw - ci * a.splits;
   // the cluster's tiles are its kRowParts rows read one after the other;
   // this warp takes tiles [t0, t1) of that sequence
   static_assert(kRowParts == 4, "one int4 of row counts per cluster");
   const int4 c4 = *reinterpret_cast<const int4 *>(a.tile_count + kRowParts * ci);
-  const int cnt = c4.x + c4.y + c4.z + c4.w;
+  const int cnt = item ? c4.x + c4.y + c4.z + c4.w : 0;
   const int t0 = (int)((long long)cnt * sp / a.splits);
   const int t1 = (int)((long long)cnt * (sp + 1) / a.splits);
-  if (t1 <= t0) continue;
   const int islot = 8 * ci + il;
   const int oi = a.sorted[islot];
+  Real fx = 0, fy = 0, fz = 0;
+  if (t1 > t0) {
   const double4 wi = a.xw[islot];  // the FP64 kernel only
   Real xi_h[3], xi_l[3];
   Real qi;
@@ -416,7 +447,6 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   int cur = kZeroShift;
   Real xs_h[3] = {xi_h[0], xi_h[1], xi_h[2]};
   Real xs_l[3] = {xi_l[0], xi_l[1], xi_l[2]};
-  Real fx = 0, fy = 0, fz = 0;
   constexpr int kAllTerms = ((TERMS & TERM_LJ) ? kQLJ : 0) | ((TERMS & TERM_COUL) ? kQCoul : 0) |
                             ((TERMS & TERM_EWALD) ? kQEwald : 0);
   // tile t0 is index kb of row part p; the warp walks the parts in order
@@ -589,6 +619,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
       kb = 0;
     }
   }
+  }  // tiles
   // i's share: summed over the 4 j lanes of each i atom
 #pragma unroll
   for (int o = 8; o < 32; o <<= 1) {
@@ -596,35 +627,41 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
     fy += __shfl_xor_sync(kAll, fy, o);
     fz += __shfl_xor_sync(kAll, fz, o);
   }
-  if (jl == 0 && oi >= 0) {
-    red_add(&a.fslot[islot], fixed_force(fx));
-    red_add(&a.fslot[a.ns + islot], fixed_force(fy));
-    red_add(&a.fslot[2 * a.ns + islot], fixed_force(fz));
+  if constexpr (MIXED) {
+    if (jl == 0 && oi >= 0 && t1 > t0) {
+      red_add(&a.fslot[islot], fixed_force(fx));
+      red_add(&a.fslot[a.ns + islot], fixed_force(fy));
+      red_add(&a.fslot[2 * a.ns + islot], fixed_force(fz));
+    }
+  } else {
+    // in FP64 the rounding to fixed point is the forces' only error: the
+    // block's warps of one cluster add up first, so that an atom's i share is
+    // rounded once a block, not once a warp
+    __shared__ double s_f[kPairWarps][24];
+    __shared__ int s_ci[kPairWarps];
+    if (jl == 0) {
+      s_f[wib][il] = fx;
+      s_f[wib][8 + il] = fy;
+      s_f[wib][16 + il] = fz;
+    }
+    if (lane == 0) s_ci[wib] = item ? ci : -1;
+    __syncthreads();
+    if (item && (wib == 0 || s_ci[wib - 1] != ci) && lane < 24) {
+      double f = 0.0;
+      for (int w = wib; w < kPairWarps && s_ci[w] == ci; w++) f += s_f[w][lane];
+      const int slot = 8 * ci + (lane & 7);
+      if (f != 0.0 && a.sorted[slot] >= 0)
+        red_add(&a.fslot[(lane >> 3) * a.ns + slot], fixed_force(f));
+    }
   }
-  }  // work items
   if (ENERGY || a.count_pairs) {
     int np = warp_sum(npairs);
     if (lane == 0) red_add(&a.acc[ACC_PAIRS], (long long)np);
   }
-  if (ENERGY) {
-    double dlj = warp_sum(Elj);
-    double dc = warp_sum(Ec);
-    double V[6] = {0, 0, 0, 0, 0, 0};
-    if (VIRIAL) {
-      V[0] = warp_sum((double)vxx); V[1] = warp_sum((double)vxy);
-      V[2] = warp_sum((double)vxz); V[3] = warp_sum((double)vyy);
-      V[4] = warp_sum((double)vyz); V[5] = warp_sum((double)vzz);
-    }
-    if (lane == 0) {
-      if (TERMS & TERM_LJ) red_add(&a.acc[ACC_LJ], to_fixed(dlj, kEnergyScale));
-      if (TERMS & (TERM_COUL | TERM_EWALD))
-        red_add(&a.acc[ACC_COULOMB], to_fixed(dc, kEnergyScale));
-      if (VIRIAL) {
-        const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-        for (int q = 0; q < 9; q++)
-          red_add(&a.acc[ACC_VIRIAL + q], to_fixed(V[map[q]], kEnergyScale));
-      }
-    }
+  if constexpr (ENERGY) {
+    const double v[8] = {Elj,         Ec,          (double)vxx, (double)vxy,
+                         (double)vxz, (double)vyy, (double)vyz, (double)vzz};
+    block_energies<TERMS, VIRIAL, kPairWarps>(a.acc, v);
   }
 }
 

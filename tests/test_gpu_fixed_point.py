@@ -1,0 +1,80 @@
+"""Rounding of FP64 sums to fixed point (2^-32 kcal/mol and kcal/mol/A).
+
+Every add into a fixed-point accumulator rounds its term by up to half a
+unit, so N adds leave an error of sqrt(N / 12) units RMS: the only error of
+FP64 forces and energies that is visible beside the FP64 oracle.  N follows
+from the kernels' layout and the list's counts of clusters and tiles; bounds
+on a few energies carry a factor for the scatter of their RMS over SEEDS
+systems (1.5 is the 99.99 % point of 24)."""
+import numpy as np
+import pytest
+
+import oracle
+from protomol_b200 import ForceFactory, GpuSystem, ScalarStructure, systems
+
+pytestmark = pytest.mark.gpu
+
+UNIT = 2.0 ** -32
+SEEDS = 24
+BLOCK = 8  # warps a block of the pair kernels
+
+
+def _water_cluster(seed):
+    """64 waters without periodicity, all within the cutoff of one another, so
+    every tile of the list has pairs."""
+    s = systems.tip3p_box(64, 12.42, seed=seed, lattice=4)
+    s.periodic, s.box = False, np.zeros(12)
+    return s, 30.0
+
+
+def _water_box(seed):
+    """A periodic box, whose atoms nearly fill the list's clusters."""
+    return systems.tip3p_box(216, 18.64, seed=seed, jitter=0.2), 8.0
+
+
+def _oracle(s):
+    return oracle.System(pos=s.pos, charge=s.charge, type=s.type, molecule=s.molecule, lj=s.lj,
+                         excl=s.exclusions, periodic=s.periodic, box=s.box)
+
+
+def _cutoff_errors(ctx, make, precision):
+    """Per seed: force errors (n, 3), energy errors (2), virial errors (9) in
+    units, and the list's clusters and tiles."""
+    out = []
+    for seed in range(SEEDS):
+        s, rc = make(seed)
+        gs = GpuSystem(ctx, s, precision)
+        force = ForceFactory(gs, rc).make(
+            f"LennardJones Coulomb -algorithm NonbondedCutoff -switchingFunction C1 -cutoff {rc} "
+            f"-switchingFunction C1 -cutoff {rc} -cutoff {rc}")
+        f, e = np.zeros_like(s.pos), ScalarStructure()
+        force.evaluate(s.pos, f, e, virial=True)
+        st = force.stats()
+        sw = oracle.Switch("C1", rc)
+        fo, eo, vo = oracle.cutoff_force(_oracle(s), rc, rc,
+                                         [("LennardJones", sw), ("Coulomb", sw)])
+        out.append(((f - fo) / UNIT, np.array([e[0] - eo["coulomb"], e[1] - eo["lj"]]) / UNIT,
+                    (e[7:16] - np.asarray(vo).ravel()) / UNIT, st["clusters"],
+                    st["list_entries"]))
+        gs.close()
+    return out
+
+
+def _rms(parts):
+    return float(np.sqrt(np.mean(np.square(np.concatenate([np.ravel(p) for p in parts])))))
+
+
+def test_double_pair_forces(ctx):
+    """An atom takes one add for each tile that has it as a j atom, and for
+    its own cluster, whose tiles go to at most 32 warps, one a block of 8."""
+    got = _cutoff_errors(ctx, _water_cluster, "double")
+    adds = np.mean([4 * tiles / 192 + 32 / BLOCK for *_, tiles in got])
+    assert _rms([g[0] for g in got]) <= np.sqrt(adds / 12)
+
+
+def test_double_pair_energies(ctx):
+    """Energies and virial: one add a block, at most 32 / 8 blocks a cluster."""
+    got = _cutoff_errors(ctx, _water_box, "double")
+    bound = 1.5 * np.sqrt(np.mean([clusters * 32 / BLOCK for *_, clusters, _ in got]) / 12)
+    assert _rms([g[1] for g in got]) <= bound
+    assert _rms([g[2] for g in got]) <= bound
