@@ -1359,20 +1359,9 @@ __device__ __forceinline__ void pairs_e64_body(const PairArgs<float> &a, Blk blk
   }
   if (lane < queued) evaluate(lane);
   const int np = warp_sum(npairs);
-  const double dlj = warp_sum(Elj), dc = warp_sum(Ec);
-  if (VIRIAL)
-    for (int q = 0; q < 6; q++) V[q] = warp_sum(V[q]);
-  if (lane == 0) {
-    red_add(&a.acc[ACC_PAIRS], (long long)np);
-    if (TERMS & TERM_LJ) red_add(&a.acc[ACC_LJ], to_fixed(dlj, kEnergyScale));
-    if (TERMS & (TERM_COUL | TERM_EWALD))
-      red_add(&a.acc[ACC_COULOMB], to_fixed(dc, kEnergyScale));
-    if (VIRIAL) {
-      const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-      for (int q = 0; q < 9; q++)
-        red_add(&a.acc[ACC_VIRIAL + q], to_fixed(V[map[q]], kEnergyScale));
-    }
-  }
+  if (lane == 0) red_add(&a.acc[ACC_PAIRS], (long long)np);
+  const double v[8] = {Elj, Ec, V[0], V[1], V[2], V[3], V[4], V[5]};
+  block_energies<TERMS, VIRIAL, kE64Warps>(a.acc, v);
 }
 
 extern __shared__ __align__(16) unsigned char e64_smem[];

@@ -78,3 +78,12 @@ def test_double_pair_energies(ctx):
     bound = 1.5 * np.sqrt(np.mean([clusters * 32 / BLOCK for *_, clusters, _ in got]) / 12)
     assert _rms([g[1] for g in got]) <= bound
     assert _rms([g[2] for g in got]) <= bound
+
+
+def test_mixed_energies(ctx):
+    """The mixed path's FP64 energies and virial: at most 12 warps a cluster,
+    one add a block."""
+    got = _cutoff_errors(ctx, _water_box, "mixed")
+    bound = 1.5 * np.sqrt(np.mean([clusters * 12 / BLOCK for *_, clusters, _ in got]) / 12)
+    assert _rms([g[1] for g in got]) <= bound
+    assert _rms([g[2] for g in got]) <= bound
