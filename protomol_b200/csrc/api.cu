@@ -650,8 +650,12 @@ int take_results(System *s, int only, double *energies, double *virial, int add,
       return fail(PMGPU_ERR_UNSUPPORTED, "more atoms in one pair-list column than the sort holds");
   }
   double e[PMGPU_E_COUNT], v[9];
-  for (int k = 0; k < PMGPU_E_COUNT; k++) e[k] = (double)s->h_acc[k] / kEnergyScale;
-  for (int k = 0; k < 9; k++) v[k] = (double)s->h_acc[ACC_VIRIAL + k] / kEnergyScale;
+  auto value = [s](int k) {
+    return (double)s->h_acc[k] / kEnergyScale +
+           (double)s->h_acc[ACC_LOW + k] / (kEnergyScale * kLowScale);
+  };
+  for (int k = 0; k < PMGPU_E_COUNT; k++) e[k] = value(k);
+  for (int k = 0; k < 9; k++) v[k] = value(ACC_VIRIAL + k);
   if (energies_valid) constant_terms(s, only, e, v);
   else
     for (int k = 0; k < PMGPU_E_COUNT; k++) e[k] = 0.0;

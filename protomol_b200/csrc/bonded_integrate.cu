@@ -463,6 +463,7 @@ int set_device_step(System *s) {
 }
 
 constexpr int kUpdateThreads = 64;  // small blocks: the update is latency-bound FP64 work
+static_assert(ACC_COUNT <= kUpdateThreads, "the first block clears the accumulators");
 __device__ __forceinline__ void update_body(const UpdateArgs &a, Blk blk) {
   const double *__restrict__ mass = a.mass;
   double *__restrict__ pos = a.pos;

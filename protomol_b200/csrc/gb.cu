@@ -182,7 +182,7 @@ __device__ __forceinline__ Real gb_dBT(Real dist, Real oi, Real oj, Real Sj) {
 }
 
 __global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
-  __shared__ double sm[kRowThreads / 32];
+  __shared__ double sm[kRowWarps];
   RowWarp r;
   double epair = 0.0;
   if (row_warp(a.n, split, &r)) {
@@ -1070,7 +1070,7 @@ namespace pmgpu {
 namespace {
 
 constexpr int kGbStaticMaxAtoms = PMGPU_GB_STATIC_MAX_ATOMS;
-constexpr int kGbStaticAccWords = 32;
+constexpr int kGbStaticAccWords = 64;
 static_assert(ACC_COUNT <= kGbStaticAccWords, "accumulator block too small");
 // per atom: born, psi, partial (double), burial and partial sums (int64),
 // three force planes (int64); then the energy/virial accumulator block;

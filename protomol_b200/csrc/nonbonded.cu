@@ -1859,23 +1859,58 @@ struct SfArgs {
   int em;
 };
 
-// The virial of a warp's pairs (upper triangle) into the accumulators.
-__device__ __forceinline__ void row_virial(long long *acc, double (&v)[6], double *sm) {
-  const int map[9] = {0, 1, 2, 1, 3, 4, 2, 4, 5};
-  for (int q = 0; q < 6; q++) {
-    v[q] = row_block_sum(v[q], sm);
-    if (threadIdx.x == 0)
-      for (int k = 0; k < 9; k++)
-        if (map[k] == q) red_add(&acc[ACC_VIRIAL + k], to_fixed(v[q], kEnergyScale));
+// The energies (em >= 1; v[0] LJ, v[1] Coulomb, of the terms asked for) and
+// virial (em 2; v[2..7] the upper triangle) of a lane's pairs into the
+// accumulators: summed over the block, then one two-word add a slot, a
+// thread each.  Every thread of the block calls it.
+__device__ __forceinline__ void row_energies(long long *acc, int em, bool lj, bool coul,
+                                             const double (&v)[8]) {
+  __shared__ double se[kRowWarps][8];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, t = threadIdx.x;
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    if (q >= 2 && em != 2) break;
+    const double x = warp_sum(v[q]);
+    if (lane == 0) se[wib][q] = x;
   }
+  __syncthreads();
+  if (t >= (em == 2 ? 11 : 2) || (t == 0 && !lj) || (t == 1 && !coul)) return;
+  // threads 2 to 10: the nine entries of the symmetric virial
+  const int row = (t - 2) / 3, col = (t - 2) % 3, lo = min(row, col), hi = max(row, col);
+  const int q = t < 2 ? t : 2 + (lo == 0 ? hi : lo + hi + 1);
+  double x = 0.0;
+#pragma unroll
+  for (int w = 0; w < kRowWarps; w++) x += se[w][q];
+  red_add_energy(acc, t == 0 ? ACC_LJ : (t == 1 ? ACC_COULOMB : ACC_VIRIAL + t - 2), x);
 }
-// The force on atom i, summed over its warp's lanes.
-__device__ __forceinline__ void row_force(long long *force, int n, int i, double fx, double fy,
-                                          double fz) {
+
+// The force on atom i, summed over its warps in the block (split, a power of
+// two, or all of them) and then rounded to fixed point: in FP64 that rounding
+// is the force's only error, and one a warp would make it larger than with
+// one thread an atom.  Every thread of the block calls it.
+__device__ __forceinline__ void row_force(long long *force, int n, int i, int split, double fx,
+                                          double fy, double fz) {
+  __shared__ double sf[kRowWarps][3];
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
   fx = warp_sum(fx);
   fy = warp_sum(fy);
   fz = warp_sum(fz);
-  if ((threadIdx.x & 31) == 0) {
+  const int warps = min(split, kRowWarps);
+  if (warps > 1) {
+    if (lane == 0) {
+      sf[wib][0] = fx;
+      sf[wib][1] = fy;
+      sf[wib][2] = fz;
+    }
+    __syncthreads();
+    if (lane != 0 || (wib & (warps - 1))) return;
+    for (int w = wib + 1; w < wib + warps; w++) {
+      fx += sf[w][0];
+      fy += sf[w][1];
+      fz += sf[w][2];
+    }
+  }
+  if (lane == 0 && i < n) {
     red_add(&force[i], to_fixed(fx, kForceScale));
     red_add(&force[n + i], to_fixed(fy, kForceScale));
     red_add(&force[2 * n + i], to_fixed(fz, kForceScale));
@@ -1884,16 +1919,14 @@ __device__ __forceinline__ void row_force(long long *force, int n, int i, double
 
 template <bool LJ, bool COUL>
 __global__ void __launch_bounds__(kRowThreads) k_simplefull(SfArgs a) {
-  __shared__ double sm[kRowThreads / 32];
   RowWarp r;
-  double elj = 0, ec = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  double elj = 0, ec = 0, fx = 0, fy = 0, fz = 0, v[6] = {0, 0, 0, 0, 0, 0};
   if (row_warp(a.n, a.split, &r)) {
     const int i = r.i;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
     const double qi = a.charge[i];
     const int ti = a.type[i];
     const int2 er = a.ex_range[i];
-    double fx = 0, fy = 0, fz = 0;
     for (int j = r.j0; j < a.n; j += r.dj) {
       if (j == i) continue;
       int excl = PMGPU_EXCL_NONE;
@@ -1928,16 +1961,11 @@ __global__ void __launch_bounds__(kRowThreads) k_simplefull(SfArgs a) {
       }
     }
     __syncwarp();
-    row_force(a.force, a.n, i, fx, fy, fz);
   }
+  row_force(a.force, a.n, r.i, a.split, fx, fy, fz);
   if (!a.em) return;
-  elj = row_block_sum(elj, sm) * 0.5;
-  ec = row_block_sum(ec, sm) * 0.5;
-  if (threadIdx.x == 0) {
-    if (LJ) red_add(&a.acc[ACC_LJ], to_fixed(elj, kEnergyScale));
-    if (COUL) red_add(&a.acc[ACC_COULOMB], to_fixed(ec, kEnergyScale));
-  }
-  if (a.em == 2) row_virial(a.acc, v, sm);
+  const double sums[8] = {0.5 * elj, 0.5 * ec, v[0], v[1], v[2], v[3], v[4], v[5]};
+  row_energies(a.acc, a.em, LJ, COUL, sums);
 }
 
 // NonbondedSimpleFull with switching functions: OneAtomPair /
@@ -1987,9 +2015,8 @@ __device__ __forceinline__ void scpism_pair(double qq, double sai, double saj, d
 }
 
 __global__ void __launch_bounds__(kRowThreads) k_simplefull_sw(SfSwArgs a) {
-  __shared__ double sm[kRowThreads / 32];
   RowWarp r;
-  double elj = 0, ec = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  double elj = 0, ec = 0, fx = 0, fy = 0, fz = 0, v[6] = {0, 0, 0, 0, 0, 0};
   if (row_warp(a.n, a.split, &r)) {
     const int i = r.i;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
@@ -1998,7 +2025,6 @@ __global__ void __launch_bounds__(kRowThreads) k_simplefull_sw(SfSwArgs a) {
     const bool wi = a.water && a.water[i];
     const int ti = a.type[i], mi = a.mol[i];
     const int2 er = a.ex_range[i];
-    double fx = 0, fy = 0, fz = 0;
     for (int j = r.j0; j < a.n; j += r.dj) {
       if (j == i) continue;
       double dx, dy, dz;
@@ -2064,16 +2090,11 @@ __global__ void __launch_bounds__(kRowThreads) k_simplefull_sw(SfSwArgs a) {
       }
     }
     __syncwarp();
-    row_force(a.force, a.n, i, fx, fy, fz);
   }
+  row_force(a.force, a.n, r.i, a.split, fx, fy, fz);
   if (!a.em) return;
-  elj = row_block_sum(elj, sm) * 0.5;
-  ec = row_block_sum(ec, sm) * 0.5;
-  if (threadIdx.x == 0) {
-    if (a.lj) red_add(&a.acc[ACC_LJ], to_fixed(elj, kEnergyScale));
-    if (a.coul) red_add(&a.acc[ACC_COULOMB], to_fixed(ec, kEnergyScale));
-  }
-  if (a.em == 2) row_virial(a.acc, v, sm);
+  const double sums[8] = {0.5 * elj, 0.5 * ec, v[0], v[1], v[2], v[3], v[4], v[5]};
+  row_energies(a.acc, a.em, a.lj, a.coul, sums);
 }
 
 // The FP32 pass over each unordered pair once, as the reference visits
@@ -2464,13 +2485,11 @@ __global__ void __launch_bounds__(kRowThreads) k_born_radii(BornArgs a) {
 }
 
 __global__ void __launch_bounds__(kRowThreads) k_born_self(BornArgs a) {
-  __shared__ double sm[kRowThreads / 32];
   RowWarp w;
   const int n = a.n;
-  double e = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  double e = 0, fx = 0, fy = 0, fz = 0, v[6] = {0, 0, 0, 0, 0, 0};
   if (row_warp(n, 1, &w)) {
     const int i = w.i;
-    double fx = 0, fy = 0, fz = 0;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
     const double eta = a.scp[3 * n + i], C = a.scp[4 * n + i], Qi = a.born_q[i];
     const int2 er = a.ex_range[i];
@@ -2505,12 +2524,11 @@ __global__ void __launch_bounds__(kRowThreads) k_born_self(BornArgs a) {
     // the self energy of every atom that took part in a pair
     // (BornSelfForce.h:108-117, postProcess :128-135)
     if (__any_sync(0xffffffffu, used) && (threadIdx.x & 31) == 0) e = a.born_q[n + i];
-    row_force(a.force, n, i, fx, fy, fz);
   }
+  row_force(a.force, n, w.i, 1, fx, fy, fz);
   if (!a.em) return;
-  e = row_block_sum(e, sm);
-  if (threadIdx.x == 0) red_add(&a.acc[ACC_COULOMB], to_fixed(e, kEnergyScale));
-  if (a.em == 2) row_virial(a.acc, v, sm);
+  const double sums[8] = {0.0, e, v[0], v[1], v[2], v[3], v[4], v[5]};
+  row_energies(a.acc, a.em, false, true, sums);
 }
 
 int nb_born(System *s, const Force &f, int em) {

@@ -380,6 +380,16 @@ __device__ __forceinline__ void red_add(long long *p, long long v) {
             static_cast<unsigned long long>(v));
 }
 
+// v into energy or virial slot `slot` in two words: what rounding to
+// kEnergyScale leaves goes into the slot's low word, so the sum of many adds
+// is as exact as the FP64 sums that it adds.
+__device__ __forceinline__ void red_add_energy(long long *acc, int slot, double v) {
+  const double x = v * kEnergyScale;
+  const long long q = __double2ll_rn(x);
+  red_add(acc + slot, q);
+  red_add(acc + ACC_LOW + slot, __double2ll_rn((x - (double)q) * kLowScale));
+}
+
 // Pair-list rebuild decision, taken on the device by the last block of a
 // grid to finish: every thread passes the squared displacement of its atom
 // from its position at the last build (0 for no atom); the list is rebuilt
@@ -469,11 +479,12 @@ __device__ __forceinline__ const A &batch_args_shared(const A *__restrict__ tab,
 // Coulomb 80 -> 7.1, GB burial 40 -> 9.1, partial 28 -> 6.4, force 115 ->
 // 17.4 us.
 constexpr int kRowThreads = 128;
+constexpr int kRowWarps = kRowThreads / 32;
 struct RowWarp {
   int i, j0, dj;  // atom, this lane's first partner, partner stride
 };
 __device__ __forceinline__ bool row_warp(int n, int split, RowWarp *r) {
-  const int gw = blockIdx.x * (kRowThreads / 32) + (threadIdx.x >> 5);
+  const int gw = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
   r->i = gw / split;
   r->j0 = (gw - r->i * split) * 32 + (threadIdx.x & 31);
   r->dj = 32 * split;
@@ -487,8 +498,7 @@ __host__ inline int row_split(int n) {
   return s;
 }
 __host__ inline int row_blocks(int n, int split) {
-  const int per = kRowThreads / 32;
-  return (int)(((long long)n * split + per - 1) / per);
+  return (int)(((long long)n * split + kRowWarps - 1) / kRowWarps);
 }
 // Sums v over the block's warps (each lane's v first summed over its warp);
 // thread 0 returns the total.  Every thread calls it; kRowThreads threads.
@@ -500,7 +510,7 @@ __device__ __forceinline__ double row_block_sum(double v, double *sm) {
   __syncthreads();
   double t = 0.0;
   if (threadIdx.x == 0)
-    for (int w = 0; w < kRowThreads / 32; w++) t += sm[w];
+    for (int w = 0; w < kRowWarps; w++) t += sm[w];
   return t;
 }
 

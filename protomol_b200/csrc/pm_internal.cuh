@@ -42,10 +42,14 @@ constexpr double kBoltzmann = 0.001987191;              // PMConstants.cpp:70
 constexpr double kEpsilon = 1.0e-14;                    // PMConstants.cpp:50
 constexpr int kMaxInt2 = 2147483647 / 2;                // PMConstants.cpp:45
 
-// Accumulator slots on the device (int64 fixed point, kEnergyScale).
+// Accumulator slots on the device (int64 fixed point, kEnergyScale): the
+// energies, the virial and the pair count, then the low words of energies
+// and virial (units of 1 / (kEnergyScale kLowScale)) that the passes with
+// many small adds keep beside them (red_add_energy).
 enum { ACC_COULOMB = 0, ACC_LJ, ACC_BOND, ACC_ANGLE, ACC_DIHEDRAL,
        ACC_IMPROPER, ACC_OTHER, ACC_VIRIAL = 7, ACC_PAIRS = 16,
-       ACC_COUNT = 18 };
+       ACC_LOW = 18, ACC_COUNT = ACC_LOW + 16 };
+constexpr double kLowScale = 16777216.0;  // 2^24
 
 // Status word bits (device side).
 enum { ST_LIST_OVERFLOW = 1, ST_NONFINITE = 2, ST_CELL_OVERFLOW = 4,

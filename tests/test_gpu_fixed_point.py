@@ -6,6 +6,8 @@ FP64 forces and energies that is visible beside the FP64 oracle.  N follows
 from the kernels' layout and the list's counts of clusters and tiles; bounds
 on a few energies carry a factor for the scatter of their RMS over SEEDS
 systems (1.5 is the 99.99 % point of 24)."""
+import math
+
 import numpy as np
 import pytest
 
@@ -87,3 +89,46 @@ def test_mixed_energies(ctx):
     bound = 1.5 * np.sqrt(np.mean([clusters * 12 / BLOCK for *_, clusters, _ in got]) / 12)
     assert _rms([g[1] for g in got]) <= bound
     assert _rms([g[2] for g in got]) <= bound
+
+
+def _coulomb_pairs(s, rc=0.0):
+    """Coulomb (with rc: C1 switched) energy and virial of every pair of a
+    molecule, summed exactly, and the sums of their absolute values."""
+    i, j = np.triu_indices(len(s.pos), 1)
+    scale = np.ones((len(s.pos),) * 2)
+    for a, b, kind in s.exclusions:
+        scale[a, b] = scale[b, a] = 0.0 if kind == 2 else s.coulomb_scaling
+    d = s.pos[j] - s.pos[i]
+    r2 = (d * d).sum(1)
+    r = np.sqrt(r2)
+    e = scale[i, j] * s.charge[i] * s.charge[j] / r
+    f = e / r2
+    if rc:  # C1SwitchingFunction.h:41-50
+        value = 1.0 - 1.5 * r / rc + 0.5 * (r / rc) ** 3
+        f = f * value - e * (-1.5 / rc + 1.5 * r2 / rc ** 3) / r
+        e = e * value
+    v = d[:, :, None] * d[:, None, :] * f[:, None, None]
+    terms = np.concatenate([e[:, None], v.reshape(-1, 9)], 1)
+    return np.array([math.fsum(t) for t in terms.T]), np.abs(terms).sum(0)
+
+
+@pytest.mark.parametrize("rc", [0.0, 400.0], ids=["plain", "switched"])
+@pytest.mark.parametrize("n", [3, 64, 200, 296, 297, 547, 1185])
+def test_row_passes(ctx, n, rc):
+    """The FP64 all-pairs passes: one add an atom (two where eight warps share
+    it, 129 to 296 atoms), each within half a unit; energies and virial in two words, so only their FP64 sums' rounding
+    is left (16 roundings of the terms' absolute sum, far less than it takes)."""
+    s = systems.gb_polymer(n, seed=n)
+    gs = GpuSystem(ctx, s, "double")
+    sw = f" -switchingFunction C1 -cutoff {rc}" if rc else ""
+    force = ForceFactory(gs).make("Coulomb -algorithm NonbondedSimpleFull" + sw)
+    f, e = np.zeros_like(s.pos), ScalarStructure()
+    force.evaluate(s.pos, f, e, virial=True)
+    gs.close()
+    o = _oracle(s)
+    fo = oracle.simplefull_force(o, "Coulomb", oracle.Switch("C1", rc) if rc else None)[0]
+    # a thousandth of a unit (2.3e-13) for the FP64 sums of forces up to 30
+    assert np.abs(f - fo).max() <= (0.5 * (2 if 128 < n <= 296 else 1) + 1e-3) * UNIT
+    exact, size = _coulomb_pairs(s, rc)
+    got = np.concatenate([[e[0]], e[7:16]])
+    assert (np.abs(got - exact) <= 16 * 2.0 ** -53 * size + 2.0 ** -50).all()
