@@ -1152,9 +1152,10 @@ static void fill_pair_args(PairArgs<Real> &a, System *s, NeighborList *nl,
   a.coul_sw64 = make_switch_dev<double>(t.coul_sw);
   a.lj_modify = t.lj_sw.modify;
   a.coul_modify = t.coul_sw.modify;
-  // The FP32 squared distance is within ~1e-5 A^2 of the exact one; pairs
-  // inside this relative band are re-tested in FP64.
-  const double band = sizeof(Real) == 4 ? 4.0e-5 : 1.0e-12;
+  // The FP32 squared distance is within ~1e-5 A^2 of the exact one, the FP64
+  // one of wrapped coordinates within their rounding (kBand64); pairs inside
+  // this relative band take the reference's test.
+  const double band = sizeof(Real) == 4 ? 4.0e-5 : kBand64;
   a.lj_cut2 = t.lj_cut2;
   a.coul_cut2 = t.coul_cut2;
   a.ew_cut2 = t.ewald_rc2;

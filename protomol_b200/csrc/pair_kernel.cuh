@@ -72,6 +72,12 @@ struct PairArgs {
   int same_sw;           // both cutoff terms take one switch (the same constants)
 };
 
+// Relative band around a cutoff^2 in which a squared distance formed from
+// the wrapped FP64 coordinates does not decide.  Its error is that of the
+// raw coordinates: 4e-14 of r^2 for atoms at 1e3 A, 3e-11 at 1e6 A; one pair
+// in 1e8 takes the exact test needlessly.
+constexpr double kBand64 = 1.0e-8;
+
 // Exact FP64 squared distance of the image in hand, formed the way the
 // reference forms it: the minimal difference (PeriodicBoundaryConditions.h:
 // 72-110) plus a lattice vector (NonbondedFullEwaldSystemForce.h:790-805;
@@ -1170,7 +1176,6 @@ __device__ __forceinline__ void pairs_e64_body(const PairArgs<float> &a, Blk blk
   E64Warp<VIRIAL> &W = warps[wib];
   constexpr int kAllTerms = ((TERMS & TERM_LJ) ? kQLJ : 0) | ((TERMS & TERM_COUL) ? kQCoul : 0) |
                             ((TERMS & TERM_EWALD) ? kQEwald : 0);
-  constexpr double kBand = 1.0e-12;  // of a squared distance formed in FP64
   double Elj = 0, Ec = 0, V[6] = {0, 0, 0, 0, 0, 0};
   int npairs = 0, queued = 0;  // (queued: the same in every lane)
 
@@ -1288,24 +1293,24 @@ __device__ __forceinline__ void pairs_e64_body(const PairArgs<float> &a, Blk blk
         const double4 wi = W.wi[il];
         const double dx = jx - wi.x, dy = jy - wi.y, dz = jz - wi.z;
         const double r2 = dx * dx + dy * dy + dz * dz;
-        if (!((mi >> il) & 1u) || r2 > a.max_cut2 * (1.0 + kBand)) continue;
+        if (!((mi >> il) & 1u) || r2 > a.max_cut2 * (1.0 + kBand64)) continue;
         int flags = 0;
         bool band = false;
         if (a.same_cut) {
-          if (r2 <= a.max_cut2 * (1.0 - kBand)) flags = kAllTerms;
+          if (r2 <= a.max_cut2 * (1.0 - kBand64)) flags = kAllTerms;
           else band = true;
         } else {
           if (TERMS & TERM_LJ) {
-            if (r2 <= a.lj_cut2 * (1.0 - kBand)) flags |= kQLJ;
-            else band |= r2 <= a.lj_cut2 * (1.0 + kBand);
+            if (r2 <= a.lj_cut2 * (1.0 - kBand64)) flags |= kQLJ;
+            else band |= r2 <= a.lj_cut2 * (1.0 + kBand64);
           }
           if (TERMS & TERM_COUL) {
-            if (r2 <= a.coul_cut2 * (1.0 - kBand)) flags |= kQCoul;
-            else band |= r2 <= a.coul_cut2 * (1.0 + kBand);
+            if (r2 <= a.coul_cut2 * (1.0 - kBand64)) flags |= kQCoul;
+            else band |= r2 <= a.coul_cut2 * (1.0 + kBand64);
           }
           if (TERMS & TERM_EWALD) {
-            if (r2 <= a.ew_cut2 * (1.0 - kBand)) flags |= kQEwald;
-            else band |= r2 <= a.ew_cut2 * (1.0 + kBand);
+            if (r2 <= a.ew_cut2 * (1.0 - kBand64)) flags |= kQEwald;
+            else band |= r2 <= a.ew_cut2 * (1.0 + kBand64);
           }
         }
         if (band) {  // rare: the reference's own arithmetic decides
