@@ -653,8 +653,14 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
     if (lane == 0) s_ci[wib] = item ? ci : -1;
     __syncthreads();
     if (item && (wib == 0 || s_ci[wib - 1] != ci) && lane < 24) {
-      double f = 0.0;
-      for (int w = wib; w < kPairWarps && s_ci[w] == ci; w++) f += s_f[w][lane];
+      double t[kPairWarps];
+#pragma unroll
+      for (int w = 0; w < kPairWarps; w++) t[w] = s_ci[w] == ci ? s_f[w][lane] : 0.0;
+#pragma unroll
+      for (int o = kPairWarps / 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int w = 0; w < o; w++) t[w] += t[w + o];
+      const double f = t[0];
       const int slot = 8 * ci + (lane & 7);
       if (f != 0.0 && a.sorted[slot] >= 0)
         red_add(&a.fslot[(lane >> 3) * a.ns + slot], fixed_force(f));
