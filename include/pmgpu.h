@@ -478,6 +478,11 @@ int pmgpu_profile_read(pmgpu_system *sys, double *ms, long long *launches,
 /* Number of this library's own kernels launched on the system so far
  * (library kernels such as cuFFT's are not counted). */
 int pmgpu_kernel_count(pmgpu_system *sys, long long *count);
+/* CUDA graph launches of the system so far: an evaluation's kind is replayed
+ * from its third call on, a run's inner steps from the first run on, its
+ * first and last step from the third.  Eager work (profiling on, or a capture
+ * that failed: its reason is printed when PMGPU_DEBUG is set) adds none. */
+int pmgpu_graph_replays(pmgpu_system *sys, long long *count);
 
 /* ProtoMol cell assignment (topology/Topology.h:44-86 with
  * CubicCellManager, cellsize given) computed by the device binning kernel

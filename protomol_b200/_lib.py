@@ -46,6 +46,7 @@ EXPORTED = [
     "pmgpu_ensemble_member", "pmgpu_debug_limit_list_rows", "pmgpu_system_set_step",
     "pmgpu_force_full_add", "pmgpu_force_simplefull_switched_add", "pmgpu_force_scpism_add",
     "pmgpu_force_born_add", "pmgpu_debug_set_column_capacity", "pmgpu_run_discard",
+    "pmgpu_graph_replays",
 ]
 PHASES = ["list", "pairs", "pme", "correction", "bonded", "gb", "simplefull", "integrate"]
 
@@ -156,6 +157,7 @@ def load() -> C.CDLL:
     lib.pmgpu_profile_enable.argtypes = [vp, i32]
     lib.pmgpu_profile_read.argtypes = [vp, vp, vp, i32]
     lib.pmgpu_kernel_count.argtypes = [vp, C.POINTER(C.c_longlong)]
+    lib.pmgpu_graph_replays.argtypes = [vp, C.POINTER(C.c_longlong)]
     lib.pmgpu_run_async.argtypes = [vp, C.POINTER(Integrator), C.c_long]
     lib.pmgpu_run_query.argtypes = [vp, C.POINTER(i32)]
     lib.pmgpu_run_wait.argtypes = [vp]

@@ -1417,6 +1417,39 @@ int pmgpu_force_set_enabled(pmgpu_system *h, int id, int enabled) {
   return PMGPU_OK;
 }
 
+// Ends the capture of a graph (r: what enqueueing it returned) and makes it
+// executable.  When that fails *exec is null and the system's work stays
+// eager from then on; the reason is kept for pmgpu_last_error and, with
+// PMGPU_DEBUG set, printed.
+static void graph_finish(System *s, int r, const char *what, cudaGraphExec_t *exec) {
+  cudaGraph_t graph = nullptr;
+  const cudaError_t ec = cudaStreamEndCapture(s->stream, &graph);
+  cudaError_t ei = cudaSuccess;
+  *exec = nullptr;
+  if (r == PMGPU_OK && ec == cudaSuccess && graph)
+    ei = cudaGraphInstantiate(exec, graph, cudaGraphInstantiateFlagUseNodePriority);
+  if (r != PMGPU_OK || ec != cudaSuccess || !graph || ei != cudaSuccess) {
+    if (std::getenv("PMGPU_DEBUG"))
+      std::fprintf(stderr, "pmgpu: %s graph not used (%s; end capture: %s; instantiate: %s)\n",
+                   what, r != PMGPU_OK ? g_last_error.c_str() : "capture ok",
+                   cudaGetErrorString(ec), cudaGetErrorString(ei));
+    cudaGetLastError();
+    *exec = nullptr;
+    s->graphs_disabled = 1;
+  }
+  if (graph) cudaGraphDestroy(graph);
+}
+static bool graph_begin(System *s, const char *what) {
+  const cudaError_t e = cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal);
+  if (e == cudaSuccess) return true;
+  if (std::getenv("PMGPU_DEBUG"))
+    std::fprintf(stderr, "pmgpu: %s graph not used (begin capture: %s)\n", what,
+                 cudaGetErrorString(e));
+  cudaGetLastError();
+  s->graphs_disabled = 1;
+  return false;
+}
+
 // One evaluation's work on the system's stream: the staged positions to the
 // device (with_pos), clear, evaluate, accumulators and status to the host,
 // the forces to the staging buffer (with_forces).
@@ -1468,31 +1501,19 @@ static int eval_run(System *s, int only, int mode, int with_pos, int with_forces
     g->version = s->graph_version;
     g->uses = 0;
   }
-  if (g && !g->exec && g->uses++ >= kEvalEager) {
+  if (g && !g->exec && g->uses++ >= kEvalEager && graph_begin(s, "evaluation")) {
     const long long k0 = s->kernels;
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-      const int r = eval_enqueue(s, only, mode, with_pos, with_forces);
-      const cudaError_t ec = cudaStreamEndCapture(s->stream, &graph);
-      if (r != PMGPU_OK || ec != cudaSuccess || !graph ||
-          cudaGraphInstantiate(&g->exec, graph, cudaGraphInstantiateFlagUseNodePriority) !=
-              cudaSuccess)
-        g->exec = nullptr;
-      if (graph) cudaGraphDestroy(graph);
-      g->kernels = s->kernels - k0;
-      s->kernels = k0;
-      g->forms.clear();
-      for (auto &nl : s->lists) g->forms.push_back(nl.last_form);
-      // nothing has run yet: the lists are as they were
-      for (size_t k = 0; k < s->lists.size(); k++) s->lists[k].built = (key >> (40 + k)) & 1;
-    }
-    if (!g->exec) {
-      cudaGetLastError();
-      s->graphs_disabled = 1;
-    }
+    graph_finish(s, eval_enqueue(s, only, mode, with_pos, with_forces), "evaluation", &g->exec);
+    g->kernels = s->kernels - k0;
+    s->kernels = k0;
+    g->forms.clear();
+    for (auto &nl : s->lists) g->forms.push_back(nl.last_form);
+    // nothing has run yet: the lists are as they were
+    for (size_t k = 0; k < s->lists.size(); k++) s->lists[k].built = (key >> (40 + k)) & 1;
   }
   if (g && g->exec) {
     PM_CUDA(cudaGraphLaunch(g->exec, s->stream));
+    s->replays++;
     s->kernels += g->kernels;
     // the host state eval_enqueue leaves
     for (auto &f : s->forces)
@@ -1625,40 +1646,18 @@ static int run_graph(System *s, const pmgpu_integrator *it, int part, int *used)
     if (in_use[k] && !s->lists[k].built) return PMGPU_OK;
   if (!sg.exec && part >= RUN_FIRST && sg.uses++ < kEvalEager) return PMGPU_OK;
   if (!sg.exec) {
-    long long k0 = s->kernels;
-    cudaGraph_t graph = nullptr;
-    if (cudaStreamBeginCapture(s->stream, cudaStreamCaptureModeThreadLocal) != cudaSuccess) {
-      cudaGetLastError();
-      s->graphs_disabled = 1;
-      return PMGPU_OK;
-    }
-    const int r = run_part(s, it, part);
-    cudaError_t ec = cudaStreamEndCapture(s->stream, &graph);
-    const long long per_launch = s->kernels - k0;
+    if (!graph_begin(s, "step")) return PMGPU_OK;
+    const long long k0 = s->kernels;
+    graph_finish(s, run_part(s, it, part), "step", &sg.exec);
+    sg.kernels = s->kernels - k0;
     s->kernels = k0;
-    cudaError_t ei = cudaSuccess;
-    if (r == PMGPU_OK && ec == cudaSuccess && graph)
-      ei = cudaGraphInstantiate(&sg.exec, graph, cudaGraphInstantiateFlagUseNodePriority);
-    if (r != PMGPU_OK || ec != cudaSuccess || !graph || ei != cudaSuccess) {
-      // the reason is kept for pmgpu_last_error and, with PMGPU_DEBUG set,
-      // printed; the run continues with eager launches
-      if (std::getenv("PMGPU_DEBUG"))
-        std::fprintf(stderr, "pmgpu: step graph not used (%s; end capture: %s; instantiate: %s)\n",
-                     r != PMGPU_OK ? g_last_error.c_str() : "capture ok",
-                     cudaGetErrorString(ec), cudaGetErrorString(ei));
-      if (graph) cudaGraphDestroy(graph);
-      cudaGetLastError();
-      sg.exec = nullptr;
-      s->graphs_disabled = 1;  // fall back to eager launches from now on
-      return PMGPU_OK;
-    }
-    cudaGraphDestroy(graph);
-    sg.kernels = per_launch;
+    if (!sg.exec) return PMGPU_OK;
     sg.lists.clear();
     for (auto &nl : s->lists) sg.lists.push_back({nl.slot_pending, nl.last_form});
     sg.rec_fresh = s->rec_fresh;
   }
   PM_CUDA(cudaGraphLaunch(sg.exec, s->stream));
+  s->replays++;
   s->kernels += sg.kernels;
   // the host state the part leaves
   for (size_t k = 0; k < s->lists.size(); k++) {
@@ -1916,6 +1915,12 @@ int pmgpu_profile_read(pmgpu_system *h, double *ms, long long *launches, int res
 int pmgpu_kernel_count(pmgpu_system *h, long long *count) {
   if (!h || !count) return fail(PMGPU_ERR_ARG, "null argument");
   *count = sysp(h)->kernels;
+  return PMGPU_OK;
+}
+
+int pmgpu_graph_replays(pmgpu_system *h, long long *count) {
+  if (!h || !count) return fail(PMGPU_ERR_ARG, "null argument");
+  *count = sysp(h)->replays;
   return PMGPU_OK;
 }
 

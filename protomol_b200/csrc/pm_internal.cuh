@@ -364,6 +364,7 @@ struct System {
   // graph_version): several inner steps, one, a run's first and its last
   int graph_version = 0;
   int graphs_disabled = 0;
+  long long replays = 0;  // graph launches (see pmgpu_graph_replays)
   struct StepGraph {
     int version = -1;
     int count_pairs = 0;

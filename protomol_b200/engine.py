@@ -257,6 +257,13 @@ class GpuSystem:
         L.check(self.lib.pmgpu_kernel_count(self.h, C.byref(c)))
         return int(c.value)
 
+    def graph_replays(self) -> int:
+        """CUDA graph launches of this system so far (0 while its work is
+        eager: profiling, or a capture that failed)."""
+        c = C.c_longlong()
+        L.check(self.lib.pmgpu_graph_replays(self.h, C.byref(c)))
+        return int(c.value)
+
     def set_list_capacity(self, tiles_per_row: int) -> None:
         """Fix the pair lists' capacity (testing the growth path)."""
         L.check(self.lib.pmgpu_debug_set_list_capacity(self.h, int(tiles_per_row)))
