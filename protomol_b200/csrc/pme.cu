@@ -934,14 +934,17 @@ int pme_batch_build(PmeBatch *b, System *const *m, int n, Force *const *fs) {
   b->sizes = (int)seen.size();
   for (auto &bk : b->buckets) {
     const int B = (int)bk.members.size();
-    const size_t G = (size_t)bk.K[0] * bk.K[1] * bk.K[2];
+    // slices of an even number of floats: a member's own plan transforms its
+    // slice too, and cuFFT refuses a real grid that is not 8-byte aligned
+    const size_t G = ((size_t)bk.K[0] * bk.K[1] * bk.K[2] + 1) / 2 * 2;
     const size_t Gc = (size_t)bk.K[0] * bk.K[1] * (bk.K[2] / 2 + 1);
     PM_CUDA(cudaMalloc(&bk.grid, sizeof(float) * G * B));
     PM_CUDA(cudaMalloc(&bk.cgrid, sizeof(float2) * Gc * B));
-    int dims[3] = {bk.K[0], bk.K[1], bk.K[2]};
-    if (cufftPlanMany(&bk.r2c, 3, dims, nullptr, 1, (int)G, nullptr, 1, (int)Gc, CUFFT_R2C, B) !=
+    // (without the embedding arrays cuFFT takes the slices as packed)
+    int dims[3] = {bk.K[0], bk.K[1], bk.K[2]}, half[3] = {bk.K[0], bk.K[1], bk.K[2] / 2 + 1};
+    if (cufftPlanMany(&bk.r2c, 3, dims, dims, 1, (int)G, half, 1, (int)Gc, CUFFT_R2C, B) !=
             CUFFT_SUCCESS ||
-        cufftPlanMany(&bk.c2r, 3, dims, nullptr, 1, (int)Gc, nullptr, 1, (int)G, CUFFT_C2R, B) !=
+        cufftPlanMany(&bk.c2r, 3, dims, half, 1, (int)Gc, dims, 1, (int)G, CUFFT_C2R, B) !=
             CUFFT_SUCCESS)
       return fail(PMGPU_ERR_CUDA, "batched cuFFT plan creation failed");
     for (int q = 0; q < B; q++) {
