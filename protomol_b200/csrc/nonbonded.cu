@@ -1222,11 +1222,9 @@ static void fill_pair_args(PairArgs<Real> &a, System *s, NeighborList *nl,
 }
 
 // Compile-time switch kind of a term for the specialised force-only
-// kernel: -2 when the configuration has no specialisation.
+// kernel: -1 when the configuration has no specialisation.
 static int spec_kind(const SwitchParams &sw) {
-  if (!sw.modify) return kSwNone;
-  if (sw.kind == PMGPU_SW_C2 || sw.kind == PMGPU_SW_C1) return sw.kind;
-  return -2;
+  return sw.modify && (sw.kind == PMGPU_SW_C2 || sw.kind == PMGPU_SW_C1) ? sw.kind : -1;
 }
 
 static int sm_count() {
@@ -1241,32 +1239,34 @@ static int sm_count() {
   return sms;
 }
 
-// Warps per i cluster of the tile kernel: about four waves of the
-// force-only kernel's resident warps (40 per SM), at most kPairMaxSplits per
-// cluster, so blocks that finish early are refilled and the tail stays
-// short.  A small box has few clusters and each warp's tiles are one serial
-// chain (FP64 or run-time switches), so it takes many: with 8 at most, 648
-// atoms in FP64 left five warps an SM (38 us a launch; 12.8 us with 32), and
-// the generic members of a 24-box ensemble took 46 instead of 34 us.  The split depends only on the
-// system, so every launch of a system sums its forces in the same order.
+// Warps per i cluster of the tile kernel: about 160 warps an SM (five waves
+// of the 32 FP32 ones that are resident, ten of the 16 FP64 ones), at most
+// kPairMaxSplits per cluster, so blocks that finish early are refilled and
+// the tail stays short.  A small box has few clusters and each warp's tiles
+// are one serial chain (FP64 or run-time switches), so it takes many: with 8
+// at most, 648 atoms in FP64 left five warps an SM (38 us a launch; 13 us
+// with 32), and the generic members of a 24-box ensemble took 46 instead of
+// 34 us.  The split depends only on the system, so every launch of a system
+// sums its forces in the same order.
 constexpr int kPairMaxSplits = 32;
 static int pair_splits(int nclusters) {
-  const long long want = 4LL * sm_count() * 40;
-  return (int)std::max(1LL, std::min((long long)kPairMaxSplits, (want + nclusters / 2) / std::max(1, nclusters)));
+  const long long want = 160LL * sm_count();
+  return (int)std::max(1LL, std::min((long long)kPairMaxSplits,
+                                     (want + nclusters / 2) / std::max(1, nclusters)));
 }
 
-template <typename Real, int TERMS, typename SPEC>
-static void launch_pairs_spec(PairArgs<Real> &a, cudaStream_t st, int mode) {
+template <typename Real, int TERMS>
+static void launch_tiles(const PairArgs<Real> &a, cudaStream_t st, int mode) {
   const int T = kPairWarps * 32;
   const int nb = (int)(((long long)a.nclusters * a.splits + kPairWarps - 1) / kPairWarps);
   if (nb == 0) return;
   if (mode == PAIR_FORCE) {
-    k_pairs<Real, TERMS, PAIR_FORCE, SPEC><<<nb, T, 0, st>>>(a);
+    k_pairs<Real, TERMS, PAIR_FORCE><<<nb, T, 0, st>>>(a);
   } else if (mode == PAIR_RECORD) {
-    k_pairs<Real, TERMS, PAIR_RECORD, SPEC><<<nb, T, 0, st>>>(a);
+    k_pairs<Real, TERMS, PAIR_RECORD><<<nb, T, 0, st>>>(a);
   } else if constexpr (sizeof(Real) == 8) {  // mixed precision: launch_e64
-    if (mode == PAIR_ENERGY) k_pairs<Real, TERMS, PAIR_ENERGY, SPEC><<<nb, T, 0, st>>>(a);
-    else k_pairs<Real, TERMS, PAIR_VIRIAL, SPEC><<<nb, T, 0, st>>>(a);
+    if (mode == PAIR_ENERGY) k_pairs<Real, TERMS, PAIR_ENERGY><<<nb, T, 0, st>>>(a);
+    else k_pairs<Real, TERMS, PAIR_VIRIAL><<<nb, T, 0, st>>>(a);
   }
 }
 
@@ -1326,22 +1326,18 @@ static void launch_jl(const PairArgs<float> &a, int nb, cudaStream_t st) {
 // The specialised force-only FP32 kernels: j atoms on the lanes
 // (k_pairs_jl), a cluster's LJ parameters in shared memory when the types
 // are few.
-template <typename Real, int TERMS, typename SPEC>
-static void launch_force_spec(PairArgs<Real> &a, cudaStream_t st) {
-  if constexpr (sizeof(Real) == 4) {
-    a.splits = jl_splits(a.nclusters);
-    const long long items = (long long)a.nclusters * a.splits;
-    const int nb = (int)((items + kJlWarps - 1) / kJlWarps);
-    if (nb == 0) return;
-    // the Ewald force table for the LJ + Ewald real form when the list has one
-    constexpr bool kTab = TERMS == (TERM_LJ | TERM_EWALD) && SPEC::exact == 0;
-    const bool tab = kTab && a.ewtab != nullptr;
-    if (tab && a.ntypes <= kJlMaxTypes) launch_jl<TERMS, SPEC, kTab, kTab>(a, nb, st);
-    else if (tab) launch_jl<TERMS, SPEC, false, kTab>(a, nb, st);
-    else launch_jl<TERMS, SPEC, false, false>(a, nb, st);
-  } else {
-    launch_pairs_spec<Real, TERMS, SPEC>(a, st, PAIR_FORCE);
-  }
+template <int TERMS, typename SPEC>
+static void launch_force_spec(PairArgs<float> a, cudaStream_t st) {
+  a.splits = jl_splits(a.nclusters);
+  const long long items = (long long)a.nclusters * a.splits;
+  const int nb = (int)((items + kJlWarps - 1) / kJlWarps);
+  if (nb == 0) return;
+  // the Ewald force table for the LJ + Ewald real form when the list has one
+  constexpr bool kTab = TERMS == (TERM_LJ | TERM_EWALD) && SPEC::exact == 0;
+  const bool tab = kTab && a.ewtab != nullptr;
+  if (tab && a.ntypes <= kJlMaxTypes) launch_jl<TERMS, SPEC, kTab, kTab>(a, nb, st);
+  else if (tab) launch_jl<TERMS, SPEC, false, kTab>(a, nb, st);
+  else launch_jl<TERMS, SPEC, false, false>(a, nb, st);
 }
 
 // The specialised force-only form of a launch's terms (every term with one
@@ -1420,22 +1416,20 @@ static int launch_pairs_t(PairArgs<Real> &a, cudaStream_t st, int mode, const Pa
       PairArgs<Real> fa = a;
       if (mode != PAIR_FORCE) fa.count_pairs = 0;  // the energy pass counts
       if (form == PMGPU_PAIRK_LJC2_EWALD)
-        launch_force_spec<Real, TERM_LJ | TERM_EWALD, PairSpec<PMGPU_SW_C2, -1, 0>>(fa, st);
+        launch_force_spec<TERM_LJ | TERM_EWALD, PairSpec<PMGPU_SW_C2, -1, 0>>(fa, st);
       else if (form == PMGPU_PAIRK_LJC2_COULC2)
-        launch_force_spec<Real, TERM_LJ | TERM_COUL, PairSpec<PMGPU_SW_C2, PMGPU_SW_C2, -1>>(fa,
-                                                                                          st);
+        launch_force_spec<TERM_LJ | TERM_COUL, PairSpec<PMGPU_SW_C2, PMGPU_SW_C2, -1>>(fa, st);
       else if (form == PMGPU_PAIRK_LJC2_COULC1)
-        launch_force_spec<Real, TERM_LJ | TERM_COUL, PairSpec<PMGPU_SW_C2, PMGPU_SW_C1, -1>>(fa,
-                                                                                          st);
+        launch_force_spec<TERM_LJ | TERM_COUL, PairSpec<PMGPU_SW_C2, PMGPU_SW_C1, -1>>(fa, st);
       else
-        launch_pairs_spec<Real, TERMS, GenericSpec>(fa, st, PAIR_FORCE);
+        launch_tiles<Real, TERMS>(fa, st, PAIR_FORCE);
       // (a failed launch is found by the caller's cudaGetLastError)
       if (mode == PAIR_ENERGY) (void)launch_e64<false>(a, form, st);
       if (mode == PAIR_VIRIAL) (void)launch_e64<true>(a, form, st);
       return form;
     }
   }
-  launch_pairs_spec<Real, TERMS, GenericSpec>(a, st, mode);
+  launch_tiles<Real, TERMS>(a, st, mode);
   return PMGPU_PAIRK_GENERIC;
 }
 
@@ -1616,7 +1610,7 @@ int nb_batch_list(NbBatch *b, cudaStream_t st, long long *launched) {
 template <int TERMS>
 static int launch_generic_batch(BatchTable<PairArgs<float>> &t, cudaStream_t st) {
   if (!t.members() || !t.total()) return 0;
-  k_pairs_batch<float, TERMS, PAIR_FORCE, GenericSpec>
+  k_pairs_batch<float, TERMS, PAIR_FORCE>
       <<<t.total(), kPairWarps * 32, 0, st>>>(t.d, t.d_first, t.members());
   return 1;
 }

@@ -125,43 +125,14 @@ __device__ __forceinline__ void apply_switch(const SwitchDev<Real> &sw,
   en = en * sv;
 }
 
-// Compile-time description of a pair-kernel instantiation's switching
-// functions and erfc variant; -1 means "read from the arguments at run
-// time".  The force-only FP32 kernel of the common configurations is
-// specialised so that the per-pair arithmetic carries no run-time dispatch.
-constexpr int kSwNone = 9;  // switch not applied (Universal, Cutoff: MODIFY = 0)
+// Compile-time description of a j-lane force-only kernel's switching
+// functions and erfc variant (-1: the term has no switch), so that the
+// per-pair arithmetic of the common configurations carries no run-time
+// dispatch.
 template <int LJK, int CK, int EXACT>
 struct PairSpec {
   static constexpr int lj = LJK, coul = CK, exact = EXACT;
 };
-using GenericSpec = PairSpec<-1, -1, -1>;
-
-template <typename Real, int KIND>
-__device__ __forceinline__ void switch_k(const SwitchDev<Real> &sw, const SwitchDev<double> &sw64,
-                                         int modify, Real r2, Real &ff, Real &en, Real &sv,
-                                         Real &sd, int known) {
-  if (KIND < 0) {
-    if (modify) apply_switch<Real>(sw, sw64, r2, ff, en, sv, sd, known);
-  } else if (KIND == PMGPU_SW_C2) {
-    // C2SwitchingFunction::operator() (switch/C2SwitchingFunction.h:42-52)
-    if (r2 > sw.cutoff2) {
-      ff = Real(0);
-      en = Real(0);
-    } else if (r2 >= sw.switchon2) {
-      Real c2 = sw.cutoff2 - r2;
-      Real c4 = c2 * (sw.s2 + Real(2) * r2);
-      Real val = sw.s1 * (c2 * c4);
-      Real der = sw.s3 * (c2 * c2 - c4);
-      ff = ff * val - en * der;
-      en = en * val;
-    }
-  } else if (KIND == PMGPU_SW_C1) {
-    Real val, der;
-    switch_eval<Real>(sw, r2, val, der);
-    ff = ff * val - en * der;
-    en = en * val;
-  }
-}
 
 // Per-pair flags of an accepted pair: which terms are inside their cutoff,
 // and whether the pair is a modified (scaled 1-4) one.
@@ -170,7 +141,7 @@ constexpr int kQLJ = 1, kQCoul = 2, kQEwald = 4, kQModified = 8;
 // Pair force, energies of one accepted pair (the terms' arithmetic of
 // OneAtomPairTwo::doOneAtomPair, force/OneAtomPairTwo.h:55-100).
 // Returns f with F_i -= d * f.
-template <typename Real, int TERMS, typename SPEC>
+template <typename Real, int TERMS>
 __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *ljrow, Real r2,
                                            Real qq, int tj, int flags, Real &en_lj,
                                            Real &en_c) {
@@ -196,7 +167,7 @@ __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *
     Real r12A = A * r6 * r6;
     Real en = r12A - r6B;
     Real ff = (Real(12) * r12A - Real(6) * r6B) * rinv2;
-    switch_k<Real, SPEC::lj>(a.lj_sw, a.lj_sw64, a.lj_modify, r2, ff, en, sv, sd, 0);
+    if (a.lj_modify) apply_switch<Real>(a.lj_sw, a.lj_sw64, r2, ff, en, sv, sd, 0);
     known = a.same_sw;
     en_lj += en;
     f += ff;
@@ -206,7 +177,7 @@ __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *
     // CoulombForce::operator() (force/CoulombForce.h:29-40)
     Real en = qq * rinv;
     Real ff = en * rinv2;
-    switch_k<Real, SPEC::coul>(a.coul_sw, a.coul_sw64, a.coul_modify, r2, ff, en, sv, sd, known);
+    if (a.coul_modify) apply_switch<Real>(a.coul_sw, a.coul_sw64, r2, ff, en, sv, sd, known);
     en_c += en;
     f += ff;
   }
@@ -216,7 +187,7 @@ __device__ __forceinline__ Real pair_force(const PairArgs<Real> &a, const Real *
     Real ar = a.alpha * r;
     Real ee = qq * fast_exp(-ar * ar);
     Real en;
-    if (SPEC::exact == 0 || (SPEC::exact < 0 && !a.exact_erf))
+    if (!a.exact_erf)
       en = poly5_fast<Real>(ar) * ee * rinv;  // A&S erfc (MathUtilities.cpp:39-49)
     else
       en = qq * erfc(ar) * rinv;  // USE_EWALD_EXACT_ERF: C library erfc
@@ -292,19 +263,19 @@ __device__ __forceinline__ Real pair_force_p(const PairArgs<Real> &a, const P4 &
 // square root, exponential or erfc per pair.  r2 must lie in the table's
 // range [2^kEwTabLoExp, 2^(kEwTabLoExp + kEwTabOctaves)); others read the
 // nearest end interval (the callers keep them out of the accepted pairs).
-template <typename SPEC, bool MOD>
+template <typename SPEC>
 __device__ __forceinline__ float pair_force_tab(const PairArgs<float> &a, const float4 &p,
                                                 float r2, float qq, bool modified,
                                                 const float4 *s_ew) {
   const float rinv2 = __fdividef(1.f, r2);
-  const float A = MOD && modified ? p.z : p.x;
-  const float B = MOD && modified ? p.w : p.y;
+  const float A = modified ? p.z : p.x;
+  const float B = modified ? p.w : p.y;
   const float r6 = rinv2 * rinv2 * rinv2;
   const float r6B = B * r6;
   const float r12A = A * r6 * r6;
   float ff = (12.f * r12A - 6.f * r6B) * rinv2;
   switch_fast<float, SPEC::lj>(a.lj_sw, r2, 0.f, ff, r12A - r6B);
-  if (MOD) qq = modified ? qq * a.csf : qq;
+  qq = modified ? qq * a.csf : qq;
   const unsigned bits = __float_as_uint(r2);
   const int idx = min(max((int)(bits >> (23 - kEwTabSubBits)) - (int)kEwTabBase, 0), kEwTabN - 1);
   const float t =
@@ -313,25 +284,11 @@ __device__ __forceinline__ float pair_force_tab(const PairArgs<float> &a, const 
   return fmaf(qq, fmaf(t, fmaf(t, fmaf(t, c.w, c.z), c.y), c.x), ff);
 }
 
-template <typename Real, int TERMS, typename SPEC, bool MOD>
-__device__ __forceinline__ Real pair_force_fast(const PairArgs<Real> &a, const Real *ljrow,
-                                                Real r2, Real qq, int tj, bool modified) {
-  if (sizeof(Real) == 4) {
-    const float4 p = __ldg(reinterpret_cast<const float4 *>(ljrow) + tj);
-    return pair_force_p<Real, TERMS, SPEC, MOD>(a, p, r2, qq, modified);
-  }
-  const double4 p = reinterpret_cast<const double4 *>(ljrow)[tj];
-  return pair_force_p<Real, TERMS, SPEC, MOD>(a, p, r2, qq, modified);
-}
-
-// Registers: the specialised force-only FP32 kernels (the inner MD steps)
-// are held to 48 so five blocks fit per SM, the generic force-only FP32
-// kernel to 64; energy/virial/record and FP64 variants get more.
-template <typename Real, int MODE, typename SPEC>
+// Registers: the force-only FP32 kernels are held to 64 so four blocks fit
+// per SM; the record and FP64 variants get more.
+template <typename Real, int MODE>
 struct PairOccupancy {
-  static constexpr bool fast = MODE == PAIR_FORCE && sizeof(Real) == 4 && SPEC::lj >= 0 &&
-                               SPEC::exact >= 0;
-  static constexpr int warps = fast ? 40 : ((MODE == PAIR_FORCE && sizeof(Real) == 4) ? 32 : 16);
+  static constexpr int warps = MODE == PAIR_FORCE && sizeof(Real) == 4 ? 32 : 16;
   static constexpr int blocks = warps / kPairWarps;
 };
 
@@ -399,23 +356,17 @@ __device__ __forceinline__ void block_energies(long long *acc, const double (&v)
 // Pairs are accepted by the cutoff tests of the reference (with the exact
 // FP64 re-test near a cutoff); the tile mask carries the list's exclusion
 // and modified (scaled 1-4) status.
-template <typename Real, int TERMS, int MODE, typename SPEC>
+template <typename Real, int TERMS, int MODE>
 __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   constexpr bool MIXED = sizeof(Real) == 4;
   // (in mixed precision energies come from k_pairs_e64)
   constexpr bool ENERGY = !MIXED && (MODE == PAIR_ENERGY || MODE == PAIR_VIRIAL);
   constexpr bool VIRIAL = !MIXED && MODE == PAIR_VIRIAL;
   constexpr bool RECORD = MODE == PAIR_RECORD;
-  // force-only kernels of a specialised configuration (launched only when
-  // every term shares one cutoff and the box holds twice the cutoff): every
-  // accepted pair takes every term, evaluated without branches
-  constexpr bool FAST = MIXED && MODE == PAIR_FORCE && SPEC::lj >= 0 && SPEC::exact >= 0;
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int il = lane & 7, jl = lane >> 3;
-  const unsigned lanebit = 1u << lane;        // this lane's bit of a tile mask
-  const unsigned jbyte = 0xFFu << (8 * jl);   // the 8 lanes of this lane's j atom
-  const bool jcomp = il < 3;                  // lane adds j's force component il
+  const unsigned lanebit = 1u << lane;  // this lane's bit of a tile mask
   double Elj = 0, Ec = 0;
   Real vxx = 0, vxy = 0, vxz = 0, vyy = 0, vyz = 0, vzz = 0;
   int npairs = 0;
@@ -509,39 +460,6 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
       qj = wj.w;
     }
     const Real r2 = dx * dx + dy * dy + dz * dz;
-    if constexpr (FAST) {
-      bool act = live && r2 <= a.max_lo;
-      const bool band = live && !act && r2 <= a.max_hi;
-      if (__any_sync(kAll, band)) {
-        if (band)
-          act = exact_r2(a, oi, a.sorted[jslot], (double)dx, (double)dy, (double)dz) <=
-                a.max_cut2;
-      }
-      const unsigned actm = __ballot_sync(kAll, act);
-      if (a.count_pairs) npairs += act;
-      if (!actm) continue;
-      const Real rr = act ? r2 : Real(1);
-      Real f;
-      // modified (scaled 1-4) pairs are rare: tiles without any take the
-      // path without their selects (the mask is the tile's, so the branch
-      // is uniform)
-      if (__any_sync(kAll, tile.z != 0u))
-        f = pair_force_fast<Real, TERMS, SPEC, true>(a, ljrow, rr, qi * qj, tj,
-                                                     (tile.z & lanebit) != 0u);
-      else
-        f = pair_force_fast<Real, TERMS, SPEC, false>(a, ljrow, rr, qi * qj, tj, false);
-      f = act ? f : Real(0);
-      const Real jx = dx * f, jy = dy * f, jz = dz * f;
-      fx -= jx;
-      fy -= jy;
-      fz -= jz;
-      const Real js = group8_sum3<Real>(jx, jy, jz, lane);
-      // address and value formed by every lane, one predicated atomic
-      long long *dst = a.fslot + il * a.ns + jslot;
-      const long long v = fixed_force(js);
-      if (jcomp && (actm & jbyte)) red_add(dst, v);
-      continue;
-    }
     int flags = 0;
     bool band = false;
     if (live && a.same_cut) {  // every term shares one cutoff
@@ -582,7 +500,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
       if ((tile.z >> lane) & 1u) flags |= kQModified;
       if (!MIXED) tj = a.type[a.sorted[jslot]];
       Real en_lj = 0, en_c = 0;
-      const Real f = pair_force<Real, TERMS, SPEC>(a, ljrow, r2, qi * qj, tj, flags, en_lj, en_c);
+      const Real f = pair_force<Real, TERMS>(a, ljrow, r2, qi * qj, tj, flags, en_lj, en_c);
       jx = dx * f;
       jy = dy * f;
       jz = dz * f;
@@ -677,18 +595,18 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   }
 }
 
-template <typename Real, int TERMS, int MODE, typename SPEC>
-__global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE, SPEC>::blocks)
+template <typename Real, int TERMS, int MODE>
+__global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE>::blocks)
     k_pairs(PairArgs<Real> a) {
-  pairs_body<Real, TERMS, MODE, SPEC>(a, own_blk());
+  pairs_body<Real, TERMS, MODE>(a, own_blk());
 }
 
-template <typename Real, int TERMS, int MODE, typename SPEC>
-__global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE, SPEC>::blocks)
+template <typename Real, int TERMS, int MODE>
+__global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE>::blocks)
     k_pairs_batch(const PairArgs<Real> *__restrict__ tab, const int *__restrict__ first, int nm) {
   __shared__ __align__(16) unsigned char raw[sizeof(PairArgs<Real>)];
   const int m = batch_member(first, nm, blockIdx.x);
-  pairs_body<Real, TERMS, MODE, SPEC>(batch_args_shared(tab, m, raw), batch_blk(first, m));
+  pairs_body<Real, TERMS, MODE>(batch_args_shared(tab, m, raw), batch_blk(first, m));
 }
 
 // ---------------------------------------------------------------------------
@@ -718,7 +636,8 @@ constexpr int kJlMaxSplits = 16;  // warps one i cluster's tiles may be divided 
 constexpr float kEwTabMin = 1.0f / (1 << -kEwTabLoExp);  // the table's lowest r^2
 
 // The eight pairs of one lane's j atom with the cluster's i atoms (mi: the
-// pairs of the list's interaction mask).
+// pairs of the list's interaction mask); unmodified pairs of the table form
+// take jl_pairs8_x2.
 template <int TERMS, typename SPEC, bool MOD, bool TAB>
 __device__ __forceinline__ void jl_pairs8(const PairArgs<float> &a, const float4 *s_ew,
                                           const float4 *xi, const int *ti, float rjx, float rjy,
@@ -739,7 +658,7 @@ __device__ __forceinline__ void jl_pairs8(const PairArgs<float> &a, const float4
     const float4 p = __ldg(a.lj32 + ti[il] + tj);
     float f;
     if constexpr (TAB)
-      f = pair_force_tab<SPEC, MOD>(a, p, rr, x.w * qj, MOD && ((mm >> il) & 1u), s_ew);
+      f = pair_force_tab<SPEC>(a, p, rr, x.w * qj, (mm >> il) & 1u, s_ew);
     else
       f = pair_force_p<float, TERMS, SPEC, MOD>(a, p, rr, x.w * qj, MOD && ((mm >> il) & 1u));
     f = act ? f : 0.f;
@@ -1198,7 +1117,7 @@ __device__ __forceinline__ void pairs_e64_body(const PairArgs<float> &a, Blk blk
       const double2 p = __ldg(tab + (modified ? 1 : 0));  // A, B or A14, B14
       const double r6 = rr2 * rr2 * rr2, r6B = p.y * r6, r12A = p.x * r6 * r6;
       double en = r12A - r6B, ff = VIRIAL ? (12.0 * r12A - 6.0 * r6B) * rr2 : 0.0;
-      if (LJK != kSwNone && (LJK >= 0 || a.lj_modify)) {
+      if (LJK >= 0 || a.lj_modify) {
         double sv, sd;
         switch64<LJK, VIRIAL>(a.lj_sw64, r2, rinv, sv, sd);
         if (VIRIAL) ff = ff * sv - en * sd;
@@ -1210,7 +1129,7 @@ __device__ __forceinline__ void pairs_e64_body(const PairArgs<float> &a, Blk blk
     if (modified) qq *= a.csf64;
     if ((TERMS & TERM_COUL) && (code.y & kQCoul)) {
       double en = qq * rinv, ff = VIRIAL ? en * rr2 : 0.0;
-      if (CK != kSwNone && (CK >= 0 || a.coul_modify)) {
+      if (CK >= 0 || a.coul_modify) {
         double sv, sd;
         switch64<CK, VIRIAL>(a.coul_sw64, r2, rinv, sv, sd);
         if (VIRIAL) ff = ff * sv - en * sd;
