@@ -1355,29 +1355,25 @@ static int special_form(const PairArgs<Real> &a, const PairTerms &t) {
   return PMGPU_PAIRK_GENERIC;
 }
 
-// The instantiation of the FP64 energy kernel for a launch's terms, given
-// to go: compiled switch kinds for the specialised forms, run-time switches
-// for the others.
-template <bool VIRIAL, typename F>
+// The FP64 energy kernel for a launch's terms, given to go: compiled switch
+// kinds for the specialised forms, run-time switches for the others.
+template <bool VIRIAL, bool BATCH, int TERMS, int LJK = -1, int CK = -1>
+static auto e64_instance() {
+  if constexpr (BATCH) return k_pairs_e64_batch<TERMS, VIRIAL, LJK, CK>;
+  else return k_pairs_e64<TERMS, VIRIAL, LJK, CK>;
+}
+template <bool VIRIAL, bool BATCH, typename F>
 static void e64_kernel(int mask, int form, F go) {
   constexpr int LC = TERM_LJ | TERM_COUL, LE = TERM_LJ | TERM_EWALD;
   constexpr int C2 = PMGPU_SW_C2, C1 = PMGPU_SW_C1;
-  if (form == PMGPU_PAIRK_LJC2_EWALD)
-    go(k_pairs_e64<LE, VIRIAL, C2, -1>, k_pairs_e64_batch<LE, VIRIAL, C2, -1>);
-  else if (form == PMGPU_PAIRK_LJC2_COULC2)
-    go(k_pairs_e64<LC, VIRIAL, C2, C2>, k_pairs_e64_batch<LC, VIRIAL, C2, C2>);
-  else if (form == PMGPU_PAIRK_LJC2_COULC1)
-    go(k_pairs_e64<LC, VIRIAL, C2, C1>, k_pairs_e64_batch<LC, VIRIAL, C2, C1>);
-  else if (mask == TERM_LJ)
-    go(k_pairs_e64<TERM_LJ, VIRIAL, -1, -1>, k_pairs_e64_batch<TERM_LJ, VIRIAL, -1, -1>);
-  else if (mask == TERM_COUL)
-    go(k_pairs_e64<TERM_COUL, VIRIAL, -1, -1>, k_pairs_e64_batch<TERM_COUL, VIRIAL, -1, -1>);
-  else if (mask == LC)
-    go(k_pairs_e64<LC, VIRIAL, -1, -1>, k_pairs_e64_batch<LC, VIRIAL, -1, -1>);
-  else if (mask == TERM_EWALD)
-    go(k_pairs_e64<TERM_EWALD, VIRIAL, -1, -1>, k_pairs_e64_batch<TERM_EWALD, VIRIAL, -1, -1>);
-  else
-    go(k_pairs_e64<LE, VIRIAL, -1, -1>, k_pairs_e64_batch<LE, VIRIAL, -1, -1>);
+  if (form == PMGPU_PAIRK_LJC2_EWALD) go(e64_instance<VIRIAL, BATCH, LE, C2>());
+  else if (form == PMGPU_PAIRK_LJC2_COULC2) go(e64_instance<VIRIAL, BATCH, LC, C2, C2>());
+  else if (form == PMGPU_PAIRK_LJC2_COULC1) go(e64_instance<VIRIAL, BATCH, LC, C2, C1>());
+  else if (mask == TERM_LJ) go(e64_instance<VIRIAL, BATCH, TERM_LJ>());
+  else if (mask == TERM_COUL) go(e64_instance<VIRIAL, BATCH, TERM_COUL>());
+  else if (mask == LC) go(e64_instance<VIRIAL, BATCH, LC>());
+  else if (mask == TERM_EWALD) go(e64_instance<VIRIAL, BATCH, TERM_EWALD>());
+  else go(e64_instance<VIRIAL, BATCH, LE>());
 }
 
 // The energy launch's shape.
@@ -1393,7 +1389,7 @@ static cudaError_t launch_e64(PairArgs<float> a, int form, cudaStream_t st) {
   const int nb = e64_blocks(a);
   cudaError_t err = cudaSuccess;
   if (nb)
-    e64_kernel<VIRIAL>(a.mask, form, [&](auto kern, auto) {
+    e64_kernel<VIRIAL, false>(a.mask, form, [&](auto kern) {
       err = raise_smem(kern, e64_smem_bytes<VIRIAL>());
       if (err == cudaSuccess)
         kern<<<nb, kE64Warps * 32, e64_smem_bytes<VIRIAL>(), st>>>(a);
@@ -1628,7 +1624,7 @@ static int generic_batch(BatchTable<PairArgs<float>> &t, int terms, cudaStream_t
 // The energy launch of the table's members (all of one form).
 static int e64_batch(BatchTable<PairArgs<float>> &t, int terms, int form, cudaStream_t st) {
   if (!t.members() || !t.total()) return 0;
-  e64_kernel<false>(terms, form, [&](auto, auto kern) {
+  e64_kernel<false, true>(terms, form, [&](auto kern) {
     if (raise_smem(kern, e64_smem_bytes<false>()) == cudaSuccess)
       kern<<<t.total(), kE64Warps * 32, e64_smem_bytes<false>(), st>>>(t.d, t.d_first,
                                                                        t.members());
