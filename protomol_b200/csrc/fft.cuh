@@ -106,31 +106,31 @@ inline bool fft_plan(int K0, int K1, int K2, FftGrid *g) {
 }
 
 // a / b for 0 <= a < 2^20 from inv = 1.0f / b.
-__host__ __device__ __forceinline__ int fft_div(int a, float inv) {
+__device__ __forceinline__ int fft_div(int a, float inv) {
   return (int)(((float)a + 0.5f) * inv);
 }
 
-__host__ __device__ __forceinline__ float2 c_add(float2 a, float2 b) {
+__device__ __forceinline__ float2 c_add(float2 a, float2 b) {
   return make_float2(a.x + b.x, a.y + b.y);
 }
-__host__ __device__ __forceinline__ float2 c_sub(float2 a, float2 b) {
+__device__ __forceinline__ float2 c_sub(float2 a, float2 b) {
   return make_float2(a.x - b.x, a.y - b.y);
 }
-__host__ __device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
+__device__ __forceinline__ float2 c_mul(float2 a, float2 b) {
   return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 // a - i b and a + i b
-__host__ __device__ __forceinline__ float2 c_sub_i(float2 a, float2 b) {
+__device__ __forceinline__ float2 c_sub_i(float2 a, float2 b) {
   return make_float2(a.x + b.y, a.y - b.x);
 }
-__host__ __device__ __forceinline__ float2 c_add_i(float2 a, float2 b) {
+__device__ __forceinline__ float2 c_add_i(float2 a, float2 b) {
   return make_float2(a.x - b.y, a.y + b.x);
 }
 
 // exp(-2 pi i m / R) of the composite butterflies (folded: m is a constant
 // after unrolling).
 template <int R>
-__host__ __device__ __forceinline__ float2 fft_root(int m) {
+__device__ __forceinline__ float2 fft_root(int m) {
   if (R == 6) {
     constexpr float c[6] = {1.f, 0.5f, -0.5f, -1.f, -0.5f, 0.5f};
     constexpr float s[6] = {0.f, -0.86602540378443865f, -0.86602540378443865f, 0.f,
@@ -162,7 +162,7 @@ template <int R>
 struct Dft;
 template <>
 struct Dft<2> {
-  static __host__ __device__ __forceinline__ void go(float2 (&v)[2]) {
+  static __device__ __forceinline__ void go(float2 (&v)[2]) {
     const float2 a = v[0];
     v[0] = c_add(a, v[1]);
     v[1] = c_sub(a, v[1]);
@@ -170,7 +170,7 @@ struct Dft<2> {
 };
 template <>
 struct Dft<3> {
-  static __host__ __device__ __forceinline__ void go(float2 (&v)[3]) {
+  static __device__ __forceinline__ void go(float2 (&v)[3]) {
     const float2 t = c_add(v[1], v[2]), e = c_sub(v[1], v[2]);
     const float2 u = make_float2(v[0].x - 0.5f * t.x, v[0].y - 0.5f * t.y);
     const float2 d = make_float2(0.86602540378443865f * e.x, 0.86602540378443865f * e.y);
@@ -181,7 +181,7 @@ struct Dft<3> {
 };
 template <>
 struct Dft<4> {
-  static __host__ __device__ __forceinline__ void go(float2 (&v)[4]) {
+  static __device__ __forceinline__ void go(float2 (&v)[4]) {
     const float2 s0 = c_add(v[0], v[2]), d0 = c_sub(v[0], v[2]);
     const float2 s1 = c_add(v[1], v[3]), d1 = c_sub(v[1], v[3]);
     v[0] = c_add(s0, s1);
@@ -192,7 +192,7 @@ struct Dft<4> {
 };
 template <>
 struct Dft<5> {
-  static __host__ __device__ __forceinline__ void go(float2 (&v)[5]) {
+  static __device__ __forceinline__ void go(float2 (&v)[5]) {
     constexpr float c1 = 0.30901699437494742f, c2 = -0.80901699437494742f;
     constexpr float s1 = 0.95105651629515357f, s2 = 0.58778525229247313f;
     const float2 a = c_add(v[1], v[4]), b = c_add(v[2], v[3]);
@@ -212,7 +212,7 @@ struct Dft<5> {
 // R2; output k1 + R1 k2.
 template <int R1, int R2>
 struct DftSplit {
-  static __host__ __device__ __forceinline__ void go(float2 (&v)[R1 * R2]) {
+  static __device__ __forceinline__ void go(float2 (&v)[R1 * R2]) {
     constexpr int R = R1 * R2;
     float2 t[R2][R1];
 #pragma unroll
@@ -250,7 +250,7 @@ struct Dft<10> : DftSplit<5, 2> {};
 // Buffers and twiddles are given as offsets into the block's memory sm, so
 // every access compiles to a shared-memory one.
 template <int R>
-__host__ __device__ __forceinline__ void fft_pass(float2 *sm, int from, int to, int N, int Ns,
+__device__ __forceinline__ void fft_pass(float2 *sm, int from, int to, int N, int Ns,
                                                   int lines, int ld, int tw, int t0, int nt) {
   const int nb = N / R, items = nb * lines, step = nb / Ns;
   const float il = 1.0f / (float)lines, is = 1.0f / (float)Ns;
@@ -274,7 +274,7 @@ __host__ __device__ __forceinline__ void fft_pass(float2 *sm, int from, int to, 
   }
 }
 
-__host__ __device__ __forceinline__ void fft_pass_r(int R, float2 *sm, int from, int to, int N,
+__device__ __forceinline__ void fft_pass_r(int R, float2 *sm, int from, int to, int N,
                                                     int Ns, int lines, int ld, int tw, int t0,
                                                     int nt) {
   switch (R) {
@@ -289,22 +289,14 @@ __host__ __device__ __forceinline__ void fft_pass_r(int R, float2 *sm, int from,
   }
 }
 
-// The threads of a block between two passes (nothing to wait for on the
-// host, where one "thread" runs every item).
-__host__ __device__ __forceinline__ void fft_sync() {
-#ifdef __CUDA_ARCH__
-  __syncthreads();
-#endif
-}
-
 // All passes of one dimension; buffer a holds the data, b is the other
 // one.  Returns the buffer of the result (every pass ends synchronised).
-__host__ __device__ __forceinline__ int fft_lines(const FftDim &d, float2 *sm, int a, int b,
+__device__ __forceinline__ int fft_lines(const FftDim &d, float2 *sm, int a, int b,
                                                   int lines, int ld, int tw, int t0, int nt) {
   int Ns = 1;
   for (int s = 0; s < d.ns; s++) {
     fft_pass_r(d.radix[s], sm, a, b, d.n, Ns, lines, ld, tw, t0, nt);
-    fft_sync();
+    __syncthreads();
     Ns *= d.radix[s];
     const int t = a;
     a = b;
@@ -315,7 +307,7 @@ __host__ __device__ __forceinline__ int fft_lines(const FftDim &d, float2 *sm, i
 
 // z rows 2p and 2p + 1 (transformed as one complex line) into their half
 // spectra, [y][kz].
-__host__ __device__ __forceinline__ void fft_unpack_rows(const FftGrid &g, float2 *sm, int z, int c,
+__device__ __forceinline__ void fft_unpack_rows(const FftGrid &g, float2 *sm, int z, int c,
                                                          int t0, int nt) {
   const int items = g.P * g.Kh;
   const float ik = 1.0f / (float)g.Kh;
@@ -332,7 +324,7 @@ __host__ __device__ __forceinline__ void fft_unpack_rows(const FftGrid &g, float
 // (real and imaginary parts swapped) into swapped complex lines.  The
 // self-conjugate modes (kz = 0 and the Nyquist mode) are real in a real
 // row's spectrum; their imaginary rounding is dropped.
-__host__ __device__ __forceinline__ void fft_pack_rows(const FftGrid &g, float2 *sm, int c, int z,
+__device__ __forceinline__ void fft_pack_rows(const FftGrid &g, float2 *sm, int c, int z,
                                                        int t0, int nt) {
   const int items = g.P * g.Kh;
   const float ik = 1.0f / (float)g.Kh;
