@@ -132,3 +132,27 @@ def test_row_passes(ctx, n, rc):
     exact, size = _coulomb_pairs(s, rc)
     got = np.concatenate([[e[0]], e[7:16]])
     assert (np.abs(got - exact) <= 16 * 2.0 ** -53 * size + 2.0 ** -50).all()
+
+
+def test_reciprocal_root_of_the_energy_pass(ctx):
+    """The mixed path's FP64 energies take 1 / r from an estimate and two Newton
+    steps, within two units in the last place; a pair's Coulomb energy of about
+    1e8 shows it beside a fixed-point unit of 1e-18 of it.  Distances of 21 bits
+    along one axis, so r^2 is exact; two more units for the product with the
+    charges, the conversion and the comparison's own roundings."""
+    s = systems.tip3p_box(1, 20.0, seed=1)
+    s.periodic, s.box = False, np.zeros(12)
+    s.pos = np.zeros((3, 3))
+    s.pos[2, 1] = 500.0  # out of reach
+    s.charge = np.array([2.0 ** 15, 2.0 ** 15, 0.0])
+    s.exclusions, s.molecule = np.zeros((0, 3), np.int32), np.arange(3, dtype=np.int32)
+    gs = GpuSystem(ctx, s, "mixed")
+    force = ForceFactory(gs, 20.0).make("Coulomb -algorithm NonbondedCutoff -switchingFunction "
+                                        "Cutoff -cutoff 20 -cutoff 20")
+    rng = np.random.default_rng(3)
+    for r in rng.integers(2 ** 16, 20 * 2 ** 16, 300) / 2.0 ** 16:
+        s.pos[1, 0] = r
+        e = ScalarStructure()
+        force.evaluate(s.pos, np.zeros_like(s.pos), e)
+        assert abs(e[0] * r / 2.0 ** 30 - 1.0) <= 4 * 2.0 ** -52, r
+    gs.close()
