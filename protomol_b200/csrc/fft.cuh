@@ -17,7 +17,8 @@
 // (swap, transform, swap), so only forward butterflies exist.
 //
 // Sizes: every dimension a product of 2, 3 and 5 whose plane fits the
-// shared memory (fft_plan); others keep cuFFT (pme.cu).
+// shared memory (fft_plan) and where the kernels are the faster form
+// (fft_pays, pme.cu); others keep cuFFT (pme.cu).
 #pragma once
 
 #include <cuda_runtime.h>
@@ -88,7 +89,7 @@ inline bool fft_radices(int n, FftDim *d) {
 }
 
 // Plans a grid; false when the kernels do not take its dimensions.
-// A block has up to 227 KB of shared memory: cubic grids up to 162^3 fit.
+// A block has up to 227 KB of shared memory: planes up to 162 x 162 fit.
 constexpr size_t kFftSmem = 216 * 1024;
 inline bool fft_plan(int K0, int K1, int K2, FftGrid *g) {
   g->K0 = K0; g->K1 = K1; g->K2 = K2;

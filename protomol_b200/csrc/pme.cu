@@ -632,6 +632,27 @@ static int fft_plane_threads(const FftGrid &g) {
 }
 static int fft_x_blocks(const FftGrid &g) { return (g.K1 * g.Kh + g.cols - 1) / g.cols; }
 
+// Whether the three kernels are the faster form of a grid they take.  Not
+// where a plane kernel's blocks come in a second wave (more planes than are
+// resident at once, one an SM from about 118 x 118 points on), where few
+// planes are large, or where a column block's 128 threads have more than 32
+// elements each.  Reciprocal term of a small box, cuFFT and the kernels, us:
+//   128^3 69 and 67, 144^3 80 and 74, 160^3 113 and 135;
+//   144 x 128 x 128 70 and 68, 160 x 128 x 128 78 and 97, 200 x 100 x 100
+//   (two planes an SM) 78 and 69;
+//   48 x 128 x 128 58 and 58, 32 x 128 x 128 51 and 59, 32 x 108 x 108 51 and
+//   52, 32 x 144 x 144 52 and 63;
+//   256 x 64 x 64 61 and 53, 512 x 64 x 64 74 and 80; 512 x 16 x 16 51 and 45,
+//   1024 x 16 x 16 58 and 67.
+constexpr int kFftSms = 148;
+constexpr size_t kSmSmem = 228 * 1024;  // shared memory of an SM; a block takes 1 KB more
+static bool fft_pays(const FftGrid &g) {
+  const int per_sm = std::min((int)(kSmSmem / (fft_plane_smem(g) + 1024)),
+                              2048 / fft_plane_threads(g));
+  return g.K0 <= kFftSms * per_sm && (g.K0 >= 48 || g.K1 * g.K2 < 128 * 128) &&
+         g.K0 * g.cols <= 32 * kFftXThreads;
+}
+
 static FftArgs fft_args(const System *s, const Force *f, int em) {
   return FftArgs{f->fft, f->d_grid_fixed, f->d_grid,
                  ConvolveArgs{f->grid[0], f->grid[1], f->grid[2], s->box.e[0], s->box.e[1],
@@ -681,7 +702,7 @@ int pme_init(System *s, Force *f) {
                             cudaMemcpyHostToDevice, s->stream));
     PM_CUDA(cudaStreamSynchronize(s->stream));
   }
-  if (fft_plan(K0, K1, K2, &f->fft)) {
+  if (fft_plan(K0, K1, K2, &f->fft) && fft_pays(f->fft)) {
     std::vector<float2> tw;
     for (int a = 0; a < 3; a++)
       for (int m = 0; m < f->grid[a]; m++) {
