@@ -1082,7 +1082,8 @@ int nb_build(System *s, NeighborList *nl) {
   return PMGPU_OK;
 }
 
-static int pair_splits(int nclusters);
+static int tile_splits32(int nclusters);
+static int tile_splits64(int nclusters);
 
 // The Ewald real-space force factor of one pair in FP64, the reference's
 // form with the A&S erfc (MathUtilities.cpp:39-49; Abramowitz & Stegun
@@ -1187,7 +1188,9 @@ static void fill_pair_args(PairArgs<Real> &a, System *s, NeighborList *nl,
   a.csf64 = t.coulomb_scaling;
   a.cap = nl->cap;
   a.nclusters = nl->nclusters;
-  a.splits = pair_splits(nl->nclusters);
+  a.splits = sizeof(Real) == 4 ? tile_splits32(nl->nclusters) : tile_splits64(nl->nclusters);
+  a.shares = a.splits;
+  a.group = 1;
   a.sorted = nl->d_sorted;
   a.pos = s->d_pos;
   a.excl_start = s->d_excl_start;
@@ -1239,20 +1242,47 @@ static int sm_count() {
   return sms;
 }
 
-// Warps per i cluster of the tile kernel: about 160 warps an SM (five waves
-// of the 32 FP32 ones that are resident, ten of the 16 FP64 ones), at most
-// kPairMaxSplits per cluster, so blocks that finish early are refilled and
-// the tail stays short.  A small box has few clusters and each warp's tiles
-// are one serial chain (FP64 or run-time switches), so it takes many: with 8
-// at most, 648 atoms in FP64 left five warps an SM (38 us a launch; 13 us
-// with 32), and the generic members of a 24-box ensemble took 46 instead of
-// 34 us.  The split depends only on the system, so every launch of a system
-// sums its forces in the same order.
-constexpr int kPairMaxSplits = 32;
-static int pair_splits(int nclusters) {
+// Warps per i cluster of the FP32 tile kernel: about 160 an SM (five waves
+// of the 32 that are resident), at most 32, so blocks that finish early are
+// refilled and the tail stays short.  A small box has few clusters and each
+// warp's tiles are one serial chain with run-time switches, so it takes many:
+// 50 steps of 60 waters with PME, 8 | 16 | 32 at most: 2586 | 1876 | 1676 us.
+// Depends only on the system, so every launch of a system sums its forces in
+// the same order.
+static int tile_splits32(int nclusters) {
   const long long want = 160LL * sm_count();
-  return (int)std::max(1LL, std::min((long long)kPairMaxSplits,
-                                     (want + nclusters / 2) / std::max(1, nclusters)));
+  return (int)std::max(1LL, std::min(32LL, (want + nclusters / 2) / std::max(1, nclusters)));
+}
+
+// Shares of a cluster's tiles that a warp of a batched launch takes, over
+// `clusters` clusters in all, where one system's own launch has `shares`
+// warps a cluster.  Few boxes want all of those warps; many fill the device
+// with fewer, and each warp costs its start and its i sums: warps a cluster
+// shrink with the root of the clusters.  20 steps of N boxes of 100 waters
+// (46 clusters each, 32 shares) with 4 | 8 | 16 | 32 warps a cluster, us:
+//   4: 1857 | 1272 |  982 |  910      16: 2173 | 1660 | 1561 | 1682
+//  64: 4300 | 4020 | 4129 | 4709
+// and of 128 boxes of 120: 8516 | 8485 | 9088 | 10588.
+static int batch_group(long long clusters, int shares) {
+  const long long most = 9LL * sm_count() * sm_count();
+  int group = 1;
+  while (group < shares && clusters * (shares / group) * (shares / group) > most) group *= 2;
+  return group;
+}
+
+// Warps per i cluster of the FP64 tile kernel (16 are resident on an SM): two
+// and a half waves, which a small box takes in up to 32 warps a cluster, and
+// at least nearly four waves in up to 8.  A step with a fixed 8 | and with
+// the rule of the FP32 kernel | and with this, us:
+//     648 atoms (95 clusters)  52.1 | 28.8 | 28.7
+//   2,100      (300)           55.7 | 45.3 | 42.5
+//   3,600      (500)           61.1 | 63.6 | 57.5
+//   7,500      (1,000)         92.0 | 104  | 92.2
+//  24,000      (3,100)          241 | 237  | 227
+static int tile_splits64(int nclusters) {
+  const int few = std::min(32, 40 * sm_count() / std::max(1, nclusters));
+  const int many = std::min(8, (60 * sm_count() + nclusters / 2) / std::max(1, nclusters));
+  return std::max(1, std::max(few, many));
 }
 
 template <typename Real, int TERMS>
@@ -1536,6 +1566,8 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
   b->form = PMGPU_PAIRK_GENERIC;
   b->smem_lj = 1;
   b->tab = 1;
+  std::vector<PairArgs<float>> generic;
+  long long generic_clusters = 0;
   for (int k = 0; k < n; k++) {
     System *s = m[k];
     NeighborList *nl = &s->lists[0];
@@ -1567,7 +1599,8 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
       b->jl.add(fa, (int)(((long long)fa.nclusters * fa.splits + kJlWarps - 1) / kJlWarps));
       b->has_form[k] = 1;
     } else {
-      b->gforce.add(a, (int)(((long long)a.nclusters * a.splits + kPairWarps - 1) / kPairWarps));
+      generic.push_back(a);
+      generic_clusters += a.nclusters;
     }
     // the energy kernel of a special form compiles its switches in, so the
     // members without one take a table of their own
@@ -1576,6 +1609,11 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
     (form != PMGPU_PAIRK_GENERIC ? b->energy : b->genergy).add(ea, e64_blocks(ea));
     b->slots.add(SlotArgs{nl->ns_max, s->n, nl->d_sorted, nl->d_fslot, s->d_force},
                  (nl->ns_max + 255) / 256);
+  }
+  for (auto &a : generic) {
+    a.group = batch_group(generic_clusters, a.shares);
+    a.splits = (a.shares + a.group - 1) / a.group;
+    b->gforce.add(a, (int)(((long long)a.nclusters * a.splits + kPairWarps - 1) / kPairWarps));
   }
   BatchTable<PairArgs<float>> *pt[] = {&b->jl, &b->gforce, &b->energy, &b->genergy};
   PM_CUDA(b->bin.upload());

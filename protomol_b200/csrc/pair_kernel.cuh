@@ -47,6 +47,8 @@ struct PairArgs {
   int cap;              // tiles per row
   int nclusters;        // 8-atom i clusters (kRowParts tile rows each)
   int splits;           // warps per i cluster
+  int shares, group;    // batched FP32 tile kernel: a cluster's shares of tiles
+                        // and how many a warp takes
   const int *sorted;
   const double *pos;     // raw positions (exact re-test)
   const int *excl_start, *excl_partner, *excl_class;
@@ -356,7 +358,11 @@ __device__ __forceinline__ void block_energies(long long *acc, const double (&v)
 // Pairs are accepted by the cutoff tests of the reference (with the exact
 // FP64 re-test near a cutoff); the tile mask carries the list's exclusion
 // and modified (scaled 1-4) status.
-template <typename Real, int TERMS, int MODE>
+//
+// SHARES (FP32, batched launches): a warp takes `group` of the `shares` that
+// the single-system launch gives a warp each, and rounds its i sums to fixed
+// point share by share, so it leaves the same forces with fewer warps.
+template <typename Real, int TERMS, int MODE, bool SHARES>
 __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   constexpr bool MIXED = sizeof(Real) == 4;
   // (in mixed precision energies come from k_pairs_e64)
@@ -379,11 +385,24 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
   static_assert(kRowParts == 4, "one int4 of row counts per cluster");
   const int4 c4 = *reinterpret_cast<const int4 *>(a.tile_count + kRowParts * ci);
   const int cnt = item ? c4.x + c4.y + c4.z + c4.w : 0;
-  const int t0 = (int)((long long)cnt * sp / a.splits);
-  const int t1 = (int)((long long)cnt * (sp + 1) / a.splits);
+  const int t0 = SHARES ? (int)((long long)cnt * (sp * a.group) / a.shares)
+                        : (int)((long long)cnt * sp / a.splits);
+  const int t1 = SHARES ? (int)((long long)cnt * min((sp + 1) * a.group, a.shares) / a.shares)
+                        : (int)((long long)cnt * (sp + 1) / a.splits);
   const int islot = 8 * ci + il;
   const int oi = a.sorted[islot];
   Real fx = 0, fy = 0, fz = 0;
+  // an i component's sum over the 4 j lanes of each i atom: lane (il, jl)
+  // ends with component jl (x, y, z, none) of i atom il
+  auto i_sum = [&]() {
+    const bool b0 = jl & 1, b1 = jl & 2;
+    const Real r0 = (b0 ? fy : fx) + __shfl_xor_sync(kAll, b0 ? fx : fy, 8);
+    const Real r1 = (b0 ? Real(0) : fz) + __shfl_xor_sync(kAll, b0 ? fz : Real(0), 8);
+    return (b1 ? r1 : r0) + __shfl_xor_sync(kAll, b1 ? r0 : r1, 16);
+  };
+  // this warp's i sums in fixed point, of the shares done (SHARES)
+  __shared__ long long s_i[SHARES ? kPairWarps : 1][24];
+  if (SHARES && jl < 3) s_i[wib][lane] = 0;
   if (t1 > t0) {
   const double4 wi = a.xw[islot];  // the FP64 kernel only
   Real xi_h[3], xi_l[3];
@@ -413,11 +432,18 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
     p++;
     rowlen = p == 1 ? c4.y : (p == 2 ? c4.z : c4.w);
   }
-  for (int left = t1 - t0; left > 0;) {
+  // tb: the end of the share tile tc is in (this warp's only one without
+  // SHARES)
+  int tc = t0, tb = t1;
+  unsigned share = SHARES ? sp * a.group : 0;
+  while (tc < t1) {
+    if (SHARES) {
+      while ((tb = (int)((unsigned)cnt * (share + 1u) / (unsigned)a.shares)) == tc) share++;
+    }
     const size_t row0 = (size_t)(kRowParts * ci + p) * a.cap;
     const uint2 *row = a.tiles + row0;
-    const int ke = min(rowlen, kb + left);
-    left -= ke - kb;
+    const int ke = min(rowlen, kb + (tb - tc));
+    tc += ke - kb;
   for (int k = kb; k < ke; k++) {
     const uint2 t2 = __ldg(row + k);
     const uint3 tile = make_uint3(t2.x, t2.y,
@@ -535,7 +561,13 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
       if (il < 3 && ((act >> (8 * jl)) & 0xFFu)) red_add(dst, v);
     }
   }
-    if (left > 0) {  // next non-empty row part
+    kb = ke;
+    if (SHARES && tc == tb) {
+      const Real v = i_sum();
+      if (jl < 3) s_i[wib][lane] += fixed_force(v);
+      fx = fy = fz = 0;
+    }
+    if (tc < t1 && kb == rowlen) {  // next non-empty row part
       do {
         p++;
         rowlen = __ldg(a.tile_count + kRowParts * ci + p);
@@ -544,30 +576,17 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
     }
   }
   }  // tiles
-  // i's share: summed over the 4 j lanes of each i atom
-#pragma unroll
-  for (int o = 8; o < 32; o <<= 1) {
-    fx += __shfl_xor_sync(kAll, fx, o);
-    fy += __shfl_xor_sync(kAll, fy, o);
-    fz += __shfl_xor_sync(kAll, fz, o);
-  }
+  const Real isum = SHARES ? Real(0) : i_sum();
   if constexpr (MIXED) {
-    if (jl == 0 && oi >= 0 && t1 > t0) {
-      red_add(&a.fslot[islot], fixed_force(fx));
-      red_add(&a.fslot[a.ns + islot], fixed_force(fy));
-      red_add(&a.fslot[2 * a.ns + islot], fixed_force(fz));
-    }
+    if (jl < 3 && oi >= 0 && t1 > t0)
+      red_add(&a.fslot[jl * a.ns + islot], SHARES ? s_i[wib][lane] : fixed_force(isum));
   } else {
     // in FP64 the rounding to fixed point is the forces' only error: the
     // block's warps of one cluster add up first, so that an atom's i share is
     // rounded once a block, not once a warp
     __shared__ double s_f[kPairWarps][24];
     __shared__ int s_ci[kPairWarps];
-    if (jl == 0) {
-      s_f[wib][il] = fx;
-      s_f[wib][8 + il] = fy;
-      s_f[wib][16 + il] = fz;
-    }
+    if (jl < 3) s_f[wib][lane] = isum;
     if (lane == 0) s_ci[wib] = item ? ci : -1;
     __syncthreads();
     if (item && (wib == 0 || s_ci[wib - 1] != ci) && lane < 24) {
@@ -598,7 +617,7 @@ __device__ __forceinline__ void pairs_body(const PairArgs<Real> &a, Blk blk) {
 template <typename Real, int TERMS, int MODE>
 __global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE>::blocks)
     k_pairs(PairArgs<Real> a) {
-  pairs_body<Real, TERMS, MODE>(a, own_blk());
+  pairs_body<Real, TERMS, MODE, false>(a, own_blk());
 }
 
 template <typename Real, int TERMS, int MODE>
@@ -606,7 +625,7 @@ __global__ void __launch_bounds__(kPairWarps * 32, PairOccupancy<Real, MODE>::bl
     k_pairs_batch(const PairArgs<Real> *__restrict__ tab, const int *__restrict__ first, int nm) {
   __shared__ __align__(16) unsigned char raw[sizeof(PairArgs<Real>)];
   const int m = batch_member(first, nm, blockIdx.x);
-  pairs_body<Real, TERMS, MODE>(batch_args_shared(tab, m, raw), batch_blk(first, m));
+  pairs_body<Real, TERMS, MODE, true>(batch_args_shared(tab, m, raw), batch_blk(first, m));
 }
 
 // ---------------------------------------------------------------------------
