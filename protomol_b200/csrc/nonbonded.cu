@@ -1313,9 +1313,14 @@ static void launch_tiles(const PairArgs<Real> &a, cudaStream_t st, int mode) {
 //   16,666 (6,534)               7166 | 7193 | 7537 | 7796 | 8530 | 9311
 //   20,000 (7,816)               8401 | 8626
 // and 24 boxes of 100 to 1,000 waters as one ensemble: 4440 us with 8 each,
-// 4270 by this rule.  Depends only on the system, so every launch of a
-// system sums its forces in the same order.
-static int jl_splits(int nclusters) {
+// 4270 by this rule.  Those are at a cutoff of 9 A; one beyond 10 A gives each
+// cluster more entries, over which the cost of a split spreads, so the warps
+// grow with them (at most 6).  At 12 A, 2 | 3 | 4 | 6 | 8 warps, 30 steps:
+//   2,500 waters (1,000)  2289 | 2038 | 1955 | 1917 | 1896
+//   5,000 (2,000)         2960 | 2902 | 2824 | 2842 | 2882
+// Depends only on the system, so every launch of a system sums its forces in
+// the same order.
+static int jl_splits(int nclusters, double cut2) {
   const int wave = 3 * sm_count() * kJlWarps;
   static int forced = -1;
   if (forced < 0) {
@@ -1324,7 +1329,9 @@ static int jl_splits(int nclusters) {
   }
   if (forced) return std::min(forced, kJlMaxSplits);
   if (nclusters >= 2 * wave) return 1;
-  return std::max(2, std::min(6, wave * 3 / 4 / std::max(1, nclusters)));
+  // a cluster's entries over those at 9.9 A (reach: the cutoff and the skin)
+  const double r = (std::sqrt(cut2) + 1.3) / 11.2, len = std::max(1.0, r * r * r);
+  return std::max(2, std::min(6, (int)(wave * 3 / 4 * len / std::max(1, nclusters))));
 }
 
 // Warps per i cluster of the FP64 energy kernel: two and a quarter waves of
@@ -1358,7 +1365,7 @@ static void launch_jl(const PairArgs<float> &a, int nb, cudaStream_t st) {
 // are few.
 template <int TERMS, typename SPEC>
 static void launch_force_spec(PairArgs<float> a, cudaStream_t st) {
-  a.splits = jl_splits(a.nclusters);
+  a.splits = jl_splits(a.nclusters, a.max_cut2);
   const long long items = (long long)a.nclusters * a.splits;
   const int nb = (int)((items + kJlWarps - 1) / kJlWarps);
   if (nb == 0) return;
@@ -1594,7 +1601,7 @@ int nb_batch_build(NbBatch *b, System *const *m, int n, const PairTerms *terms,
       b->tab = b->tab && a.ewtab != nullptr;
       PairArgs<float> fa = a;
       fa.splits = splits && splits[k] > 0 ? std::min(splits[k], kJlMaxSplits)
-                                          : jl_splits(fa.nclusters);
+                                          : jl_splits(fa.nclusters, fa.max_cut2);
       b->base[k] = fa;
       b->jl.add(fa, (int)(((long long)fa.nclusters * fa.splits + kJlWarps - 1) / kJlWarps));
       b->has_form[k] = 1;
@@ -1749,7 +1756,7 @@ int nb_batch_time_jl(NbBatch *b, System *const *m, int n, const int *splits, int
   for (int k = 0; k < n && k < (int)b->has_form.size(); k++) {
     if (!b->has_form[k]) continue;
     PairArgs<float> a = b->base[k];
-    a.splits = splits[k] > 0 ? std::min(splits[k], kJlMaxSplits) : jl_splits(a.nclusters);
+    a.splits = splits[k] > 0 ? std::min(splits[k], kJlMaxSplits) : jl_splits(a.nclusters, a.max_cut2);
     b->probe.add(a, (int)(((long long)a.nclusters * a.splits + kJlWarps - 1) / kJlWarps));
   }
   if (!b->probe.members()) return PMGPU_OK;

@@ -71,3 +71,26 @@ def test_double_at_every_division(ctx, waters):
     assert abs(e[0] - eo["coulomb"]) <= 1e-8 * max(1.0, abs(eo["coulomb"]))
     assert abs(e[1] - eo["lj"]) <= 1e-8 * max(1.0, abs(eo["lj"]))
     assert np.abs(e[7:16] - np.ravel(vo)).max() <= 1e-8 * max(1.0, np.abs(vo).max())
+
+
+@pytest.mark.parametrize("waters,rc,splits", [(600, 9.0, 6), (1667, 9.0, 3), (1667, 12.0, 6),
+                                              (2600, 9.0, 2), (2600, 12.0, 4), (5000, 12.0, 2)])
+def test_force_kernel_at_long_cutoffs(ctx, waters, rc, splits):
+    """The force-only kernel's division grows with the cutoff; FP32 forces
+    against the oracle (1e-5 relative, the repository's mixed-precision bound)."""
+    s = systems.water_box_for_density(waters, 0.0334, 7, jitter=0.2)
+    gs = GpuSystem(ctx, s, "mixed")
+    force = ForceFactory(gs, rc).make(
+        f"LennardJones Coulomb -algorithm NonbondedCutoff -switchingFunction C2 -switchon "
+        f"{rc - 1} -cutoff {rc} -switchingFunction C1 -cutoff {rc} -cutoff {rc}")
+    f = np.zeros_like(s.pos)
+    force.evaluate(s.pos, f, None)
+    one = SystemEnsemble([gs])
+    assert one.member(0)[1] == splits
+    one.close()
+    gs.close()
+    o = oracle.System(pos=s.pos, charge=s.charge, type=s.type, molecule=s.molecule, lj=s.lj,
+                      excl=s.exclusions, periodic=True, box=s.box)
+    fo, _, _ = oracle.cutoff_force(o, rc, rc, [
+        ("LennardJones", oracle.Switch("C2", rc, rc - 1)), ("Coulomb", oracle.Switch("C1", rc))])
+    assert F.rms_rel(f, fo) <= 1e-5
