@@ -184,7 +184,7 @@ __device__ __forceinline__ Real gb_dBT(Real dist, Real oi, Real oj, Real Sj) {
 __global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
   __shared__ double sm[kRowWarps];
   RowWarp r;
-  double epair = 0.0;
+  double epair = 0.0, fx = 0, fy = 0, fz = 0;
   if (row_warp(a.n, split, &r)) {
     const int i = r.i;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
@@ -194,7 +194,6 @@ __global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
     const double part_i = a.partial[i];
     const double ace_i = a.ace ? a.ace[i] : 0.0;
     const double d = a.dielec;
-    double fx = 0, fy = 0, fz = 0;
     for (int j = r.j0; j < a.n; j += r.dj) {
       if (j == i) continue;
       const double dx = a.pos[3 * j] - xi, dy = a.pos[3 * j + 1] - yi, dz = a.pos[3 * j + 2] - zi;
@@ -225,17 +224,10 @@ __global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
       fx -= dx * f; fy -= dy * f; fz -= dz * f;
     }
     __syncwarp();
-    fx = warp_sum(fx);
-    fy = warp_sum(fy);
-    fz = warp_sum(fz);
-    if ((threadIdx.x & 31) == 0) {
-      red_add(&a.force[i], to_fixed(fx, kForceScale));
-      red_add(&a.force[a.n + i], to_fixed(fy, kForceScale));
-      red_add(&a.force[2 * a.n + i], to_fixed(fz, kForceScale));
-    }
   }
+  row_force(a.force, a.n, r.i, split, fx, fy, fz);
   epair = row_block_sum(epair, sm) * 0.5 * a.dielec;
-  if (threadIdx.x == 0) red_add(&a.acc[ACC_COULOMB], to_fixed(epair, kEnergyScale));
+  if (threadIdx.x == 0) red_add_energy(a.acc, ACC_COULOMB, epair);
 }
 
 // ---------------------------------------------------------------------
@@ -1120,7 +1112,9 @@ __global__ void k_gb_static_out(int n, const long long *__restrict__ force,
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n)
     for (int c = 0; c < 3; c++) out[3 * i + c] = (double)force[c * n + i] * (1.0 / kForceScale);
-  if (i == 0) *energy = (double)acc[ACC_COULOMB] / kEnergyScale;
+  if (i == 0)
+    *energy = (double)acc[ACC_COULOMB] / kEnergyScale +
+              (double)acc[ACC_LOW + ACC_COULOMB] / (kEnergyScale * kLowScale);
 }
 
 }  // namespace

@@ -1920,39 +1920,6 @@ __device__ __forceinline__ void row_energies(long long *acc, int em, bool lj, bo
   red_add_energy(acc, t == 0 ? ACC_LJ : (t == 1 ? ACC_COULOMB : ACC_VIRIAL + t - 2), x);
 }
 
-// The force on atom i, summed over its warps in the block (split, a power of
-// two, or all of them) and then rounded to fixed point: in FP64 that rounding
-// is the force's only error, and one a warp would make it larger than with
-// one thread an atom.  Every thread of the block calls it.
-__device__ __forceinline__ void row_force(long long *force, int n, int i, int split, double fx,
-                                          double fy, double fz) {
-  __shared__ double sf[kRowWarps][3];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  fx = warp_sum(fx);
-  fy = warp_sum(fy);
-  fz = warp_sum(fz);
-  const int warps = min(split, kRowWarps);
-  if (warps > 1) {
-    if (lane == 0) {
-      sf[wib][0] = fx;
-      sf[wib][1] = fy;
-      sf[wib][2] = fz;
-    }
-    __syncthreads();
-    if (lane != 0 || (wib & (warps - 1))) return;
-    for (int w = wib + 1; w < wib + warps; w++) {
-      fx += sf[w][0];
-      fy += sf[w][1];
-      fz += sf[w][2];
-    }
-  }
-  if (lane == 0 && i < n) {
-    red_add(&force[i], to_fixed(fx, kForceScale));
-    red_add(&force[n + i], to_fixed(fy, kForceScale));
-    red_add(&force[2 * n + i], to_fixed(fz, kForceScale));
-  }
-}
-
 template <bool LJ, bool COUL>
 __global__ void __launch_bounds__(kRowThreads) k_simplefull(SfArgs a) {
   RowWarp r;

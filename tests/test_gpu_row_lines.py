@@ -58,6 +58,11 @@ def _born(o):
     return f, {"coulomb": e, "lj": 0.0}, None
 
 
+def _gb(o):
+    f, e, _ = oracle.gb_force(o, 1.0, 78.5)
+    return f, {"coulomb": e, "lj": 0.0}, None
+
+
 def _ace(o):
     f, e = oracle.gbace_force(o)
     return f, {"coulomb": e, "lj": 0.0}, None
@@ -77,12 +82,13 @@ LINES = {
                lambda o: oracle.scpism_pair_force(o, [(LJ, CN[1]), ("CoulombSCPISM", CN[1])])),
     "born": ([f"{name} {SCP} -switchingFunction Cutoff -bornswitch 3 -cutoff 5 -cutoff 5"
               for name in ("BornRadii", "BornSelf")], _born),
+    "gb": ([f"GBForce {SIMPLE} -soluteDielec 1.0 -solventDielec 78.5"], _gb),
     "ace": ([f"GBACEForce {SIMPLE}"], _ace),
 }
 
 
 @pytest.mark.parametrize("line", sorted(LINES))
-@pytest.mark.parametrize("n", [2, 5, 31, 33, 64, 149, 297, 593, 1185])
+@pytest.mark.parametrize("n", [2, 5, 31, 33, 64, 149, 297, 593, 1185, 2400])
 def test_row_line(ctx, n, line):
     s, o = _polymer(n)
     text, reference = LINES[line]
@@ -91,7 +97,7 @@ def test_row_line(ctx, n, line):
     ff = ForceFactory(gs)
     force = [ff.make(t) for t in text][-1]
     f, e = np.zeros_like(s.pos), ScalarStructure()
-    force.evaluate(s.pos, f, e, virial=line != "ace")  # (GB has no virial)
+    force.evaluate(s.pos, f, e, virial=line not in ("gb", "ace"))  # (GB has none)
     f2, e2 = np.zeros_like(s.pos), ScalarStructure()
     force.evaluate(s.pos, f2, e2)  # without the virial: the same launches otherwise
     f3 = np.zeros_like(s.pos)
@@ -102,7 +108,7 @@ def test_row_line(ctx, n, line):
     assert F.rms_rel(f, fo) <= TOL or np.abs(f - fo).max() <= 4 * UNIT
     assert abs(e[0] - eo["coulomb"]) <= TOL * max(1.0, abs(eo["coulomb"]))
     assert abs(e[1] - eo["lj"]) <= TOL * max(1.0, abs(eo["lj"]))
-    if line == "ace":
+    if line in ("gb", "ace"):
         return
     v = np.asarray(e[7:16]).reshape(3, 3)
     moment = s.pos.T @ fo
