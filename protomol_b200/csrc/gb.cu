@@ -182,7 +182,6 @@ __device__ __forceinline__ Real gb_dBT(Real dist, Real oi, Real oj, Real Sj) {
 }
 
 __global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
-  __shared__ double sm[kRowWarps];
   RowWarp r;
   double epair = 0.0, fx = 0, fy = 0, fz = 0;
   if (row_warp(a.n, split, &r)) {
@@ -225,9 +224,8 @@ __global__ void __launch_bounds__(kRowThreads) k_gb_force(GbArgs a, int split) {
     }
     __syncwarp();
   }
-  row_force(a.force, a.n, r.i, split, fx, fy, fz);
-  epair = row_block_sum(epair, sm) * 0.5 * a.dielec;
-  if (threadIdx.x == 0) red_add_energy(a.acc, ACC_COULOMB, epair);
+  row_finish(a.force, a.acc, a.n, split, 1, false, true,
+             {fx, fy, fz, 0.0, epair * 0.5 * a.dielec, 0.0, 0.0, 0.0}, {});
 }
 
 // ---------------------------------------------------------------------

@@ -1895,35 +1895,10 @@ struct SfArgs {
   int em;
 };
 
-// The energies (em >= 1; v[0] LJ, v[1] Coulomb, of the terms asked for) and
-// virial (em 2; v[2..7] the upper triangle) of a lane's pairs into the
-// accumulators: summed over the block, then one two-word add a slot, a
-// thread each.  Every thread of the block calls it.
-__device__ __forceinline__ void row_energies(long long *acc, int em, bool lj, bool coul,
-                                             const double (&v)[8]) {
-  __shared__ double se[kRowWarps][8];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, t = threadIdx.x;
-#pragma unroll
-  for (int q = 0; q < 8; q++) {
-    if (q >= 2 && em != 2) break;
-    const double x = warp_sum(v[q]);
-    if (lane == 0) se[wib][q] = x;
-  }
-  __syncthreads();
-  if (t >= (em == 2 ? 11 : 2) || (t == 0 && !lj) || (t == 1 && !coul)) return;
-  // threads 2 to 10: the nine entries of the symmetric virial
-  const int row = (t - 2) / 3, col = (t - 2) % 3, lo = min(row, col), hi = max(row, col);
-  const int q = t < 2 ? t : 2 + (lo == 0 ? hi : lo + hi + 1);
-  double x = 0.0;
-#pragma unroll
-  for (int w = 0; w < kRowWarps; w++) x += se[w][q];
-  red_add_energy(acc, t == 0 ? ACC_LJ : (t == 1 ? ACC_COULOMB : ACC_VIRIAL + t - 2), x);
-}
-
 template <bool LJ, bool COUL>
 __global__ void __launch_bounds__(kRowThreads) k_simplefull(SfArgs a) {
   RowWarp r;
-  double elj = 0, ec = 0, fx = 0, fy = 0, fz = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  double elj = 0, ec = 0, fx = 0, fy = 0, fz = 0, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (row_warp(a.n, a.split, &r)) {
     const int i = r.i;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
@@ -1965,10 +1940,8 @@ __global__ void __launch_bounds__(kRowThreads) k_simplefull(SfArgs a) {
     }
     __syncwarp();
   }
-  row_force(a.force, a.n, r.i, a.split, fx, fy, fz);
-  if (!a.em) return;
-  const double sums[8] = {0.5 * elj, 0.5 * ec, v[0], v[1], v[2], v[3], v[4], v[5]};
-  row_energies(a.acc, a.em, LJ, COUL, sums);
+  row_finish(a.force, a.acc, a.n, a.split, a.em, LJ, COUL,
+             {fx, fy, fz, 0.5 * elj, 0.5 * ec, 0.0, 0.0, 0.0}, v);
 }
 
 // NonbondedSimpleFull with switching functions: OneAtomPair /
@@ -2019,7 +1992,7 @@ __device__ __forceinline__ void scpism_pair(double qq, double sai, double saj, d
 
 __global__ void __launch_bounds__(kRowThreads) k_simplefull_sw(SfSwArgs a) {
   RowWarp r;
-  double elj = 0, ec = 0, fx = 0, fy = 0, fz = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  double elj = 0, ec = 0, fx = 0, fy = 0, fz = 0, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (row_warp(a.n, a.split, &r)) {
     const int i = r.i;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
@@ -2094,10 +2067,8 @@ __global__ void __launch_bounds__(kRowThreads) k_simplefull_sw(SfSwArgs a) {
     }
     __syncwarp();
   }
-  row_force(a.force, a.n, r.i, a.split, fx, fy, fz);
-  if (!a.em) return;
-  const double sums[8] = {0.5 * elj, 0.5 * ec, v[0], v[1], v[2], v[3], v[4], v[5]};
-  row_energies(a.acc, a.em, a.lj, a.coul, sums);
+  row_finish(a.force, a.acc, a.n, a.split, a.em, a.lj, a.coul,
+             {fx, fy, fz, 0.5 * elj, 0.5 * ec, 0.0, 0.0, 0.0}, v);
 }
 
 // The FP32 pass over each unordered pair once, as the reference visits
@@ -2490,7 +2461,7 @@ __global__ void __launch_bounds__(kRowThreads) k_born_radii(BornArgs a) {
 __global__ void __launch_bounds__(kRowThreads) k_born_self(BornArgs a) {
   RowWarp w;
   const int n = a.n;
-  double e = 0, fx = 0, fy = 0, fz = 0, v[6] = {0, 0, 0, 0, 0, 0};
+  double e = 0, fx = 0, fy = 0, fz = 0, v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (row_warp(n, 1, &w)) {
     const int i = w.i;
     const double xi = a.pos[3 * i], yi = a.pos[3 * i + 1], zi = a.pos[3 * i + 2];
@@ -2528,10 +2499,7 @@ __global__ void __launch_bounds__(kRowThreads) k_born_self(BornArgs a) {
     // (BornSelfForce.h:108-117, postProcess :128-135)
     if (__any_sync(0xffffffffu, used) && (threadIdx.x & 31) == 0) e = a.born_q[n + i];
   }
-  row_force(a.force, n, w.i, 1, fx, fy, fz);
-  if (!a.em) return;
-  const double sums[8] = {0.0, e, v[0], v[1], v[2], v[3], v[4], v[5]};
-  row_energies(a.acc, a.em, false, true, sums);
+  row_finish(a.force, a.acc, n, 1, a.em, false, true, {fx, fy, fz, 0.0, e, 0.0, 0.0, 0.0}, v);
 }
 
 int nb_born(System *s, const Force &f, int em) {

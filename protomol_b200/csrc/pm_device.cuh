@@ -171,16 +171,17 @@ __device__ __forceinline__ float exp2f_fast(float x) {
 // (9 shuffles): each exchange step hands half of the remaining slots to the
 // partner lane, so lane l ends with the total of slot (l >> 2) & 7, as do
 // the other three lanes of its quad.  The order of the additions is fixed.
-__device__ __forceinline__ float warp_tsum8(const float (&v)[8], int lane) {
+template <typename T>
+__device__ __forceinline__ T warp_tsum8(const T (&v)[8], int lane) {
   const bool b4 = lane & 16, b3 = lane & 8, b2 = lane & 4;
-  float a[4], b[2];
+  T a[4], b[2];
 #pragma unroll
   for (int m = 0; m < 4; m++)
     a[m] = (b4 ? v[m + 4] : v[m]) + __shfl_xor_sync(0xffffffffu, b4 ? v[m] : v[m + 4], 16);
 #pragma unroll
   for (int m = 0; m < 2; m++)
     b[m] = (b3 ? a[m + 2] : a[m]) + __shfl_xor_sync(0xffffffffu, b3 ? a[m] : a[m + 2], 8);
-  float c = (b2 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, b2 ? b[0] : b[1], 4);
+  T c = (b2 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, b2 ? b[0] : b[1], 4);
   c += __shfl_xor_sync(0xffffffffu, c, 2);
   c += __shfl_xor_sync(0xffffffffu, c, 1);
   return c;
@@ -508,20 +509,6 @@ __host__ inline int row_split(int n) {
 __host__ inline int row_blocks(int n, int split) {
   return (int)(((long long)n * split + kRowWarps - 1) / kRowWarps);
 }
-// Sums v over the block's warps (each lane's v first summed over its warp);
-// thread 0 returns the total.  Every thread calls it; kRowThreads threads.
-__device__ __forceinline__ double row_block_sum(double v, double *sm) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) sm[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  if (threadIdx.x == 0)
-    for (int w = 0; w < kRowWarps; w++) t += sm[w];
-  return t;
-}
-
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
@@ -529,37 +516,44 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// The force on atom i, summed over its warps in the block (split, a power of
-// two, or all of them) and then rounded to fixed point: in FP64 that rounding
-// is the force's only error, and one a warp would make it larger than with
-// one thread an atom.  Every thread of the block calls it.
-__device__ __forceinline__ void row_force(long long *force, int n, int i, int split, double fx,
-                                          double fy, double fz) {
-  __shared__ double sf[kRowWarps][3];
+// The end of a row pass: a lane's sums of its pairs go out.  s: the force on
+// its atom (x, y, z) and the LJ and Coulomb energies; v: the virial's upper
+// triangle.  em: 0 forces only, 1 + energies (of the terms asked for), 2 +
+// virial.  Everything is summed over the warp and then over the block's
+// warps of the atom (split, a power of two, or all of them) or of the block;
+// a force is then rounded to fixed point once (in FP64 that rounding is its
+// only error, and one a warp would make it larger than with one thread an
+// atom), energies and virial in two words.  Every thread of the block calls
+// it.
+__device__ __forceinline__ void row_finish(long long *force, long long *acc, int n, int split,
+                                           int em, bool lj, bool coul, const double (&s)[8],
+                                           const double (&v)[8]) {
+  __shared__ double sm[2][kRowWarps][8];
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  fx = warp_sum(fx);
-  fy = warp_sum(fy);
-  fz = warp_sum(fz);
+  const double a = warp_tsum8(s, lane);
+  if ((lane & 3) == 0) sm[0][wib][lane >> 2] = a;
+  if (em == 2) {
+    const double b = warp_tsum8(v, lane);
+    if ((lane & 3) == 0) sm[1][wib][lane >> 2] = b;
+  }
+  __syncthreads();
   const int warps = min(split, kRowWarps);
-  if (warps > 1) {
-    if (lane == 0) {
-      sf[wib][0] = fx;
-      sf[wib][1] = fy;
-      sf[wib][2] = fz;
-    }
-    __syncthreads();
-    if (lane != 0 || (wib & (warps - 1))) return;
-    for (int w = wib + 1; w < wib + warps; w++) {
-      fx += sf[w][0];
-      fy += sf[w][1];
-      fz += sf[w][2];
-    }
+  if (threadIdx.x < 3 * kRowWarps / warps) {  // a thread per component of each atom
+    const int w0 = threadIdx.x / 3 * warps, c = threadIdx.x % 3;
+    const int i = (blockIdx.x * kRowWarps + w0) / split;
+    double f = sm[0][w0][c];
+    for (int w = 1; w < warps; w++) f += sm[0][w0 + w][c];
+    if (i < n) red_add(&force[(size_t)c * n + i], to_fixed(f, kForceScale));
   }
-  if (lane == 0 && i < n) {
-    red_add(&force[i], to_fixed(fx, kForceScale));
-    red_add(&force[n + i], to_fixed(fy, kForceScale));
-    red_add(&force[2 * n + i], to_fixed(fz, kForceScale));
-  }
+  // the second warp: a thread per energy and per entry of the symmetric virial
+  const int t = (int)threadIdx.x - 32;
+  if (!em || t < 0 || t >= (em == 2 ? 11 : 2) || (t == 0 && !lj) || (t == 1 && !coul)) return;
+  const int row = (t - 2) / 3, col = (t - 2) % 3, lo = min(row, col), hi = max(row, col);
+  const int set = t < 2 ? 0 : 1, q = t < 2 ? 3 + t : (lo == 0 ? hi : lo + hi + 1);
+  double x = 0.0;
+#pragma unroll
+  for (int w = 0; w < kRowWarps; w++) x += sm[set][w][q];
+  red_add_energy(acc, t == 0 ? ACC_LJ : (t == 1 ? ACC_COULOMB : ACC_VIRIAL + t - 2), x);
 }
 
 }  // namespace pmgpu
