@@ -381,10 +381,10 @@ int pmgpu_footprint_estimate(int n_atoms, const double box[3], double reach,
 /* Many resident systems advanced together.  Every kernel of an MD step is
  * one launch over all members (a device table of per-member arguments and
  * first-block offsets; each block finds its member by binary search), the
- * members whose PME grids have the same dimensions share one batched FFT
- * plan pair, and the steps of a segment replay as captured CUDA graphs, so
- * the launches per step do not grow with the member count.  A member's
- * launches compute what its own single-system launches compute, in the
+ * PME transforms of all members included (grids those kernels do not take
+ * share a batched cuFFT plan pair per grid size), and the steps of a segment
+ * replay as captured CUDA graphs, so the launches per step do not grow with
+ * the member count.  A member's launches compute what its own single-system launches compute, in the
  * same fixed-point sums: its trajectory is bitwise the same in any
  * ensemble, alone or beside others, for the same pair-kernel splits.
  *
@@ -415,7 +415,7 @@ int pmgpu_ensemble_set_splits(pmgpu_ensemble *e, const int *splits);
 int pmgpu_ensemble_time_pairs(pmgpu_ensemble *e, const int *splits, int reps, double *ms);
 typedef struct {
   int members;
-  int fft_buckets;         /* distinct PME grids (one batched FFT pair each) */
+  int fft_buckets;         /* distinct PME grids */
   long long kernels;       /* own kernel launches of the last run */
   long long graph_replays; /* CUDA graph launches of the last run */
   long long steps;         /* MD steps of the last run */

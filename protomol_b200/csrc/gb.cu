@@ -919,10 +919,10 @@ k_gb_force_packed(GbArgs a, int tiles, long long items) {
   if (lane == 0 && epair != 0.0) red_add(&a.acc[ACC_COULOMB], to_fixed(epair, kEnergyScale));
 }
 
-// Whether a molecule gives every warp of the packed passes two and a half
-// items (from 3,457 atoms on 148 SMs).  One evaluation, the passes above and
-// these: 3,000 atoms 79.5 and 80.6 us, 3,600 104.6 and 92.9, 4,352 128.8 and
-// 107.3.
+// Whether a molecule gives every warp of the 16-warp passes (partial sums and
+// forces; the burial pass has 24) two and a half items: from 3,457 atoms on
+// 148 SMs.  One evaluation, the passes above and these: 3,000 atoms 79.5 and
+// 80.6 us, 3,600 104.6 and 92.9, 4,352 128.8 and 107.3.
 constexpr int kGbWarps = 16;
 static bool gb_packed(long long items, int blocks) { return 2 * items >= 5LL * blocks * kGbWarps; }
 

@@ -1053,9 +1053,9 @@ __global__ void __launch_bounds__(kJlWarps * 32, 3)
 // run on full warps instead of a third of their lanes, and the reciprocal
 // and the square root share one Newton iteration.  FP64 issue bounds the
 // kernel.  Against one pair per lane of a tile with run-time switches:
-// 49,998 atoms, LJ C2 + Ewald, energies: 488 -> 160 us; 648 atoms, LJ C2 +
-// Coulomb C1: 37 -> 12 us; 12,000 atoms, Cn at 10 A, energies and virial:
-// 650 us with the forces -> 146 us, and 119 us for the forces.
+// 49,998 atoms, LJ C2 + Ewald, energies: 488 -> 157 us; 648 atoms, LJ C2 +
+// Coulomb C1: 37 -> 10 us; 12,000 atoms, Cn at 10 A, energies and virial:
+// 650 us with the forces -> 117 us, and 115 us for the forces.
 constexpr int kE64Warps = 8;
 constexpr int kE64Queue = 32 + 256;  // pairs left over + pairs of one warp step
 template <bool VIRIAL>

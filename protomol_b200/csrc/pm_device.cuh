@@ -471,14 +471,16 @@ __device__ __forceinline__ const A &batch_args_shared(const A *__restrict__ tab,
 }
 
 // All pairs in FP64, a warp (or `split` of them) per atom i with its lanes
-// on the partners j: the sums over j end in one warp reduction and one
-// fixed-point add per atom, and even a few hundred atoms give every SM
-// several warps.  One thread per i over chunks of j (the layout before)
-// left 25 or fewer blocks of long serial FP64 chains on a protein-sized
-// molecule: 5 to 25 of 148 SMs busy.  547 atoms: SCPISM pairs 440 -> 15 us,
-// Born radii 196 -> 13 us, Born self 223 -> 15 us; 544 atoms: LJ 94 -> 7.8,
-// Coulomb 80 -> 7.1, GB burial 40 -> 9.1, partial 28 -> 6.4, force 115 ->
-// 17.4 us.
+// on the partners j: the sums over j end in one reduction (row_finish), and
+// even a few hundred atoms give every SM several warps.  One thread per i
+// over chunks of j, staged in shared memory (the layout before), left 25 or
+// fewer blocks of long serial FP64 chains on a protein-sized molecule: 5 to
+// 25 of 148 SMs busy.  547 atoms: SCPISM pairs 440 -> 15 us, Born radii 196
+// -> 12, Born self 223 -> 14; 544 atoms: LJ 94 -> 8, Coulomb 80 -> 8, GB
+// burial 40 -> 9, partial 28 -> 6.5, force 115 -> 18 us.  Larger molecules
+// gain less, but none loses: whole evaluations of 2,000, 4,000, 8,191 atoms,
+// GB 358 -> 265, 1345 -> 898, 4632 -> 4010 us, SCPISM pairs 516 -> 129, 1567
+// -> 422, 4978 -> 1660, LJ 120 -> 46, 254 -> 103, 759 -> 405.
 constexpr int kRowThreads = 128;
 constexpr int kRowWarps = kRowThreads / 32;
 struct RowWarp {
@@ -494,8 +496,9 @@ __device__ __forceinline__ bool row_warp(int n, int split, RowWarp *r) {
 // Warps per atom: four, eight while they are one wave (about 16 warps an SM
 // are resident), at most one per 32 partners.  One warp an atom from half a
 // wave on, as few as fill the device, runs into a second wave at 2,369 atoms
-// and is latency-bound below it; from three waves on (7,104 atoms) it is as
-// good and saves the partial sums.  GB evaluations of 1,500, 2,500, 3,300
+// and is latency-bound below it.  From three waves on (7,104 atoms) one, where
+// four give GB and LJ another 11 to 16 % but cost SCPISM and Coulomb 1 to 2
+// (8,191 atoms).  GB evaluations of 1,500, 2,500, 3,300
 // atoms in FP64, a thread per atom | 1 | 4 warps an atom: 219 | 237 | 170,
 // 457 | 574 | 387, 738 | 823 | 617 us; SCPISM pairs of 3,000 860 | 403 | 254.
 __host__ inline int row_split(int n) {

@@ -243,9 +243,9 @@ __global__ void k_pme_convolve_batch(const ConvolveArgs *__restrict__ tab,
 // become five, and an ensemble's launches no longer grow with the number of
 // its grid sizes: a launch's plane or column blocks come from every member.
 // Bound by latency (trips to memory, then five to seven short synchronised
-// passes): at 64^3 the three kernels take 8.1, 8.8 and 7.6 us against 28 us
-// for the eight they replace, at 40^3 6.9, 7.6 and 6.5 against 23 us (caches
-// warm); a 5,001-atom MD step 52.7 against 55.2 us, 24 boxes of nine grid
+// passes): at 64^3 the three kernels take 8.0, 7.3 and 7.3 us against 28 us
+// for the eight they replace, at 40^3 6.8, 5.9 and 6.2 against 23 us (caches
+// warm); with the first version of them a 5,001-atom MD step 52.7 against 55.2 us, 24 boxes of nine grid
 // sizes 259 against 338 us a step.  Launching the chain as programmatic
 // dependents was slower (5,776 against 5,048 us for 50 steps of 23,550
 // atoms: waiting blocks hold room the pair kernel needs).
@@ -283,8 +283,8 @@ __device__ __forceinline__ void fft_stream(int n, L load, S store) {
 // The block's n twiddles into dst.  A thread's first one is loaded before
 // the data (fft_first) and stored after it, so the block waits for memory
 // once, not twice; k_fft_x has the influence function on its way as well.
-// 50 steps of 5,001 atoms 1942 -> 1909 us, of 750 1685 -> 1654, of 23,550
-// 3614 -> 3598.
+// Langevin runs of 50 steps by themselves (no copies to or from the host):
+// 5,001 atoms 1942 -> 1909 us, 750 1685 -> 1654, 23,550 3614 -> 3598.
 __device__ __forceinline__ float2 fft_first(const float2 *tw, int n) {
   return (int)threadIdx.x < n ? __ldg(tw + threadIdx.x) : make_float2(0.f, 0.f);
 }

@@ -698,9 +698,8 @@ class LangevinLeapfrogIntegrator(_Integrator):
 
 class SystemEnsemble:
     """Resident systems advanced together (pmgpu_ensemble_*): every kernel
-    of an MD step is one launch over all members, members with the same PME
-    grid share one batched FFT, and segments replay as captured CUDA
-    graphs.  A member's trajectory is bitwise the one it follows in any
+    of an MD step is one launch over all members, their PME transforms
+    included, and segments replay as captured CUDA graphs.  A member's trajectory is bitwise the one it follows in any
     other ensemble with the same pair-kernel splits.  The members stay
     owned by the caller and must outlive the ensemble."""
 
